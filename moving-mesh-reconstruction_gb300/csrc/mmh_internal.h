@@ -36,6 +36,9 @@ void launch_residual_fma(const double* phi, const double* rhs, const double* coe
                          unsigned long long* maxbits, cudaStream_t s);
 template <class T> void launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
                                           bool zero_init = false);
+// the FP64 sweeps of launch_gs_sweeps (mmh_gs64.cu), phi in place
+void launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
+                        double* scratch, cudaStream_t s);
 // FP32 plane-kernel tile autotuning: the shape pinned for every grid (-1:
 // timed per grid size and device), and the shape chosen for n (-1: none yet)
 constexpr int kGsShapes = 6;

@@ -288,10 +288,8 @@ __device__ __forceinline__ void op_eval(const Stencil<T>& s, T& tdiag, T& t1, T&
         - (s.imkp - s.imkm) * s.f3im) * T(0.25);
 }
 
-// The Gauss-Seidel update's division: IEEE in FP64 (the oracle's bits); the
-// fast reciprocal-based division in FP32 (the mixed form's smoother, which is
-// not bit-matched; within 2 ulp).
-__device__ __forceinline__ double gs_div(double a, double b) { return a / b; }
+// The FP32 Gauss-Seidel update's division: the fast reciprocal-based one (the
+// mixed form's smoother is not bit-matched; within 2 ulp).
 __device__ __forceinline__ float gs_div(float a, float b) { return __fdividef(a, b); }
 
 // Gather the stencil of cell (i,j,k) from global memory.
@@ -455,16 +453,11 @@ __device__ __forceinline__ void gs_put(float* f, int sw, int h2, const float4& v
   *reinterpret_cast<float2*>(f + sw) = make_float2(v.x, v.z);
   *reinterpret_cast<float2*>(f + sw + h2) = make_float2(v.y, v.w);
 }
-__device__ __forceinline__ void gs_put(double* f, int sw, int h2, const double2& v) {
-  f[sw] = v.x;
-  f[sw + h2] = v.y;
-}
 __device__ __forceinline__ float4 gs_get(const float* f, int sw, int h2) {
   float2 e = *reinterpret_cast<const float2*>(f + sw);
   float2 o = *reinterpret_cast<const float2*>(f + sw + h2);
   return make_float4(e.x, o.x, e.y, o.y);
 }
-__device__ __forceinline__ double2 gs_get(const double* f, int sw, int h2) { return make_double2(f[sw], f[sw + h2]); }
 
 // All four in-plane colours of one plane P (k%2 == kpar) for one tile (see
 // GsGeom).  The half sweep reads its own planes from src, the neighbour planes

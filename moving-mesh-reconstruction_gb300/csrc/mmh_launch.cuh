@@ -17,13 +17,16 @@ static const int kBlock = 256;
 // launch that needs the attribute then fails and is reported by the entry
 // point's launch-error check.
 template <class K>
-inline void smem_attr_once(K* kernel, int bytes, std::atomic<unsigned long long>& done) {
+inline void func_attr_once(K* kernel, cudaFuncAttribute attr, int value, std::atomic<unsigned long long>& done) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
   const unsigned long long bit = 1ull << dev;
   if (done.load(std::memory_order_acquire) & bit) return;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
-    done.fetch_or(bit, std::memory_order_acq_rel);
+  if (cudaFuncSetAttribute(kernel, attr, value) == cudaSuccess) done.fetch_or(bit, std::memory_order_acq_rel);
+}
+template <class K>
+inline void smem_attr_once(K* kernel, int bytes, std::atomic<unsigned long long>& done) {
+  func_attr_once(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes, done);
 }
 
 template <class T>
@@ -45,7 +48,8 @@ void launch_metric(const T* def, const T* rho, int n, T dx, T* coef, cudaStream_
 // threads per colour phase and shared memory.  Shapes 4-5 are the strips of
 // 64 cells marching in y over 128 or 256 cell rows (k_gs_strip, LY = ty/2
 // sub-rows).  FP32 levels try the shapes below once per grid size and device
-// and keep the fastest (gs_tile_choice); FP64 levels keep (32, 8).
+// and keep the fastest (gs_tile_choice); FP64 sweeps have kernels of their own
+// (mmh_gs64.cu).
 struct GsShape {
   int tx, ty;
 };
@@ -68,24 +72,17 @@ void gs_plane_launch(const T* src, const T* nbr, T* dst, const T* rhs, const T* 
   k_gs_plane<T, TX, TY, Z><<<dim3(n / TX, n / TY, n / 2), 256, smem, s>>>(src, nbr, dst, rhs, coef, n, dx2, kpar);
 }
 
-// one half sweep with tile shape v (FP64: always (32, 8))
-// (the zero-field variants Z = 1, 2 exist for FP32 only)
+// one FP32 half sweep with tile shape v (Z: the zero-field variants)
 template <class T, int Z = 0>
 void gs_plane_half(int v, const T* src, const T* nbr, T* dst, const T* rhs, const T* coef, int n, T dx2, int kpar,
                    cudaStream_t s) {
-  if constexpr (std::is_same<T, double>::value) {
-    static_assert(Z == 0, "FP64 sweeps read their fields");
-    (void)v;
-    gs_plane_launch<T, 32, 8>(src, nbr, dst, rhs, coef, n, dx2, kpar, s);
-  } else {
-    switch (v) {
-      case 1: gs_plane_launch<T, 64, 8, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
-      case 2: gs_plane_launch<T, 16, 32, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
-      case 3: gs_plane_launch<T, 32, 8, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
-      case 4: gs_strip_launch<64, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
-      case 5: gs_strip_launch<128, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
-      default: gs_plane_launch<T, 32, 16, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
-    }
+  switch (v) {
+    case 1: gs_plane_launch<T, 64, 8, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
+    case 2: gs_plane_launch<T, 16, 32, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
+    case 3: gs_plane_launch<T, 32, 8, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
+    case 4: gs_strip_launch<64, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
+    case 5: gs_strip_launch<128, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
+    default: gs_plane_launch<T, 32, 16, Z>(src, nbr, dst, rhs, coef, n, dx2, kpar, s); break;
   }
 }
 
@@ -104,41 +101,34 @@ inline bool gs_shape_fits(int v, int n) {
 int gs_tile_choice(int n, const float* phi, const float* rhs, const float* coef, float dx2, float* scratch,
                    cudaStream_t s);
 
-// nsweeps 8-colour Gauss-Seidel sweeps.  Grids of 64^3 and up run one fused
+// nsweeps FP32 8-colour Gauss-Seidel sweeps.  Grids of 64^3 and up run one fused
 // launch per half sweep (all in-plane colours of every plane of one parity);
 // smaller grids run one launch per colour.
-// zero_init: phi holds no field yet and the sweeps start from zero (FP32
-// grids of 64^3 and up run the first sweep in place without reading phi;
+// zero_init: phi holds no field yet and the sweeps start from zero (grids of 64^3 and up run the first sweep in place without reading phi;
 // elsewhere phi is zeroed first).
 template <class T>
-void launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
-                      bool zero_init) {
+void launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
+                        bool zero_init) {
   i64 h3 = (i64)(n / 2) * (n / 2) * (n / 2);
   T dx2 = dx * dx;
   int sw0 = 0;
   if (zero_init) {
-    bool done = false;
-    if constexpr (std::is_same<T, float>::value) {
-      if (n >= 64 && nsweeps > 0) {
-        const int v = gs_tile_choice(n, phi, rhs, coef, dx2, scratch, s);
-        prof_begin(kk<T>(KK_GS), s, 4 * h3, n);
-        gs_plane_half<T, 2>(v, phi, phi, phi, rhs, coef, n, dx2, 0, s);
-        prof_end(kk<T>(KK_GS), s, n);
-        prof_begin(kk<T>(KK_GS), s, 4 * h3, n);
-        gs_plane_half<T, 1>(v, phi, phi, phi, rhs, coef, n, dx2, 1, s);
-        prof_end(kk<T>(KK_GS), s, n);
-        count_launch(2);
-        sw0 = 1;
-        done = true;
-      }
+    if (n >= 64 && nsweeps > 0) {
+      const int v = gs_tile_choice(n, phi, rhs, coef, dx2, scratch, s);
+      prof_begin(kk<T>(KK_GS), s, 4 * h3, n);
+      gs_plane_half<T, 2>(v, phi, phi, phi, rhs, coef, n, dx2, 0, s);
+      prof_end(kk<T>(KK_GS), s, n);
+      prof_begin(kk<T>(KK_GS), s, 4 * h3, n);
+      gs_plane_half<T, 1>(v, phi, phi, phi, rhs, coef, n, dx2, 1, s);
+      prof_end(kk<T>(KK_GS), s, n);
+      count_launch(2);
+      sw0 = 1;
+    } else {
+      launch_fill<T>(phi, (i64)n * n * n, T(0), s);
     }
-    if (!done) launch_fill<T>(phi, (i64)n * n * n, T(0), s);
   }
   if (n >= 64) {
-    int v = 0;
-    if constexpr (std::is_same<T, float>::value) {
-      if (nsweeps > sw0) v = gs_tile_choice(n, phi, rhs, coef, dx2, scratch, s);
-    }
+    const int v = nsweeps > sw0 ? gs_tile_choice(n, phi, rhs, coef, dx2, scratch, s) : 0;
     // double buffer: a sweep reads a and leaves the swept field in b
     T* a = phi;
     T* b = scratch;
@@ -187,6 +177,17 @@ void launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nswe
           prof_end(kk<T>(KK_GS), s, n);
           count_launch();
         }
+}
+
+template <class T>
+void launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
+                      bool zero_init) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (zero_init) launch_fill<double>(phi, (i64)n * n * n, 0.0, s);
+    launch_gs64_sweeps(phi, rhs, coef, n, dx, nsweeps, scratch, s);
+  } else {
+    launch_gs32_sweeps<T>(phi, rhs, coef, n, dx, nsweeps, scratch, s, zero_init);
+  }
 }
 
 // The marching FP32 stencil (k_stencil_march) for grids of 64 and up, unless
