@@ -80,6 +80,21 @@ void launch_add(double* a, const double* b, i64 count, cudaStream_t s);  // a = 
 void launch_coarse_inverse(const double* coef, double dx, double* M, cudaStream_t s);
 void launch_coarse_apply(const float* r, const double* M, float* z, cudaStream_t s);
 
+// One FP32 V(nu1, nu2) cycle from the n^3 level (n = 32 or 16) down in one
+// launch (mmh_cycle32.cu): u = V(rhs) from zero.  c0, c1, c2: coefficients of
+// the level and of the next ones above 4^3 (c2 for n = 32 only); M: the 4^3
+// level's inverse; dx: the level's spacing; special: launch_restrict_resid's
+// argument on the level and the next ones.  The same bits as the per-level
+// launches.
+void launch_cycle32(int n, const float* c0, const float* c1, const float* c2, const double* M, double dx, int nu1,
+                    int nu2, const int* special, const float* rhs, float* u, cudaStream_t s);
+// The whole inner solve of the mixed form on such a grid, x from zero with
+// the right-hand side in rhs (left holding the residual), until max|r| <= tol
+// * bn or maxit iterations: out[0] = iterations, out[1] = max|r| (bits).
+void launch_solve32(int n, const float* c0, const float* c1, const float* c2, const double* M, double dx, int nu1,
+                    int nu2, const int* special, float* rhs, float* x, double bn, double tol, int maxit,
+                    unsigned long long* out, cudaStream_t s);
+
 // limiter / spectral / relaxing (FP64)
 struct LimDev;
 void launch_calcdefp_rhs(double* tmp, const double* rho, int n, double dtold, bool mixed, cudaStream_t s);

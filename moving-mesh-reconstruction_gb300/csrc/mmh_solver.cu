@@ -242,6 +242,20 @@ int guard_or_zerosum(mmh_ctx* c, int l, double margin, double floor_, bool guard
 
 int vcycle_fp64(mmh_ctx* c, int l);
 
+// Whether the FP32 levels from l down run as one launch (mmh_cycle32.cu): the
+// 32^3 and 16^3 levels of a cycle without guards and with the exact 4^3 solve.
+bool cycle32_at(const mmh_ctx* c, int l) {
+  const int n = c->nl[l];
+  return (n == 32 || n == 16) && c->coarse_inv && c->nl[c->nlev - 1] == 4 && c->cfg.schedule == MMH_SCHED_TOL &&
+         !c->cfg.precond_guards;
+}
+
+// the special restriction planes of the levels from n down (n, n/2, n/4)
+struct Special {
+  int v[3];
+  Special(int nu1, int n) : v{special_plane(nu1, n), special_plane(nu1, n / 2), special_plane(nu1, n / 4)} {}
+};
+
 // One V-cycle at level l (mgtemplate.f90:6-84; mg4 at multigrid.f90:94-121).
 // u_zero: the level's correction starts from zero (H.u[l] is not yet set);
 // the FP32 cycle then skips zeroing it where its first sweep runs from zero.
@@ -249,6 +263,13 @@ template <class T>
 int vcycle(mmh_ctx* c, int l, bool u_zero = false) {
   Hier<T>& H = hier<T>(c);
   int n = c->nl[l];
+  if constexpr (std::is_same<T, float>::value) {
+    if (u_zero && cycle32_at(c, l)) {
+      launch_cycle32(n, H.coef[l], H.coef[l + 1], n == 32 ? H.coef[l + 2] : nullptr, c->coarse_inv, double(1 << l),
+                     c->cfg.nu1, c->cfg.nu2, Special(c->cfg.nu1, n).v, H.rhs[l], H.u[l], c->s);
+      return MMH_OK;
+    }
+  }
   bool ref = c->cfg.schedule == MMH_SCHED_REF;
   bool at_ng = (n == c->n);
   bool guard = !at_ng && (c->cfg.schedule != MMH_SCHED_TOL || c->cfg.precond_guards);
@@ -413,8 +434,9 @@ void pcg_dot(mmh_ctx* c, const T* a, const T* b, i64 n3, const unsigned long lon
     launch_dot<T>(a, b, n3, abits, bbits, acc, c->s);
 }
 
-// x0_bmax >= 0: x is zero and H.rhs[l0] already holds b, whose max |b| is
-// x0_bmax (the initial residual is b itself: no stencil pass).
+// x0_bmax >= 0: x starts from zero (set here) and H.rhs[l0] already holds b,
+// whose max |b| is x0_bmax (the initial residual is b itself: no stencil
+// pass).
 template <class T>
 int pcg_core(mmh_ctx* c, int l0, double dx, T* x, const T* b, T* p, T* q, double bn, double tol, int maxit,
              int* iters, double* rel_out, double* r0_out, double x0_bmax = -1.0) {
@@ -424,6 +446,21 @@ int pcg_core(mmh_ctx* c, int l0, double dx, T* x, const T* b, T* p, T* q, double
   PcgDev* P = &c->sc->pcg;
   T* r = H.rhs[l0];
   T* z = H.u[l0];
+  if constexpr (std::is_same<T, float>::value) {
+    if (x0_bmax > 0.0 && x0_bmax > tol * bn && dx == double(1 << l0) && cycle32_at(c, l0)) {
+      // small grids: the whole solve in one launch
+      launch_solve32(n, H.coef[l0], H.coef[l0 + 1], n == 32 ? H.coef[l0 + 2] : nullptr, c->coarse_inv, dx, c->cfg.nu1,
+                     c->cfg.nu2, Special(c->cfg.nu1, n).v, r, x, bn, tol, maxit, P->acc[0], c->s);
+      CK(cudaGetLastError());
+      RET(pull_scal(c));
+      *r0_out = x0_bmax;
+      *iters = (int)c->hsc->pcg.acc[0][0];
+      *rel_out = bits_to_double(c->hsc->pcg.acc[0][1]) / bn;
+      if (!(*rel_out == *rel_out)) return MMH_ERR_NAN;
+      return *rel_out <= tol ? MMH_OK : MMH_ERR_DIVERGED;
+    }
+  }
+  if (x0_bmax >= 0.0) launch_fill<T>(x, n3, T(0), c->s);
   CK(cudaMemsetAsync(P, 0, sizeof(PcgDev), c->s));
   double rmax0 = x0_bmax;
   if (x0_bmax >= 0.0) {
@@ -563,7 +600,6 @@ int pcg_level(mmh_ctx* c, int l0, double dx, double rn, int* iters, double* rel_
         status = MMH_ERR_DIVERGED;
         break;
       }
-      launch_fill<float>(c->pe32, n3, 0.0f, c->s);
       int it = 0;
       double rin = 0.0, r0 = 0.0;
       // the inner solve reduces the residual by kInnerTol, or only as far as
