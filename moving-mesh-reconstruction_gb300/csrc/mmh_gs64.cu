@@ -261,7 +261,9 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
     }
   }
   if (tid == 0) stop = 0;
-  __syncthreads();
+  // every CTA of the cluster runs and has its halo before the first store into it
+  if (G::CL == 1) __syncthreads();
+  else cl.sync();
 
   // products of phase p for the cross terms [t0, 12) and the faces, y faces
   // only where they do not depend on the phase before
@@ -421,10 +423,10 @@ void box_launch(double* phi, const double* rhs, const double* coef, double dx2, 
 }  // namespace
 
 // nsweeps FP64 8-colour sweeps of phi on an n^3 grid; scratch: n^3 doubles
-// (n >= 32).
-void launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
-                        double* scratch, cudaStream_t s) {
-  if (nsweeps <= 0) return;
+// (n >= 32).  Returns the buffer that holds the swept field.
+double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
+                           double* scratch, cudaStream_t s) {
+  if (nsweeps <= 0) return phi;
   const i64 h3 = (i64)(n / 2) * (n / 2) * (n / 2);
   const double dx2 = dx * dx;
   if (n <= 16) {
@@ -434,7 +436,7 @@ void launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int 
     else box_launch<16>(phi, rhs, coef, dx2, nsweeps, s);
     prof_end(KK_GS, s, n);
     count_launch();
-    return;
+    return phi;
   }
   int lgn = 0;
   while ((1 << lgn) < n) ++lgn;
@@ -453,7 +455,7 @@ void launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int 
     }
     std::swap(a, b);
   }
-  if (a != phi) cudaMemcpyAsync(phi, a, sizeof(double) * 8 * h3, cudaMemcpyDeviceToDevice, s);
+  return a;
 }
 
 }  // namespace mmh

@@ -34,11 +34,13 @@ template <class T>
 void launch_metric(const T* def, const T* rho, int n, T dx, T* coef, cudaStream_t s, bool fast_div = false);
 void launch_residual_fma(const double* phi, const double* rhs, const double* coef, int n, double dx, float* r32,
                          unsigned long long* maxbits, cudaStream_t s);
-template <class T> void launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
-                                          bool zero_init = false);
-// the FP64 sweeps of launch_gs_sweeps (mmh_gs64.cu), phi in place
-void launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
-                        double* scratch, cudaStream_t s);
+// nsweeps 8-colour sweeps of phi; returns the buffer that holds the swept
+// field, phi or scratch (the other one is then free)
+template <class T> T* launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch,
+                                       cudaStream_t s, bool zero_init = false);
+// the FP64 sweeps of launch_gs_sweeps (mmh_gs64.cu)
+double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
+                           double* scratch, cudaStream_t s);
 // FP32 plane-kernel tile autotuning: the shape pinned for every grid (-1:
 // timed per grid size and device), and the shape chosen for n (-1: none yet)
 constexpr int kGsShapes = 6;
@@ -137,20 +139,28 @@ struct PcgDev {
 };
 template <class T>
 void launch_apply(const T* p, const T* coef, int n, T dx, T* q, unsigned long long* qbits, cudaStream_t s);
-template <class T>
-void launch_dot(const T* a, const T* b, i64 count, const unsigned long long* abits, const unsigned long long* bbits,
-                unsigned long long* acc, cudaStream_t s);
+// exact, order-free dot product (the FP64 form's)
+void launch_dot(const double* a, const double* b, i64 count, const unsigned long long* abits,
+                const unsigned long long* bbits, unsigned long long* acc, cudaStream_t s);
 template <class T>
 void launch_pcg_update(T* x, T* r, const T* p, const T* q, i64 count, const double* alpha, unsigned long long* rbits,
                        cudaStream_t s);
 template <class T>
 void launch_pcg_pupdate(T* p, const T* z, i64 count, const double* beta, unsigned long long* pbits, cudaStream_t s);
 void launch_pcg_scalar(PcgDev* st, int stage, cudaStream_t s);
-// Fast deterministic FP32 dot product (mixed form's inner solve): kDotBlocks
-// block sums in `part`, result into acc in the exact dot's fixed-point form.
+// The inner solve's scalars (mixed form): fast fixed-order FP32 dot products
+// over kDotBlocks block sums, whose last kernel also forms the scalar and
+// clears the maxima the next kernels reduce into.  part: 2 kDotBlocks doubles.
 constexpr int kDotBlocks = 152 * 8;
-void launch_dot_fast(const float* a, const float* b, i64 count, const unsigned long long* abits,
-                     const unsigned long long* bbits, unsigned long long* acc, double* part, cudaStream_t s);
+// P = 0, rbits = bmax
+void launch_pcg_start(PcgDev* P, double bmax, cudaStream_t s);
+// p = z, pbits = max|z|, rz = r.z
+void launch_pcg_first32(float* p, const float* z, const float* r, i64 count, PcgDev* P, double* part, cudaStream_t s);
+// alpha = rz / p.q (pbits, qbits: the maxima of p and q)
+void launch_pcg_alpha32(const float* p, const float* q, i64 count, PcgDev* P, double* part, cudaStream_t s);
+// beta = -(alpha z.q) / rz, rz = r.z
+void launch_pcg_beta32(const float* z, const float* q, const float* r, i64 count, PcgDev* P, double* part,
+                       cudaStream_t s);
 
 // the mixed form's nsmooth: three axis passes, `in` overwritten
 void launch_smooth_sep(double* in, int n, double* out, cudaStream_t s);
@@ -161,7 +171,6 @@ void launch_ff_split(double* a, i64 count, cudaStream_t s);
 // r32 = b rounded through its float-float split (the outer residual of a
 // zero guess), max |r32| into maxbits
 void launch_ff_rhs32(const double* b, i64 count, float* r32, unsigned long long* maxbits, cudaStream_t s);
-void launch_set_u64(unsigned long long* p, unsigned long long v, cudaStream_t s);
 void launch_ff_join(double* a, i64 count, cudaStream_t s);
 void launch_ff_add_f(double* x, const float* e, i64 count, cudaStream_t s);
 void launch_ff_sub_mean(double* x, const double* mean, i64 count, cudaStream_t s);

@@ -79,13 +79,15 @@ int gs_tile_chosen(int n, int* tx, int* ty) {
 MMH_INSTANTIATE(float)
 MMH_INSTANTIATE_PCG(float)
 
-// Dot product of two FP32 vectors for the mixed form's inner solve, whose
+// Dot products of FP32 vectors for the mixed form's inner solve, whose
 // results are not bit-matched to the oracle: a fixed grid of kDotBlocks
 // blocks, each thread summing its strided products in FP32 with four
 // accumulators, each block reducing in a fixed pattern, and one block adding
 // the block sums in FP64 in a fixed order -- deterministic, and bound by
-// memory instead of by the integer work of the exact form.  The result is
-// stored in the fixed-point form (same scale) the PCG scalar kernel reads.
+// memory.  z.q and r.z share the read of z and its maximum (three passes over
+// the vectors instead of five), and the last kernel forms the solver's
+// scalar: below 128^3 an iteration is bound by its launches, and this takes
+// ten of the seventeen between two cycles away.
 __device__ __forceinline__ float block_sum_f32(float v, float* buf) {
   for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -97,48 +99,120 @@ __device__ __forceinline__ float block_sum_f32(float v, float* buf) {
   return t;
 }
 
+// block sums of a.b into part, and with TWO of a.c into part + kDotBlocks and
+// max|a| into abits; copy (TWO) receives a when not null
+template <bool TWO, bool FIRST>
 __global__ void __launch_bounds__(256) k_dot_f32_part(const float* __restrict__ a, const float* __restrict__ b,
-                                                      i64 count, double* __restrict__ part) {
-  __shared__ float buf[32];
+                                                      const float* __restrict__ c, i64 count,
+                                                      double* __restrict__ part, unsigned long long* abits,
+                                                      float* __restrict__ copy) {
+  __shared__ float buf[32], buf2[32];
   const i64 stride = (i64)gridDim.x * blockDim.x;
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  float s[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
+  unsigned m = 0;
+  auto take = [&](i64 at, int k) {
+    const float av = a[at];
+    if (!FIRST) s[k] += av * b[at];
+    if (TWO) {
+      u[k] += c[at] * av;
+      const unsigned ab = abs_bits(av);
+      m = ab > m ? ab : m;
+    }
+    if (FIRST) copy[at] = av;
+  };
   for (; t + 3 * stride < count; t += 4 * stride) {
-    s0 += a[t] * b[t];
-    s1 += a[t + stride] * b[t + stride];
-    s2 += a[t + 2 * stride] * b[t + 2 * stride];
-    s3 += a[t + 3 * stride] * b[t + 3 * stride];
+    take(t, 0);
+    take(t + stride, 1);
+    take(t + 2 * stride, 2);
+    take(t + 3 * stride, 3);
   }
-  for (; t < count; t += stride) s0 += a[t] * b[t];
-  const float blk = block_sum_f32((s0 + s1) + (s2 + s3), buf);
-  if (threadIdx.x == 0) part[blockIdx.x] = (double)blk;
+  for (; t < count; t += stride) take(t, 0);
+  if (!FIRST) {
+    const float blk = block_sum_f32((s[0] + s[1]) + (s[2] + s[3]), buf);
+    if (threadIdx.x == 0) part[blockIdx.x] = (double)blk;
+  }
+  if (TWO) {
+    const float blk = block_sum_f32((u[0] + u[1]) + (u[2] + u[3]), buf2);
+    if (threadIdx.x == 0) part[kDotBlocks + blockIdx.x] = (double)blk;
+    block_max_commit(from_bits(m), abits);
+  }
 }
 
-__global__ void __launch_bounds__(256) k_dot_f32_final(const double* __restrict__ part, int nparts,
-                                                       const unsigned long long* abits,
-                                                       const unsigned long long* bbits, unsigned long long* acc) {
-  __shared__ double buf[256];
+// sum of the block sums of one dot product, rounded as its fixed-point form
+// (2^(E-96), 2^E > max|a| max|b|) holds it; valid in thread 0
+__device__ __forceinline__ double dot_total(const double* __restrict__ part, double* buf, unsigned long long abits,
+                                            unsigned long long bbits) {
   double s = 0.0;
-  for (int q = threadIdx.x; q < nparts; q += blockDim.x) s += part[q];
+  for (int q = threadIdx.x; q < kDotBlocks; q += 256) s += part[q];
   buf[threadIdx.x] = s;
   __syncthreads();
-  for (int h = blockDim.x / 2; h > 0; h >>= 1) {
+  for (int h = 128; h > 0; h >>= 1) {
     if ((int)threadIdx.x < h) buf[threadIdx.x] += buf[threadIdx.x + h];
     __syncthreads();
   }
+  const double v = buf[0];
+  __syncthreads();
+  const double ma = __longlong_as_double((long long)abits), mb = __longlong_as_double((long long)bbits);
+  if (!(ma > 0.0) || !(mb > 0.0) || !(fabs(v) < INFINITY)) return 0.0;
+  const int E = ilogb(ma) + ilogb(mb) + 2;
+  const __int128 fx = fx_bits(v, 96 - E);
+  const unsigned long long acc[2] = {(unsigned long long)fx, (unsigned long long)((unsigned __int128)fx >> 64)};
+  return fx_unscale(acc, E);
+}
+
+// STAGE 0: rz = r.z after the first cycle (p = z); 1: alpha = rz / p.q; 2:
+// beta = -(alpha z.q) / rz, rz = r.z.  Clears the maxima that are read here
+// and reduced into next.
+template <int STAGE>
+__global__ void __launch_bounds__(256) k_pcg_scalar32(const double* __restrict__ part, PcgDev* P) {
+  __shared__ double buf[256];
+  if (STAGE == 1) {
+    const double pq = dot_total(part, buf, P->pbits, P->qbits);
+    if (threadIdx.x == 0) {
+      P->pq = pq;
+      P->alpha = P->rz / pq;
+      P->rbits = 0;
+    }
+    return;
+  }
+  const unsigned long long rb = P->rbits, zb = P->zbits, qb = P->qbits;
+  const double zq = STAGE == 2 ? dot_total(part, buf, zb, qb) : 0.0;
+  const double rz = dot_total(part + kDotBlocks, buf, rb, zb);
   if (threadIdx.x == 0) {
-    const double ma = bits_d(abits), mb = bits_d(bbits);
-    __int128 v = 0;
-    if (ma > 0.0 && mb > 0.0 && fabs(buf[0]) < INFINITY) v = fx_bits(buf[0], 96 - (ilogb(ma) + ilogb(mb) + 2));
-    acc[0] = (unsigned long long)v;
-    acc[1] = (unsigned long long)((unsigned __int128)v >> 64);
+    if (STAGE == 2) P->beta = __ddiv_rn(-__dmul_rn(P->alpha, zq), P->rz);
+    P->rz = rz;
+    P->pbits = STAGE == 0 ? zb : 0;
+    P->zbits = 0;
+    P->qbits = 0;
   }
 }
 
-void launch_dot_fast(const float* a, const float* b, i64 count, const unsigned long long* abits,
-                            const unsigned long long* bbits, unsigned long long* acc, double* part, cudaStream_t s) {
-  k_dot_f32_part<<<kDotBlocks, 256, 0, s>>>(a, b, count, part);
-  k_dot_f32_final<<<1, 256, 0, s>>>(part, kDotBlocks, abits, bbits, acc);
+__global__ void k_pcg_start(PcgDev* P, double bmax) {
+  PcgDev z{};
+  z.rbits = (unsigned long long)__double_as_longlong(bmax);
+  *P = z;
+}
+
+void launch_pcg_start(PcgDev* P, double bmax, cudaStream_t s) {
+  k_pcg_start<<<1, 1, 0, s>>>(P, bmax);
+  count_launch();
+}
+void launch_pcg_first32(float* p, const float* z, const float* r, i64 count, PcgDev* P, double* part,
+                        cudaStream_t s) {
+  k_dot_f32_part<true, true><<<kDotBlocks, 256, 0, s>>>(z, nullptr, r, count, part, &P->zbits, p);
+  k_pcg_scalar32<0><<<1, 256, 0, s>>>(part, P);
+  count_launch(2);
+}
+void launch_pcg_alpha32(const float* p, const float* q, i64 count, PcgDev* P, double* part, cudaStream_t s) {
+  k_dot_f32_part<false, false><<<kDotBlocks, 256, 0, s>>>(p, q, nullptr, count, part, nullptr, nullptr);
+  k_pcg_scalar32<1><<<1, 256, 0, s>>>(part, P);
+  count_launch(2);
+}
+void launch_pcg_beta32(const float* z, const float* q, const float* r, i64 count, PcgDev* P, double* part,
+                       cudaStream_t s) {
+  k_dot_f32_part<true, false><<<kDotBlocks, 256, 0, s>>>(z, q, r, count, part, &P->zbits, nullptr);
+  k_pcg_scalar32<2><<<1, 256, 0, s>>>(part, P);
   count_launch(2);
 }
 

@@ -107,8 +107,8 @@ int gs_tile_choice(int n, const float* phi, const float* rhs, const float* coef,
 // zero_init: phi holds no field yet and the sweeps start from zero (grids of 64^3 and up run the first sweep in place without reading phi;
 // elsewhere phi is zeroed first).
 template <class T>
-void launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
-                        bool zero_init) {
+T* launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
+                      bool zero_init) {
   i64 h3 = (i64)(n / 2) * (n / 2) * (n / 2);
   T dx2 = dx * dx;
   int sw0 = 0;
@@ -143,8 +143,7 @@ void launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int ns
       a = b;
       b = t;
     }
-    if (a != phi) cudaMemcpyAsync(phi, a, sizeof(T) * (size_t)n * n * n, cudaMemcpyDeviceToDevice, s);
-    return;
+    return a;
   }
   if (n <= 8) {
     if (nsweeps > 0) {
@@ -156,7 +155,7 @@ void launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int ns
       prof_end(kk<T>(KK_GS), s, n);
       count_launch();
     }
-    return;
+    return phi;
   }
   if (n <= 16) {
     if (nsweeps > 0) {
@@ -165,7 +164,7 @@ void launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int ns
       prof_end(kk<T>(KK_GS), s, n);
       count_launch();
     }
-    return;
+    return phi;
   }
   unsigned g = grid_of(h3, kBlock);
   for (int sw = 0; sw < nsweeps; ++sw)
@@ -177,16 +176,17 @@ void launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int ns
           prof_end(kk<T>(KK_GS), s, n);
           count_launch();
         }
+  return phi;
 }
 
 template <class T>
-void launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
-                      bool zero_init) {
+T* launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
+                    bool zero_init) {
   if constexpr (std::is_same<T, double>::value) {
     if (zero_init) launch_fill<double>(phi, (i64)n * n * n, 0.0, s);
-    launch_gs64_sweeps(phi, rhs, coef, n, dx, nsweeps, scratch, s);
+    return launch_gs64_sweeps(phi, rhs, coef, n, dx, nsweeps, scratch, s);
   } else {
-    launch_gs32_sweeps<T>(phi, rhs, coef, n, dx, nsweeps, scratch, s, zero_init);
+    return launch_gs32_sweeps<T>(phi, rhs, coef, n, dx, nsweeps, scratch, s, zero_init);
   }
 }
 
@@ -342,7 +342,7 @@ void launch_usum_flag(const unsigned long long* acc, int* flag, cudaStream_t s) 
 
 #define MMH_INSTANTIATE(T)                                                                                          \
   template void launch_metric<T>(const T*, const T*, int, T, T*, cudaStream_t, bool);                             \
-  template void launch_gs_sweeps<T>(T*, const T*, const T*, int, T, int, T*, cudaStream_t, bool);                         \
+  template T* launch_gs_sweeps<T>(T*, const T*, const T*, int, T, int, T*, cudaStream_t, bool);                         \
   template void launch_residual<T>(const T*, const T*, const T*, int, T, T*, float*, unsigned long long*,          \
                                    cudaStream_t);                                                                   \
   template void launch_restrict_resid<T>(const T*, int, int, T*, cudaStream_t);                                   \

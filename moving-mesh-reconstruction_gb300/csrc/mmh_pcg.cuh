@@ -1,7 +1,7 @@
 // Flexible preconditioned conjugate gradients: operator application, exact
-// dot products and vector updates, templated on the vector precision.  Dot
-// products are exact and order free: each product a_i*b_i (formed in FP64,
-// exact for FP32 vectors) is scaled by 2^(96-E), 2^E > max|a|*max|b|,
+// dot products and vector updates, templated on the vector precision.  The
+// FP64 form's dot products are exact and order free: each product a_i*b_i is
+// scaled by 2^(96-E), 2^E > max|a|*max|b|,
 // truncated to a 128-bit integer and summed with two 64-bit atomics.
 #pragma once
 #include "mmh_launch.cuh"
@@ -9,6 +9,16 @@
 namespace mmh {
 
 __device__ __forceinline__ double bits_d(const unsigned long long* b) { return __longlong_as_double((long long)*b); }
+
+// value of a dot product's 128-bit fixed-point accumulator
+__device__ __forceinline__ double fx_unscale(const unsigned long long* acc, int E) {
+  __int128 s = (__int128)(((unsigned __int128)acc[1] << 64) | (unsigned __int128)acc[0]);
+  bool neg = s < 0;
+  unsigned __int128 a = neg ? (unsigned __int128)(-s) : (unsigned __int128)s;
+  double r = __dadd_rn(scalbn(__ull2double_rn((unsigned long long)(a >> 64)), E - 32),
+                       scalbn(__ull2double_rn((unsigned long long)a), E - 96));
+  return neg ? -r : r;
+}
 
 // q = L[p] = (t1 + t2 + tdiag*p) * di2, max|q| into qbits
 template <class T>
@@ -29,34 +39,16 @@ __global__ void k_apply(const T* __restrict__ p, const T* __restrict__ coef, int
   block_max_commit(m, qbits);
 }
 
-// trunc(a*b * 2^sh) for FP32 a, b from their bits: the product of the 24-bit
-// significands is exact in 64 bits, so this equals fx_bits of the (exact)
-// FP64 product without any FP64 operation.
-__device__ __forceinline__ __int128 fx_prod(float a, float b, int sh) {
-  unsigned ua = __float_as_uint(a), ub = __float_as_uint(b);
-  int ea = (int)((ua >> 23) & 0xFF), eb = (int)((ub >> 23) & 0xFF);
-  unsigned ma = ua & 0x7FFFFFu, mb = ub & 0x7FFFFFu;
-  if (ea) ma |= 0x800000u; else ea = 1;
-  if (eb) mb |= 0x800000u; else eb = 1;
-  unsigned long long m = (unsigned long long)ma * mb;
-  int s = ea + eb - 300 + sh;
-  unsigned __int128 v;
-  if (s >= 0) v = (unsigned __int128)m << s;
-  else if (s > -64) v = (unsigned __int128)(m >> (-s));
-  else v = 0;
-  return ((ua ^ ub) >> 31) ? -(__int128)v : (__int128)v;
-}
-__device__ __forceinline__ __int128 fx_prod(double a, double b, int sh) { return fx_bits(a * b, sh); }
-
-template <class T>
-__global__ void k_dot(const T* __restrict__ a, const T* __restrict__ b, i64 count, const unsigned long long* abits,
-                      const unsigned long long* bbits, unsigned long long* acc) {
+// the FP64 form's dot product
+static __global__ void k_dot(const double* __restrict__ a, const double* __restrict__ b, i64 count,
+                             const unsigned long long* abits, const unsigned long long* bbits,
+                             unsigned long long* acc) {
   double ma = bits_d(abits), mb = bits_d(bbits);
   __int128 s = 0;
   if (ma > 0.0 && mb > 0.0) {
     int E = ilogb(ma) + ilogb(mb) + 2;
     for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (i64)gridDim.x * blockDim.x)
-      s += fx_prod(a[t], b[t], 96 - E);
+      s += fx_bits(a[t] * b[t], 96 - E);
   }
   fx_block_commit(s, acc);
 }
@@ -110,16 +102,6 @@ void launch_apply(const T* p, const T* coef, int n, T dx, T* q, unsigned long lo
   else
     k_apply<T><<<grid_of(n3, kBlock), kBlock, 0, s>>>(p, coef, n, T(1) / (dx * dx), q, qbits);
   prof_end(kk<T>(KK_APPLY), s, n);
-  count_launch();
-}
-
-template <class T>
-void launch_dot(const T* a, const T* b, i64 count, const unsigned long long* abits, const unsigned long long* bbits,
-                unsigned long long* acc, cudaStream_t s) {
-  i64 blocks = (count + kBlock - 1) / kBlock;
-  if (blocks > 152 * 16) blocks = 152 * 16;
-  if (blocks < 1) blocks = 1;
-  k_dot<T><<<(unsigned)blocks, kBlock, 0, s>>>(a, b, count, abits, bbits, acc);
   count_launch();
 }
 
@@ -201,8 +183,6 @@ void launch_pcg_pupdate(T* p, const T* z, i64 count, const double* beta, unsigne
 
 #define MMH_INSTANTIATE_PCG(T)                                                                                   \
   template void launch_apply<T>(const T*, const T*, int, T, T*, unsigned long long*, cudaStream_t);             \
-  template void launch_dot<T>(const T*, const T*, i64, const unsigned long long*, const unsigned long long*,     \
-                              unsigned long long*, cudaStream_t);                                                \
   template void launch_pcg_update<T>(T*, T*, const T*, const T*, i64, const double*, unsigned long long*,        \
                                      cudaStream_t);                                                              \
   template void launch_pcg_pupdate<T>(T*, const T*, i64, const double*, unsigned long long*, cudaStream_t);

@@ -109,15 +109,15 @@ struct mmh_ctx {
   // FP32 hierarchy (mixed)
   Hier<float> h32;
   // flexible PCG vectors (solution, right-hand side, search direction, L p);
-  // FP32 correction, right-hand side and directions of the mixed inner solve
+  // FP32 correction and directions of the mixed inner solve
   double *px = nullptr, *pb = nullptr, *pp = nullptr, *pq = nullptr;
-  float *pe32 = nullptr, *pb32 = nullptr, *pp32 = nullptr, *pq32 = nullptr;
+  float *pe32 = nullptr, *pp32 = nullptr, *pq32 = nullptr;
   // relaxing
   double *baj = nullptr, *cc = nullptr, *vt = nullptr, *u1 = nullptr, *gface = nullptr;
   // spectral
   void *Xc = nullptr, *Z = nullptr;
-  double* spectab = nullptr;
-  double* dotpart = nullptr;  // block sums of the fast FP32 dot products  // twiddle and cosine tables of the spectral kernels
+  double* spectab = nullptr;  // twiddle and cosine tables of the spectral kernels
+  double* dotpart = nullptr;  // block sums of the fast FP32 dot products
   cufftHandle pd2z = 0, pz2z = 0;
   bool plans = false;
   Scal* sc = nullptr;   // device
@@ -127,6 +127,7 @@ struct mmh_ctx {
   cudaGraphExec_t pgraph[2][16] = {};
   unsigned long long pgraph_launches[2][16] = {};
   bool pgraph_seen[2][16] = {};
+  void* pz[2][16] = {};  // the buffer a preconditioner application leaves its result in
   bool graphs = true;
   std::vector<void*> allocs;
   int last_status = MMH_OK;
@@ -203,26 +204,28 @@ Hier<double>& hier<double>(mmh_ctx* c) { return c->h64; }
 template <>
 Hier<float>& hier<float>(mmh_ctx* c) { return c->h32; }
 
-// relax(): nrelax 8-colour sweeps, then residual (mode 3: full weighting into
-// rhs[l+1] and max norm; mode 2: max norm only; mode 0: none) into *maxslot.
-// zero_init: H.u[l] holds no field yet; the sweeps start from zero.
+// relax(): nrelax 8-colour sweeps of the field in u, then residual (mode 3:
+// full weighting into rhs[l+1] and max norm; mode 2: max norm only; mode 0:
+// none) into *maxslot (null: no norm).  The sweeps go back and forth between u
+// and r; the two are swapped so that u is the swept field, and r receives the
+// residual.  zero_init: u holds no field yet; the sweeps start from zero.
 template <class T>
-int relax_level(mmh_ctx* c, int l, int nrelax, int mode, unsigned long long* maxslot, bool zero_init = false) {
+int relax_level(mmh_ctx* c, int l, T*& u, T*& r, int nrelax, int mode, unsigned long long* maxslot,
+                bool zero_init = false) {
   Hier<T>& H = hier<T>(c);
   int n = c->nl[l];
   T dx = T(double(1 << l));
-  launch_gs_sweeps<T>(H.u[l], H.rhs[l], H.coef[l], n, dx, nrelax, H.r[l], c->s, zero_init);
+  if (launch_gs_sweeps<T>(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s, zero_init) != u) std::swap(u, r);
   if (mode == 0) return MMH_OK;
-  CK(cudaMemsetAsync(maxslot, 0, 8, c->s));
-  launch_residual<T>(H.u[l], H.rhs[l], H.coef[l], n, dx, mode == 3 ? H.r[l] : (T*)nullptr, nullptr, maxslot, c->s);
-  if (mode == 3) launch_restrict_resid<T>(H.r[l], n, special_plane(nrelax, n), H.rhs[l + 1], c->s);
+  if (maxslot) CK(cudaMemsetAsync(maxslot, 0, 8, c->s));
+  launch_residual<T>(u, H.rhs[l], H.coef[l], n, dx, mode == 3 ? r : (T*)nullptr, nullptr, maxslot, c->s);
+  if (mode == 3) launch_restrict_resid<T>(r, n, special_plane(nrelax, n), H.rhs[l + 1], c->s);
   return MMH_OK;
 }
 
-// post-relaxation step of a level: divergence guard or zerosum
+// post-relaxation step of a level's field u: divergence guard or zerosum
 template <class T>
-int guard_or_zerosum(mmh_ctx* c, int l, double margin, double floor_, bool guard) {
-  Hier<T>& H = hier<T>(c);
+int guard_or_zerosum(mmh_ctx* c, int l, T* u, double margin, double floor_, bool guard) {
   int n = c->nl[l];
   i64 n3 = (i64)n * n * n;
   // The mixed form's FP32 preconditioner keeps the constants its levels
@@ -230,13 +233,13 @@ int guard_or_zerosum(mmh_ctx* c, int l, double margin, double floor_, bool guard
   // sum to zero), so they change neither the PCG's residuals nor its dot
   // products with them, and the outer loop removes the solution's mean.
   if (!guard && std::is_same<T, float>::value && c->cfg.schedule == MMH_SCHED_TOL) return MMH_OK;
-  if (!guard) return zerosum<T>(c, H.u[l], n3);
+  if (!guard) return zerosum<T>(c, u, n3);
   launch_guard(&c->sc->r1bits[l], &c->sc->errbits[l], margin, floor_, &c->sc->gflag[l], &c->sc->guards, c->s);
   CK(cudaMemsetAsync(c->sc->acc[3], 0, 16, c->s));
-  launch_fxsum<T>(H.u[l], n3, c->sc->acc[3], &c->sc->bad, c->s);
+  launch_fxsum<T>(u, n3, c->sc->acc[3], &c->sc->bad, c->s);
   launch_fx_mean(c->sc->acc[3], (double)n3, &c->sc->mean, c->s);
-  launch_sub_mean_unless<T>(H.u[l], n3, &c->sc->mean, &c->sc->gflag[l], c->s);
-  launch_zero_if<T>(H.u[l], n3, &c->sc->gflag[l], c->s);
+  launch_sub_mean_unless<T>(u, n3, &c->sc->mean, &c->sc->gflag[l], c->s);
+  launch_zero_if<T>(u, n3, &c->sc->gflag[l], c->s);
   return MMH_OK;
 }
 
@@ -259,55 +262,67 @@ struct Special {
 // One V-cycle at level l (mgtemplate.f90:6-84; mg4 at multigrid.f90:94-121).
 // u_zero: the level's correction starts from zero (H.u[l] is not yet set);
 // the FP32 cycle then skips zeroing it where its first sweep runs from zero.
+// out: receives the buffer that holds the result, H.u[l] or H.r[l]; null: the
+// result is left in H.u[l].
 template <class T>
-int vcycle(mmh_ctx* c, int l, bool u_zero = false) {
+int vcycle(mmh_ctx* c, int l, bool u_zero = false, T** out = nullptr) {
   Hier<T>& H = hier<T>(c);
   int n = c->nl[l];
+  T *u = H.u[l], *r = H.r[l];
+  if (out) *out = u;
   if constexpr (std::is_same<T, float>::value) {
     if (u_zero && cycle32_at(c, l)) {
       launch_cycle32(n, H.coef[l], H.coef[l + 1], n == 32 ? H.coef[l + 2] : nullptr, c->coarse_inv, double(1 << l),
-                     c->cfg.nu1, c->cfg.nu2, Special(c->cfg.nu1, n).v, H.rhs[l], H.u[l], c->s);
+                     c->cfg.nu1, c->cfg.nu2, Special(c->cfg.nu1, n).v, H.rhs[l], u, c->s);
       return MMH_OK;
     }
   }
   bool ref = c->cfg.schedule == MMH_SCHED_REF;
   bool at_ng = (n == c->n);
   bool guard = !at_ng && (c->cfg.schedule != MMH_SCHED_TOL || c->cfg.precond_guards);
-  // the post-relaxation residual norms feed the guards and the reference's
-  // diagnostics only; the preconditioner of the tolerance schedule without
-  // guards skips them
-  const int post = (guard || c->cfg.schedule != MMH_SCHED_TOL) ? 2 : 0;
+  // the residual norms feed the guards and the reference's diagnostics only;
+  // the preconditioner of the tolerance schedule without guards skips them
+  const bool norms = guard || c->cfg.schedule != MMH_SCHED_TOL;
+  const int post = norms ? 2 : 0;
+  unsigned long long* r1 = norms ? &c->sc->r1bits[l] : nullptr;
+  unsigned long long* err = norms ? &c->sc->errbits[l] : nullptr;
   const bool zfirst = u_zero && std::is_same<T, float>::value && n > 4;
   if (u_zero && !zfirst && !(n == 4 && std::is_same<T, float>::value && c->coarse_inv && !guard))
-    launch_fill<T>(H.u[l], (i64)n * n * n, T(0), c->s);
+    launch_fill<T>(u, (i64)n * n * n, T(0), c->s);
   if (n == 4) {
     if constexpr (std::is_same<T, float>::value) {
       Hier<float>& F = c->h32;
       if (c->coarse_inv && !guard) {
         // exact FP64 solve with the level's inverse (zero-mean result)
-        launch_coarse_apply(F.rhs[l], c->coarse_inv, F.u[l], c->s);
+        launch_coarse_apply(F.rhs[l], c->coarse_inv, u, c->s);
         return MMH_OK;
       }
       // coarsest grid solved in FP64 by the reference's sweeps
       i64 n3 = 64;
       launch_f2d(F.rhs[l], c->h64.rhs[l], n3, c->s);
-      launch_f2d(F.u[l], c->h64.u[l], n3, c->s);
+      launch_f2d(u, c->h64.u[l], n3, c->s);
       RET(vcycle_fp64(c, l));
-      launch_d2f(c->h64.u[l], F.u[l], n3, c->s);
+      launch_d2f(c->h64.u[l], u, n3, c->s);
       return MMH_OK;
     } else {
-      RET(relax_level<T>(c, l, 32, post, &c->sc->r1bits[l]));
-      RET(relax_level<T>(c, l, 32, post, &c->sc->errbits[l]));
-      return guard_or_zerosum<T>(c, l, 1.001, 1.e-5, guard);
+      RET(relax_level<T>(c, l, u, r, 32, post, r1));
+      RET(relax_level<T>(c, l, u, r, 32, post, err));
+      return guard_or_zerosum<T>(c, l, u, 1.001, 1.e-5, guard);
     }
   }
   int nrelax = ref ? 4 * c->n / n : c->cfg.nu1;
   int nrelax2 = ref ? 4 * c->n / n : c->cfg.nu2;
-  RET(relax_level<T>(c, l, nrelax, 3, &c->sc->r1bits[l], zfirst));
-  RET(vcycle<T>(c, l + 1, true));
-  launch_prolong_add<T>(H.u[l], H.u[l + 1], n, c->s);
-  RET(relax_level<T>(c, l, nrelax2, post, &c->sc->errbits[l]));
-  return guard_or_zerosum<T>(c, l, 1.0, -HUGE_VAL, guard);
+  T* uc = nullptr;
+  RET(relax_level<T>(c, l, u, r, nrelax, 3, r1, zfirst));
+  RET(vcycle<T>(c, l + 1, true, &uc));
+  launch_prolong_add<T>(u, uc, n, c->s);
+  RET(relax_level<T>(c, l, u, r, nrelax2, post, err));
+  RET(guard_or_zerosum<T>(c, l, u, 1.0, -HUGE_VAL, guard));
+  if (out)
+    *out = u;
+  else if (u != H.u[l])
+    CK(cudaMemcpyAsync(H.u[l], u, sizeof(T) * (size_t)n * n * n, cudaMemcpyDeviceToDevice, c->s));
+  return MMH_OK;
 }
 
 int vcycle_fp64(mmh_ctx* c, int l) { return vcycle<double>(c, l); }
@@ -363,16 +378,15 @@ int build_levels(mmh_ctx* c, int l0) {
   return MMH_OK;
 }
 
-// One preconditioner application z = V(r) on the precision-T hierarchy:
-// r in H.rhs[l0], z to H.u[l0], max|z| into zbits.
+// One preconditioner application z = V(r) on the precision-T hierarchy: r in
+// H.rhs[l0], z in the buffer c->pz[T][l0] afterwards.
 template <class T>
-int precond(mmh_ctx* c, int l0, unsigned long long* zbits) {
-  Hier<T>& H = hier<T>(c);
-  int n = c->nl[l0];
-  i64 n3 = (i64)n * n * n;
-  RET(vcycle<T>(c, l0, true));
-  CK(cudaMemsetAsync(zbits, 0, 8, c->s));
-  launch_absmax<T>(H.u[l0], n3, zbits, c->s);
+constexpr int type_of() { return std::is_same<T, float>::value ? 1 : 0; }
+template <class T>
+int precond(mmh_ctx* c, int l0) {
+  T* z = nullptr;
+  RET(vcycle<T>(c, l0, true, &z));
+  c->pz[type_of<T>()][l0] = z;
   return MMH_OK;
 }
 
@@ -383,23 +397,23 @@ int precond(mmh_ctx* c, int l0, unsigned long long* zbits) {
 // the kernel timing hooks are armed (they time launches one by one) or when a
 // capture fails.
 template <class T>
-int precond_replay(mmh_ctx* c, int l0, unsigned long long* zbits) {
-  const int ti = std::is_same<T, float>::value ? 1 : 0;
-  if (!c->graphs || l0 >= 16 || prof_armed()) return precond<T>(c, l0, zbits);
+int precond_replay(mmh_ctx* c, int l0) {
+  const int ti = type_of<T>();
+  if (!c->graphs || l0 >= 16 || prof_armed()) return precond<T>(c, l0);
   cudaGraphExec_t& ex = c->pgraph[ti][l0];
   if (!ex) {
     if (!c->pgraph_seen[ti][l0]) {
       c->pgraph_seen[ti][l0] = true;
-      return precond<T>(c, l0, zbits);
+      return precond<T>(c, l0);
     }
     const unsigned long long before = launch_count();
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
       c->graphs = false;
-      return precond<T>(c, l0, zbits);
+      return precond<T>(c, l0);
     }
-    int rc = precond<T>(c, l0, zbits);
+    int rc = precond<T>(c, l0);
     cudaError_t e = cudaStreamEndCapture(c->s, &g);
     if (rc == MMH_OK && e == cudaSuccess && g && cudaGraphInstantiate(&ex, g, 0) == cudaSuccess) {
       cudaGraphDestroy(g);
@@ -411,7 +425,7 @@ int precond_replay(mmh_ctx* c, int l0, unsigned long long* zbits) {
     ex = nullptr;
     cudaGetLastError();
     c->graphs = false;
-    return precond<T>(c, l0, zbits);
+    return precond<T>(c, l0);
   }
   CK(cudaGraphLaunch(ex, c->s));
   count_launch((int)c->pgraph_launches[ti][l0]);
@@ -420,76 +434,46 @@ int precond_replay(mmh_ctx* c, int l0, unsigned long long* zbits) {
 
 // Flexible preconditioned conjugate gradients on L x = b at level l0 in
 // precision T, one V-cycle per iteration as preconditioner, until
-// max|r| <= tol * bn (recurrence residual) or maxit iterations.  The
-// residual lives in H.rhs[l0] (the preconditioner's right-hand side) and the
-// preconditioned residual in H.u[l0].  Dot products are exact (FP64 scalars).
-// Dot product of the PCG in precision T: exact and order-free in FP64 (the
-// oracle's bits), fast and deterministic in FP32 (the mixed inner solve).
-template <class T>
-void pcg_dot(mmh_ctx* c, const T* a, const T* b, i64 n3, const unsigned long long* abits,
-             const unsigned long long* bbits, unsigned long long* acc) {
-  if constexpr (std::is_same<T, float>::value)
-    launch_dot_fast(a, b, n3, abits, bbits, acc, c->dotpart, c->s);
-  else
-    launch_dot<T>(a, b, n3, abits, bbits, acc, c->s);
-}
-
-// x0_bmax >= 0: x starts from zero (set here) and H.rhs[l0] already holds b,
-// whose max |b| is x0_bmax (the initial residual is b itself: no stencil
-// pass).
-template <class T>
-int pcg_core(mmh_ctx* c, int l0, double dx, T* x, const T* b, T* p, T* q, double bn, double tol, int maxit,
-             int* iters, double* rel_out, double* r0_out, double x0_bmax = -1.0) {
-  Hier<T>& H = hier<T>(c);
+// max|r| <= tol * bn (recurrence residual) or maxit iterations.  The residual
+// lives in H.rhs[l0] (the preconditioner's right-hand side).  FP64: the dot
+// products are exact and order-free (the oracle's bits).
+int pcg_core64(mmh_ctx* c, int l0, double dx, double* x, const double* b, double* p, double* q, double bn, double tol,
+               int maxit, int* iters, double* rel_out, double* r0_out) {
+  Hier<double>& H = c->h64;
   int n = c->nl[l0];
   i64 n3 = (i64)n * n * n;
   PcgDev* P = &c->sc->pcg;
-  T* r = H.rhs[l0];
-  T* z = H.u[l0];
-  if constexpr (std::is_same<T, float>::value) {
-    if (x0_bmax > 0.0 && x0_bmax > tol * bn && dx == double(1 << l0) && cycle32_at(c, l0)) {
-      // small grids: the whole solve in one launch
-      launch_solve32(n, H.coef[l0], H.coef[l0 + 1], n == 32 ? H.coef[l0 + 2] : nullptr, c->coarse_inv, dx, c->cfg.nu1,
-                     c->cfg.nu2, Special(c->cfg.nu1, n).v, r, x, bn, tol, maxit, P->acc[0], c->s);
-      CK(cudaGetLastError());
-      RET(pull_scal(c));
-      *r0_out = x0_bmax;
-      *iters = (int)c->hsc->pcg.acc[0][0];
-      *rel_out = bits_to_double(c->hsc->pcg.acc[0][1]) / bn;
-      if (!(*rel_out == *rel_out)) return MMH_ERR_NAN;
-      return *rel_out <= tol ? MMH_OK : MMH_ERR_DIVERGED;
-    }
-  }
-  if (x0_bmax >= 0.0) launch_fill<T>(x, n3, T(0), c->s);
+  double* r = H.rhs[l0];
   CK(cudaMemsetAsync(P, 0, sizeof(PcgDev), c->s));
-  double rmax0 = x0_bmax;
-  if (x0_bmax >= 0.0) {
-    unsigned long long bits = 0;
-    std::memcpy(&bits, &x0_bmax, 8);
-    launch_set_u64(&P->rbits, bits, c->s);
-  } else {
-    launch_residual<T>(x, b, H.coef[l0], n, (T)dx, r, nullptr, &P->rbits, c->s);
-    RET(pull_scal(c));
-    rmax0 = bits_to_double(c->hsc->pcg.rbits);
-  }
+  launch_residual<double>(x, b, H.coef[l0], n, dx, r, nullptr, &P->rbits, c->s);
+  RET(pull_scal(c));
+  const double rmax0 = bits_to_double(c->hsc->pcg.rbits);
   double rel = rmax0 / bn;
   *r0_out = rmax0;
   int it = 0;
   int status = MMH_OK;
+  const double* z = nullptr;
+  auto precondition = [&]() {
+    RET(precond_replay<double>(c, l0));
+    z = (const double*)c->pz[0][l0];
+    CK(cudaMemsetAsync(&P->zbits, 0, 8, c->s));
+    launch_absmax<double>(z, n3, &P->zbits, c->s);
+    return (int)MMH_OK;
+  };
   if (rel > tol) {
-    RET(precond_replay<T>(c, l0, &P->zbits));
-    CK(cudaMemcpyAsync(p, z, sizeof(T) * n3, cudaMemcpyDeviceToDevice, c->s));
+    RET(precondition());
+    CK(cudaMemcpyAsync(p, z, sizeof(double) * n3, cudaMemcpyDeviceToDevice, c->s));
     CK(cudaMemcpyAsync(&P->pbits, &P->zbits, 8, cudaMemcpyDeviceToDevice, c->s));
-    pcg_dot<T>(c, r, z, n3, &P->rbits, &P->zbits, P->acc[0]);
+    launch_dot(r, z, n3, &P->rbits, &P->zbits, P->acc[0], c->s);
     launch_pcg_scalar(P, 0, c->s);
     for (it = 1;; ++it) {
       CK(cudaMemsetAsync(&P->qbits, 0, 8, c->s));
-      launch_apply<T>(p, H.coef[l0], n, (T)dx, q, &P->qbits, c->s);
+      launch_apply<double>(p, H.coef[l0], n, dx, q, &P->qbits, c->s);
       CK(cudaMemsetAsync(P->acc[1], 0, 16, c->s));
-      pcg_dot<T>(c, p, q, n3, &P->pbits, &P->qbits, P->acc[1]);
+      launch_dot(p, q, n3, &P->pbits, &P->qbits, P->acc[1], c->s);
       launch_pcg_scalar(P, 1, c->s);
       CK(cudaMemsetAsync(&P->rbits, 0, 8, c->s));
-      launch_pcg_update<T>(x, r, p, q, n3, &P->alpha, &P->rbits, c->s);
+      launch_pcg_update<double>(x, r, p, q, n3, &P->alpha, &P->rbits, c->s);
       RET(pull_scal(c));
       rel = bits_to_double(c->hsc->pcg.rbits) / bn;
       if (!(rel == rel) || rel <= tol) break;
@@ -497,14 +481,68 @@ int pcg_core(mmh_ctx* c, int l0, double dx, T* x, const T* b, T* p, T* q, double
         status = MMH_ERR_DIVERGED;
         break;
       }
-      RET(precond_replay<T>(c, l0, &P->zbits));
+      RET(precondition());
       CK(cudaMemsetAsync(P->acc[0], 0, 16, c->s));
       CK(cudaMemsetAsync(P->acc[2], 0, 16, c->s));
-      pcg_dot<T>(c, z, q, n3, &P->zbits, &P->qbits, P->acc[2]);
-      pcg_dot<T>(c, r, z, n3, &P->rbits, &P->zbits, P->acc[0]);
+      launch_dot(z, q, n3, &P->zbits, &P->qbits, P->acc[2], c->s);
+      launch_dot(r, z, n3, &P->rbits, &P->zbits, P->acc[0], c->s);
       launch_pcg_scalar(P, 2, c->s);
       CK(cudaMemsetAsync(&P->pbits, 0, 8, c->s));
-      launch_pcg_pupdate<T>(p, z, n3, &P->beta, &P->pbits, c->s);
+      launch_pcg_pupdate<double>(p, z, n3, &P->beta, &P->pbits, c->s);
+    }
+  }
+  *iters = it;
+  *rel_out = rel;
+  if (!(rel == rel)) return MMH_ERR_NAN;
+  return status;
+}
+
+// The same in FP32 from x = 0, H.rhs[l0] holding the right-hand side, whose
+// maximum is bmax (the mixed form's inner solve).  The dot products are fast,
+// fixed-order sums; z.q and r.z are formed together, and their kernels take
+// the scalars and clear the words the next kernels reduce into.
+int pcg_core32(mmh_ctx* c, int l0, double dx, float* x, float* p, float* q, double bmax, double bn, double tol,
+               int maxit, int* iters, double* rel_out) {
+  Hier<float>& H = c->h32;
+  int n = c->nl[l0];
+  i64 n3 = (i64)n * n * n;
+  PcgDev* P = &c->sc->pcg;
+  float* r = H.rhs[l0];
+  double rel = bmax / bn;
+  if (bmax > 0.0 && rel > tol && dx == double(1 << l0) && cycle32_at(c, l0)) {
+    // small grids: the whole solve in one launch
+    launch_solve32(n, H.coef[l0], H.coef[l0 + 1], n == 32 ? H.coef[l0 + 2] : nullptr, c->coarse_inv, dx, c->cfg.nu1,
+                   c->cfg.nu2, Special(c->cfg.nu1, n).v, r, x, bn, tol, maxit, P->acc[0], c->s);
+    CK(cudaGetLastError());
+    RET(pull_scal(c));
+    *iters = (int)c->hsc->pcg.acc[0][0];
+    *rel_out = bits_to_double(c->hsc->pcg.acc[0][1]) / bn;
+    if (!(*rel_out == *rel_out)) return MMH_ERR_NAN;
+    return *rel_out <= tol ? MMH_OK : MMH_ERR_DIVERGED;
+  }
+  launch_fill<float>(x, n3, 0.f, c->s);
+  launch_pcg_start(P, bmax, c->s);
+  int it = 0;
+  int status = MMH_OK;
+  if (rel > tol) {
+    RET(precond_replay<float>(c, l0));
+    const float* z = (const float*)c->pz[1][l0];
+    launch_pcg_first32(p, z, r, n3, P, c->dotpart, c->s);
+    for (it = 1;; ++it) {
+      launch_apply<float>(p, H.coef[l0], n, (float)dx, q, &P->qbits, c->s);
+      launch_pcg_alpha32(p, q, n3, P, c->dotpart, c->s);
+      launch_pcg_update<float>(x, r, p, q, n3, &P->alpha, &P->rbits, c->s);
+      RET(pull_scal(c));
+      rel = bits_to_double(c->hsc->pcg.rbits) / bn;
+      if (!(rel == rel) || rel <= tol) break;
+      if (it >= maxit) {
+        status = MMH_ERR_DIVERGED;
+        break;
+      }
+      RET(precond_replay<float>(c, l0));
+      z = (const float*)c->pz[1][l0];
+      launch_pcg_beta32(z, q, r, n3, P, c->dotpart, c->s);
+      launch_pcg_pupdate<float>(p, z, n3, &P->beta, &P->pbits, c->s);
     }
   }
   *iters = it;
@@ -557,8 +595,7 @@ int pcg_level(mmh_ctx* c, int l0, double dx, double rn, int* iters, double* rel_
   if (c->cfg.precision == MMH_FP64) {
     int it = 0;
     double r0 = 0.0;
-    status = pcg_core<double>(c, l0, dx, c->px, c->pb, c->pp, c->pq, rn, c->cfg.tol, c->cfg.max_cycles, &it, &rel,
-                              &r0);
+    status = pcg_core64(c, l0, dx, c->px, c->pb, c->pp, c->pq, rn, c->cfg.tol, c->cfg.max_cycles, &it, &rel, &r0);
     if (status != MMH_OK && status != MMH_ERR_DIVERGED) return status;
     total = it;
     *r1_out = r0;
@@ -601,12 +638,11 @@ int pcg_level(mmh_ctx* c, int l0, double dx, double rn, int* iters, double* rel_
         break;
       }
       int it = 0;
-      double rin = 0.0, r0 = 0.0;
+      double rin = 0.0;
       // the inner solve reduces the residual by kInnerTol, or only as far as
       // the outer tolerance still needs (with a margin) when that is less
       const double inner_tol = std::max(kInnerTol, 0.3 * c->cfg.tol * rn / rmax);
-      int st = pcg_core<float>(c, l0, dx, c->pe32, c->pb32, c->pp32, c->pq32, rmax, inner_tol, kInnerMax, &it, &rin,
-                               &r0, rmax);
+      int st = pcg_core32(c, l0, dx, c->pe32, c->pp32, c->pq32, rmax, rmax, inner_tol, kInnerMax, &it, &rin);
       if (st != MMH_OK && st != MMH_ERR_DIVERGED) return st;
       total += it;
       if (ff)
@@ -1516,7 +1552,6 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
       S(&c->pq, n3);
     } else {
       S(&c->pe32, n3);
-      S(&c->pb32, n3);
       S(&c->pp32, n3);
       S(&c->pq32, n3);
     }
@@ -1543,7 +1578,7 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
       c->u1 = arena + 17 * n3;
     }
   }
-  if (cfg->precision == MMH_MIXED) A(&c->dotpart, kDotBlocks);
+  if (cfg->precision == MMH_MIXED) A(&c->dotpart, 2 * kDotBlocks);
   A(&c->sc, 1);
   if (rc == MMH_OK && cudaMallocHost((void**)&c->hsc, sizeof(Scal)) != cudaSuccess) rc = MMH_ERR_NOMEM;
   if (rc == MMH_OK && cudaMemsetAsync(c->sc, 0, sizeof(Scal), c->s) != cudaSuccess) rc = MMH_ERR_CUDA;
@@ -1791,17 +1826,18 @@ int mmh_relax_f64(mmh_ctx* c, double* arr, double* resid, const double* rhs, con
     launch_d2f(c->h64.coef[l], F.coef[l], 6 * n3, c->s);
     launch_d2f(c->h64.u[l], F.u[l], n3, c->s);
     launch_d2f(c->h64.rhs[l], F.rhs[l], n3, c->s);
-    launch_gs_sweeps<float>(F.u[l], F.rhs[l], F.coef[l], n, (float)dx, nrelax, F.r[l], c->s);
+    float *fu = F.u[l], *fr = F.r[l];
+    if (launch_gs_sweeps<float>(fu, F.rhs[l], F.coef[l], n, (float)dx, nrelax, fr, c->s) != fu) std::swap(fu, fr);
     CK(cudaMemsetAsync(c->sc->errbits, 0, 8, c->s));
     if (ir != 0) {
-      launch_residual<float>(F.u[l], F.rhs[l], F.coef[l], n, (float)dx, ir == 3 ? F.r[l] : nullptr, nullptr,
+      launch_residual<float>(fu, F.rhs[l], F.coef[l], n, (float)dx, ir == 3 ? fr : nullptr, nullptr,
                              c->sc->errbits, c->s);
       if (ir == 3) {
-        launch_restrict_resid<float>(F.r[l], n, special_plane(nrelax, n), F.rhs[l + 1], c->s);
+        launch_restrict_resid<float>(fr, n, special_plane(nrelax, n), F.rhs[l + 1], c->s);
         launch_f2d(F.rhs[l + 1], c->scr, n3 / 8, c->s);
       }
     }
-    launch_f2d(F.u[l], c->h64.u[l], n3, c->s);
+    launch_f2d(fu, c->h64.u[l], n3, c->s);
     RET(pull_scal(c));
     *rinf = ir >= 2 ? bits_to_double(c->hsc->errbits[0]) : 0.0;
     RET(download(c, c->h64.u[l], arr, n3));
@@ -1809,16 +1845,17 @@ int mmh_relax_f64(mmh_ctx* c, double* arr, double* resid, const double* rhs, con
     return MMH_OK;
   }
   launch_metric<double>(c->defl[l], c->rhol[l], n, dx, c->h64.coef[l], c->s);
-  launch_gs_sweeps<double>(c->h64.u[l], c->h64.rhs[l], c->h64.coef[l], n, dx, nrelax, c->h64.r[l], c->s);
+  double *du = c->h64.u[l], *dr = c->h64.r[l];
+  if (launch_gs_sweeps<double>(du, c->h64.rhs[l], c->h64.coef[l], n, dx, nrelax, dr, c->s) != du) std::swap(du, dr);
   CK(cudaMemsetAsync(c->sc->errbits, 0, 8, c->s));
   if (ir != 0) {
-    launch_residual<double>(c->h64.u[l], c->h64.rhs[l], c->h64.coef[l], n, dx, ir == 3 ? c->h64.r[l] : nullptr,
+    launch_residual<double>(du, c->h64.rhs[l], c->h64.coef[l], n, dx, ir == 3 ? dr : nullptr,
                             nullptr, c->sc->errbits, c->s);
-    if (ir == 3) launch_restrict_resid<double>(c->h64.r[l], n, special_plane(nrelax, n), c->scr, c->s);
+    if (ir == 3) launch_restrict_resid<double>(dr, n, special_plane(nrelax, n), c->scr, c->s);
   }
   RET(pull_scal(c));
   *rinf = ir >= 2 ? bits_to_double(c->hsc->errbits[0]) : 0.0;
-  RET(download(c, c->h64.u[l], arr, n3));
+  RET(download(c, du, arr, n3));
   if (ir == 3) RET(download(c, c->scr, resid, n3 / 8));
   return MMH_OK;
 }
