@@ -115,8 +115,14 @@ void launch_limiter_mask_mixed(double* defplim, const double* def, const double*
                                uint8_t* mask, cudaStream_t s);
 void launch_lim_reset(LimDev* st, cudaStream_t s);
 void launch_spec_tables(double* tab, int n, cudaStream_t s);
-void launch_spec_pack(const void* Xc, int n, int mode, void* Z, const LimDev* st, const double* tab, cudaStream_t s);
-void launch_spec_unpack(const void* z, int n, double* out, int stride_out, int add, const LimDev* st, cudaStream_t s);
+void launch_spec_pack(const void* Xc, int n, void* Z, const LimDev* st, const double* tab, cudaStream_t s);
+void launch_spec_unpack(const void* z, int n, double* out, const LimDev* st, cudaStream_t s);
+// spectral outputs line by line (mmh_spectral.cu): grad (3 n^3) and delta (n^3)
+// of src, either may be null; tab: 4 n doubles made once by launch_fft_tables;
+// T: scratch of 2 n^2 doubles
+void launch_fft_tables(double* tab, int n, cudaStream_t s);
+void launch_spectral_lines(const double* src, int n, double* grad, double* delta, const double* tab, double* T,
+                           cudaStream_t s);
 void launch_relax_stage1(const double* rho, const double* def, const double* defp, int n, double* baj, double* cc,
                          double* sd, cudaStream_t s, bool fast_div = false);
 void launch_relax_flux(const double* u1, const double* defp, const double* baj, const double* cc, int n, double* sd,
@@ -136,6 +142,7 @@ struct PcgDev {
   unsigned long long acc[3][2];
   unsigned long long rbits, zbits, pbits, qbits;
   double rz, pq, alpha, beta;
+  unsigned arrived, pad;  // blocks of the running dot product that are done
 };
 template <class T>
 void launch_apply(const T* p, const T* coef, int n, T dx, T* q, unsigned long long* qbits, cudaStream_t s);

@@ -85,9 +85,9 @@ MMH_INSTANTIATE_PCG(float)
 // accumulators, each block reducing in a fixed pattern, and one block adding
 // the block sums in FP64 in a fixed order -- deterministic, and bound by
 // memory.  z.q and r.z share the read of z and its maximum (three passes over
-// the vectors instead of five), and the last kernel forms the solver's
-// scalar: below 128^3 an iteration is bound by its launches, and this takes
-// ten of the seventeen between two cycles away.
+// the vectors instead of five), and the block that ends last forms the
+// solver's scalar: below 128^3 an iteration is bound by its launches, and this
+// takes twelve of the seventeen between two cycles away.
 __device__ __forceinline__ float block_sum_f32(float v, float* buf) {
   for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -99,52 +99,13 @@ __device__ __forceinline__ float block_sum_f32(float v, float* buf) {
   return t;
 }
 
-// block sums of a.b into part, and with TWO of a.c into part + kDotBlocks and
-// max|a| into abits; copy (TWO) receives a when not null
-template <bool TWO, bool FIRST>
-__global__ void __launch_bounds__(256) k_dot_f32_part(const float* __restrict__ a, const float* __restrict__ b,
-                                                      const float* __restrict__ c, i64 count,
-                                                      double* __restrict__ part, unsigned long long* abits,
-                                                      float* __restrict__ copy) {
-  __shared__ float buf[32], buf2[32];
-  const i64 stride = (i64)gridDim.x * blockDim.x;
-  i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  float s[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
-  unsigned m = 0;
-  auto take = [&](i64 at, int k) {
-    const float av = a[at];
-    if (!FIRST) s[k] += av * b[at];
-    if (TWO) {
-      u[k] += c[at] * av;
-      const unsigned ab = abs_bits(av);
-      m = ab > m ? ab : m;
-    }
-    if (FIRST) copy[at] = av;
-  };
-  for (; t + 3 * stride < count; t += 4 * stride) {
-    take(t, 0);
-    take(t + stride, 1);
-    take(t + 2 * stride, 2);
-    take(t + 3 * stride, 3);
-  }
-  for (; t < count; t += stride) take(t, 0);
-  if (!FIRST) {
-    const float blk = block_sum_f32((s[0] + s[1]) + (s[2] + s[3]), buf);
-    if (threadIdx.x == 0) part[blockIdx.x] = (double)blk;
-  }
-  if (TWO) {
-    const float blk = block_sum_f32((u[0] + u[1]) + (u[2] + u[3]), buf2);
-    if (threadIdx.x == 0) part[kDotBlocks + blockIdx.x] = (double)blk;
-    block_max_commit(from_bits(m), abits);
-  }
-}
-
-// sum of the block sums of one dot product, rounded as its fixed-point form
-// (2^(E-96), 2^E > max|a| max|b|) holds it; valid in thread 0
-__device__ __forceinline__ double dot_total(const double* __restrict__ part, double* buf, unsigned long long abits,
+// Sum of the block sums of one dot product, rounded as its fixed-point form
+// (2^(E-96), 2^E > max|a| max|b|) holds it; valid in thread 0.  The sums are
+// other blocks': read past L1.
+__device__ __forceinline__ double dot_total(const double* part, double* buf, unsigned long long abits,
                                             unsigned long long bbits) {
   double s = 0.0;
-  for (int q = threadIdx.x; q < kDotBlocks; q += 256) s += part[q];
+  for (int q = threadIdx.x; q < kDotBlocks; q += 256) s += __ldcg(part + q);
   buf[threadIdx.x] = s;
   __syncthreads();
   for (int h = 128; h > 0; h >>= 1) {
@@ -161,30 +122,72 @@ __device__ __forceinline__ double dot_total(const double* __restrict__ part, dou
   return fx_unscale(acc, E);
 }
 
-// STAGE 0: rz = r.z after the first cycle (p = z); 1: alpha = rz / p.q; 2:
-// beta = -(alpha z.q) / rz, rz = r.z.  Clears the maxima that are read here
-// and reduced into next.
+// One pass over the vectors and the scalar they give, by the block that ends
+// last.  STAGE 0, after the first cycle: p = z, rz = r.z; 1: alpha = rz / p.q
+// (a = p, b = q); 2: beta = -(alpha z.q) / rz, rz = r.z (a = z, b = q, c = r).
+// 0 and 2 also take max|z|.  Clears the maxima that are read here and reduced
+// into next.
 template <int STAGE>
-__global__ void __launch_bounds__(256) k_pcg_scalar32(const double* __restrict__ part, PcgDev* P) {
-  __shared__ double buf[256];
-  if (STAGE == 1) {
-    const double pq = dot_total(part, buf, P->pbits, P->qbits);
-    if (threadIdx.x == 0) {
-      P->pq = pq;
-      P->alpha = P->rz / pq;
-      P->rbits = 0;
+__global__ void __launch_bounds__(256) k_pcg_dot(const float* __restrict__ a, const float* __restrict__ b,
+                                                 const float* __restrict__ c, float* __restrict__ p, i64 count,
+                                                 double* part, PcgDev* P) {
+  __shared__ float buf[32], buf2[32];
+  __shared__ double dbuf[256];
+  __shared__ int last;
+  const i64 stride = (i64)gridDim.x * blockDim.x;
+  i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  float s[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
+  unsigned m = 0;
+  auto take = [&](i64 at, int k) {
+    const float av = a[at];
+    if (STAGE != 0) s[k] += av * b[at];
+    if (STAGE != 1) {
+      u[k] += c[at] * av;
+      const unsigned ab = abs_bits(av);
+      m = ab > m ? ab : m;
     }
-    return;
+    if (STAGE == 0) p[at] = av;
+  };
+  for (; t + 3 * stride < count; t += 4 * stride) {
+    take(t, 0);
+    take(t + stride, 1);
+    take(t + 2 * stride, 2);
+    take(t + 3 * stride, 3);
   }
-  const unsigned long long rb = P->rbits, zb = P->zbits, qb = P->qbits;
-  const double zq = STAGE == 2 ? dot_total(part, buf, zb, qb) : 0.0;
-  const double rz = dot_total(part + kDotBlocks, buf, rb, zb);
+  for (; t < count; t += stride) take(t, 0);
+  if (STAGE != 0) {
+    const float blk = block_sum_f32((s[0] + s[1]) + (s[2] + s[3]), buf);
+    if (threadIdx.x == 0) part[blockIdx.x] = (double)blk;
+  }
+  if (STAGE != 1) {
+    const float blk = block_sum_f32((u[0] + u[1]) + (u[2] + u[3]), buf2);
+    if (threadIdx.x == 0) part[kDotBlocks + blockIdx.x] = (double)blk;
+    block_max_commit(from_bits(m), &P->zbits);
+  }
   if (threadIdx.x == 0) {
-    if (STAGE == 2) P->beta = __ddiv_rn(-__dmul_rn(P->alpha, zq), P->rz);
-    P->rz = rz;
-    P->pbits = STAGE == 0 ? zb : 0;
-    P->zbits = 0;
-    P->qbits = 0;
+    __threadfence();
+    last = atomicAdd(&P->arrived, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const unsigned long long rb = __ldcg(&P->rbits), zb = __ldcg(&P->zbits), qb = __ldcg(&P->qbits),
+                           pb = __ldcg(&P->pbits);
+  const double first = STAGE == 0 ? 0.0 : dot_total(part, dbuf, STAGE == 1 ? pb : zb, qb);
+  const double rz = STAGE == 1 ? 0.0 : dot_total(part + kDotBlocks, dbuf, rb, zb);
+  if (threadIdx.x == 0) {
+    P->arrived = 0;
+    if constexpr (STAGE == 1) {
+      P->pq = first;
+      P->alpha = P->rz / first;
+      P->rbits = 0;
+    } else {
+      if (STAGE == 2) P->beta = __ddiv_rn(-__dmul_rn(P->alpha, first), P->rz);
+      P->rz = rz;
+      P->pbits = STAGE == 0 ? zb : 0;
+      P->zbits = 0;
+      P->qbits = 0;
+    }
   }
 }
 
@@ -200,20 +203,17 @@ void launch_pcg_start(PcgDev* P, double bmax, cudaStream_t s) {
 }
 void launch_pcg_first32(float* p, const float* z, const float* r, i64 count, PcgDev* P, double* part,
                         cudaStream_t s) {
-  k_dot_f32_part<true, true><<<kDotBlocks, 256, 0, s>>>(z, nullptr, r, count, part, &P->zbits, p);
-  k_pcg_scalar32<0><<<1, 256, 0, s>>>(part, P);
-  count_launch(2);
+  k_pcg_dot<0><<<kDotBlocks, 256, 0, s>>>(z, nullptr, r, p, count, part, P);
+  count_launch();
 }
 void launch_pcg_alpha32(const float* p, const float* q, i64 count, PcgDev* P, double* part, cudaStream_t s) {
-  k_dot_f32_part<false, false><<<kDotBlocks, 256, 0, s>>>(p, q, nullptr, count, part, nullptr, nullptr);
-  k_pcg_scalar32<1><<<1, 256, 0, s>>>(part, P);
-  count_launch(2);
+  k_pcg_dot<1><<<kDotBlocks, 256, 0, s>>>(p, q, nullptr, nullptr, count, part, P);
+  count_launch();
 }
 void launch_pcg_beta32(const float* z, const float* q, const float* r, i64 count, PcgDev* P, double* part,
                        cudaStream_t s) {
-  k_dot_f32_part<true, false><<<kDotBlocks, 256, 0, s>>>(z, q, r, count, part, &P->zbits, nullptr);
-  k_pcg_scalar32<2><<<1, 256, 0, s>>>(part, P);
-  count_launch(2);
+  k_pcg_dot<2><<<kDotBlocks, 256, 0, s>>>(z, q, r, nullptr, count, part, P);
+  count_launch();
 }
 
 // FP64 residual with fused multiply-adds, for the outer loop of the mixed

@@ -1189,45 +1189,20 @@ void launch_lim_reset(LimDev* st, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// Spectral kernels
+// FFT Poisson correction (the spectral outputs are in mmh_spectral.cu)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double2 spec_mode(double2 x, int kx, int ky, int kz, int n, int mode, const double* ctab) {
-  const double pi = 3.14159265358979323846264338328;
-  double re = x.x, im = x.y;
-  if (mode <= 2) {
-    // cmp * cmplx(0,kk) / n * 2 * pi  (gradient.f90:21,43,65)
-    double kk;
-    if (mode == 0) kk = (double)kx;
-    else if (mode == 1) kk = (ky + 1 <= n / 2 + 1) ? (double)ky : (double)(ky - n);
-    else kk = (kz + 1 <= n / 2 + 1) ? (double)kz : (double)(kz - n);
-    double r2 = re * 0.0 - im * kk;
-    double i2 = re * kk + im * 0.0;
-    r2 = r2 * (1.0 / n) * 2. * pi;  // n is a power of two: exact reciprocal
-    i2 = i2 * (1.0 / n) * 2. * pi;
-    return make_double2(r2, i2);
-  } else if (mode == 3) {
-    // *(k1^2 + k2^2 + k3^2)  (reconstruct.f90:88-110)
-    double k3 = (kz + 1 <= n / 2 + 1) ? (double)kz : (double)(kz - n);
-    k3 = k3 * (1.0 / n) * 2. * pi;
-    double k2 = (ky + 1 <= n / 2 + 1) ? (double)ky : (double)(ky - n);
-    k2 = k2 * (1.0 / n) * 2. * pi;
-    double k1 = (double)kx;
-    k1 = k1 * (1.0 / n) * 2. * pi;
-    double f = k1 * k1 + k2 * k2 + k3 * k3;
-    return make_double2(re * f, im * f);
-  } else {
-    // / (2cos kx + 2cos ky + 2cos kz - 6), DC real part zeroed (limiter.f90:561-576);
-    // ctab[k] = cos(2 pi k / n), the reference's angles (ky + 1 - 1. is ky exactly)
-    double akernel = 2 * ctab[kx] + 2 * ctab[ky] + 2 * ctab[kz] - 6;
-    if (fabs(akernel) < 1e-10) akernel = 1;
-    double r2 = re / akernel, i2 = im / akernel;
-    if (kx == 0 && ky == 0 && kz == 0) r2 = 0.0;
-    return make_double2(r2, i2);
-  }
+// The FFT Poisson correction's symbol: a mode divided by 2cos kx + 2cos ky +
+// 2cos kz - 6, DC real part zeroed (limiter.f90:561-576); ctab[k] = cos(2 pi k
+// / n), the reference's angles (ky + 1 - 1. is ky exactly)
+__device__ __forceinline__ double2 spec_mode(double2 x, int kx, int ky, int kz, const double* ctab) {
+  double akernel = 2 * ctab[kx] + 2 * ctab[ky] + 2 * ctab[kz] - 6;
+  if (fabs(akernel) < 1e-10) akernel = 1;
+  double r2 = x.x / akernel, i2 = x.y / akernel;
+  if (kx == 0 && ky == 0 && kz == 0) r2 = 0.0;
+  return make_double2(r2, i2);
 }
 
-// Tables of the spectral kernels, computed once per context with the same
-// expressions the kernels used: tab[2kx], tab[2kx+1] = cos, sin(-2 pi kx / n)
+// Tables of the correction's kernels, computed once per context: tab[2kx], tab[2kx+1] = cos, sin(-2 pi kx / n)
 // for kx < n/2 (the packing twiddle), tab[n + k] = cos(2 pi k / n).
 __global__ void k_spec_tables(double* tab, int n) {
   const double pi = 3.14159265358979323846264338328;
@@ -1245,9 +1220,9 @@ void launch_spec_tables(double* tab, int n, cudaStream_t s) {
   count_launch();
 }
 
-__global__ void k_spec_pack(const double2* __restrict__ Xc, int n, int mode, double2* __restrict__ Z,
-                            const LimDev* st, const double* __restrict__ tab) {
-  if (mode == 4 && st->ncompress == 0) return;
+__global__ void k_spec_pack(const double2* __restrict__ Xc, int n, double2* __restrict__ Z, const LimDev* st,
+                            const double* __restrict__ tab) {
+  if (st->ncompress == 0) return;
   int M = n / 2, H = M + 1;
   i64 tot = (i64)M * n * n;
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1260,8 +1235,8 @@ __global__ void k_spec_pack(const double2* __restrict__ Xc, int n, int mode, dou
   double2 a = Xc[kx + (i64)H * (ky + (i64)n * kz)];
   double2 b = Xc[kx2 + (i64)H * (ky2 + (i64)n * kz2)];
   const double* ctab = tab + n;
-  double2 A = spec_mode(make_double2(a.x, -a.y), kx, ky, kz, n, mode, ctab);
-  double2 B = spec_mode(make_double2(b.x, -b.y), kx2, ky2, kz2, n, mode, ctab);
+  double2 A = spec_mode(make_double2(a.x, -a.y), kx, ky, kz, ctab);
+  double2 B = spec_mode(make_double2(b.x, -b.y), kx2, ky2, kz2, ctab);
   B.y = -B.y;  // conj
   double wr = tab[2 * kx], wi = tab[2 * kx + 1];
   double sr = A.x + B.x, si = A.y + B.y;
@@ -1271,15 +1246,14 @@ __global__ void k_spec_pack(const double2* __restrict__ Xc, int n, int mode, dou
   Z[t] = make_double2(0.5 * sr - 0.5 * wdi, 0.5 * si + 0.5 * wdr);
 }
 
-void launch_spec_pack(const void* Xc, int n, int mode, void* Z, const LimDev* st, const double* tab, cudaStream_t s) {
+void launch_spec_pack(const void* Xc, int n, void* Z, const LimDev* st, const double* tab, cudaStream_t s) {
   i64 tot = (i64)(n / 2) * n * n;
-  k_spec_pack<<<grid_of(tot, kBlock), kBlock, 0, s>>>((const double2*)Xc, n, mode, (double2*)Z, st, tab);
+  k_spec_pack<<<grid_of(tot, kBlock), kBlock, 0, s>>>((const double2*)Xc, n, (double2*)Z, st, tab);
   count_launch();
 }
 
-__global__ void k_spec_unpack(const double2* __restrict__ z, int n, double* __restrict__ out, int stride_out, int add,
-                              const LimDev* st) {
-  if (add && st->ncompress == 0) return;
+__global__ void k_spec_unpack(const double2* __restrict__ z, int n, double* __restrict__ out, const LimDev* st) {
+  if (st->ncompress == 0) return;
   i64 tot = (i64)(n / 2) * n * n;
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= tot) return;
@@ -1287,19 +1261,13 @@ __global__ void k_spec_unpack(const double2* __restrict__ z, int n, double* __re
   const double rn = 1.0 / n;  // n is a power of two: exact reciprocal
   double a = v.x * 2. * rn * rn * rn;
   double b = v.y * 2. * rn * rn * rn;
-  i64 o0 = 2 * t, o1 = 2 * t + 1;
-  if (add) {
-    out[o0] = out[o0] + a;
-    out[o1] = out[o1] + b;
-  } else {
-    out[o0 * stride_out] = a;
-    out[o1 * stride_out] = b;
-  }
+  out[2 * t] = out[2 * t] + a;
+  out[2 * t + 1] = out[2 * t + 1] + b;
 }
 
-void launch_spec_unpack(const void* z, int n, double* out, int stride_out, int add, const LimDev* st, cudaStream_t s) {
+void launch_spec_unpack(const void* z, int n, double* out, const LimDev* st, cudaStream_t s) {
   i64 tot = (i64)(n / 2) * n * n;
-  k_spec_unpack<<<grid_of(tot, kBlock), kBlock, 0, s>>>((const double2*)z, n, out, stride_out, add, st);
+  k_spec_unpack<<<grid_of(tot, kBlock), kBlock, 0, s>>>((const double2*)z, n, out, st);
   count_launch();
 }
 

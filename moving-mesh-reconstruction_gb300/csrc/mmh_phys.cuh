@@ -114,17 +114,15 @@ __global__ void k_limiter_mask(double* __restrict__ defplim, const double* __res
 // calcdefp RHS: tmp = clip(1 - rho, +-2)/30/dtold (limiter.f90:134-169)
 __global__ void k_calcdefp_rhs(double* __restrict__ tmp, const double* __restrict__ rho, i64 n3, double dtold);
 
-// Spectral stage 1: from the e^{-i} half spectrum Xc = D2Z(x), build the packed
-// complex input Z' of the reference's inverse real FFT applied to
-// mode(X_NR), X_NR = conj(Xc) the e^{+i} spectrum.  mode: 0,1,2 = gradient
-// along x,y,z; 3 = |k|^2 (defp2delta); 4 = division by the 7-point Laplacian
-// symbol (limiter.f90:561-576).
-__global__ void k_spec_pack(const double2* __restrict__ Xc, int n, int mode, double2* __restrict__ Z,
-                            const LimDev* st);
-// Spectral stage 2: x = 2/n^3 * (real samples held pairwise by z); add != 0
-// adds into out (defp += defplim) and is skipped when no cell was limited.
-__global__ void k_spec_unpack(const double2* __restrict__ z, int n, double* __restrict__ out, int stride_out,
-                              int add, const LimDev* st);
+// FFT Poisson correction, stage 1: from the e^{-i} half spectrum Xc = D2Z(x),
+// build the packed complex input Z' of the reference's inverse real FFT applied
+// to X_NR / symbol, X_NR = conj(Xc) the e^{+i} spectrum and the symbol that of
+// the 7-point Laplacian (limiter.f90:561-576).
+__global__ void k_spec_pack(const double2* __restrict__ Xc, int n, double2* __restrict__ Z, const LimDev* st,
+                            const double* __restrict__ tab);
+// Stage 2: out += 2/n^3 * (real samples held pairwise by z).  Both are skipped
+// when no cell was limited.
+__global__ void k_spec_unpack(const double2* __restrict__ z, int n, double* __restrict__ out, const LimDev* st);
 
 // relaxing-TVD (relaxing.f90) for the density component.
 __global__ void k_relax_stage1(const double* __restrict__ rho, const double* __restrict__ def,

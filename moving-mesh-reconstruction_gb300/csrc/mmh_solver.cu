@@ -116,7 +116,8 @@ struct mmh_ctx {
   double *baj = nullptr, *cc = nullptr, *vt = nullptr, *u1 = nullptr, *gface = nullptr;
   // spectral
   void *Xc = nullptr, *Z = nullptr;
-  double* spectab = nullptr;  // twiddle and cosine tables of the spectral kernels
+  double* spectab = nullptr;  // twiddle and cosine tables of the Poisson correction
+  double* linetab = nullptr;  // tables and scratch of the spectral outputs
   double* dotpart = nullptr;  // block sums of the fast FP32 dot products
   cufftHandle pd2z = 0, pz2z = 0;
   bool plans = false;
@@ -819,9 +820,9 @@ int make_plans(mmh_ctx* c) {
 int limiter_poisson(mmh_ctx* c, double* defp, const double* defplim) {
   RET(make_plans(c));
   CKF(cufftExecD2Z(c->pd2z, (cufftDoubleReal*)defplim, (cufftDoubleComplex*)c->Xc));
-  launch_spec_pack(c->Xc, c->n, 4, c->Z, &c->sc->lim, c->spectab, c->s);
+  launch_spec_pack(c->Xc, c->n, c->Z, &c->sc->lim, c->spectab, c->s);
   CKF(cufftExecZ2Z(c->pz2z, (cufftDoubleComplex*)c->Z, (cufftDoubleComplex*)c->Z, CUFFT_FORWARD));
-  launch_spec_unpack(c->Z, c->n, defp, 1, 1, &c->sc->lim, c->s);
+  launch_spec_unpack(c->Z, c->n, defp, &c->sc->lim, c->s);
   return MMH_OK;
 }
 
@@ -898,21 +899,16 @@ int relaxing_dev(mmh_ctx* c, double dt) {
   return MMH_OK;
 }
 
-// spectral outputs of src into host/device buffers (grad: 3 planes of n^3)
+// spectral outputs of src into device buffers (grad: 3 planes of n^3)
 int spectral_outputs(mmh_ctx* c, const double* src, double* d_grad, double* d_delta) {
   Stage stage_("mmh spectral outputs");
-  RET(make_plans(c));
-  CKF(cufftExecD2Z(c->pd2z, (cufftDoubleReal*)src, (cufftDoubleComplex*)c->Xc));
-  for (int ax = 0; ax < 3 && d_grad; ++ax) {
-    launch_spec_pack(c->Xc, c->n, ax, c->Z, &c->sc->lim, c->spectab, c->s);
-    CKF(cufftExecZ2Z(c->pz2z, (cufftDoubleComplex*)c->Z, (cufftDoubleComplex*)c->Z, CUFFT_FORWARD));
-    launch_spec_unpack(c->Z, c->n, d_grad + ax * c->n3, 1, 0, &c->sc->lim, c->s);
+  if (!c->linetab) {
+    const i64 n = c->n;
+    RET(c->alloc(&c->linetab, 4 * n + 2 * n * n));  // tables, then the alternating sums
+    launch_fft_tables(c->linetab, c->n, c->s);
   }
-  if (d_delta) {
-    launch_spec_pack(c->Xc, c->n, 3, c->Z, &c->sc->lim, c->spectab, c->s);
-    CKF(cufftExecZ2Z(c->pz2z, (cufftDoubleComplex*)c->Z, (cufftDoubleComplex*)c->Z, CUFFT_FORWARD));
-    launch_spec_unpack(c->Z, c->n, d_delta, 1, 0, &c->sc->lim, c->s);
-  }
+  launch_spectral_lines(src, c->n, d_grad, d_delta, c->linetab, c->linetab + 4 * (i64)c->n, c->s);
+  CK(cudaGetLastError());
   return MMH_OK;
 }
 
