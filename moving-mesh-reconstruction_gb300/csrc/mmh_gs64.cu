@@ -11,6 +11,9 @@
 // quarter keep the pipe busy.  So:
 //   - a plane is cut into whole rows, not into tiles: there is no halo in x
 //     and every warp instruction has 32 (16 at n = 32) useful lanes;
+//   - the FP64 form's solver keeps, with each metric, the face sums, the
+//     diagonal and its reciprocal (Face64) in place of three coefficient
+//     planes: 54 FP64 instructions per update instead of 69, 51 per residual;
 //   - powers of two are folded (scaling is exact and commutes with rounding):
 //     with S1 = 2 t1, S2 = 4 t2, D = -2 tdiag formed from unhalved face sums,
 //     phi = (rhs dx2 - t1 - t2) / tdiag = -(((rhs 2dx2) - S1) - S2/2) / D;
@@ -46,14 +49,80 @@ namespace {
 // ---------------------------------------------------------------------------
 constexpr int kRowThreads = 256;
 
+__device__ __forceinline__ bool mid_exp(double x) {
+  const int e = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
+  return e > 623 && e < 1423;
+}
+// num / d with y the correctly rounded 1 / d: two corrected steps from num * y
+// (the first gives a faithful quotient, the second then the correctly rounded
+// one, Markstein 1990); away from the middle of the exponent range the
+// division itself.
+__device__ __forceinline__ double div_by(double num, double d, double y) {
+  if (!(mid_exp(d) && mid_exp(num))) return num / d;
+  double q = num * y;
+  q = __fma_rn(__fma_rn(-d, q, num), y, q);
+  return __fma_rn(__fma_rn(-d, q, num), y, q);
+}
+
+// Offsets of a cell's neighbours from its plane's first element
+struct Nbr {
+  i64 c, xp, xm, yp, ym;
+};
+// S1 = 2 t1, S2 = 4 t2 and D = -2 tdiag of one cell; fields as in Face64 (PRE)
+// or the coefficient planes (else), at the cell's plane; phi: in-plane values
+// through P(dx, dy), neighbour planes Kp, Km.
+struct Fields {
+  const double *bx, *by, *bz, *f2, *f3, *f5, *d;  // !PRE: bx, by, bz = f1, f4, f6
+  i64 dkp, dkm;                                   // to the planes above and below
+};
+template <bool PRE, class P>
+__device__ __forceinline__ void sums64(const Fields& f, const Nbr& o, P&& p, const double* __restrict__ Kp,
+                                       const double* __restrict__ Km, double& s1, double& s2, double& d) {
+  double b11p, b11m, b22p, b22m, b33p, b33m;
+  if (PRE) {
+    b11p = f.bx[o.c]; b11m = f.bx[o.xm];
+    b22p = f.by[o.c]; b22m = f.by[o.ym];
+    b33p = f.bz[o.c]; b33m = f.bz[o.c + f.dkm];
+    d = f.d[o.c];
+  } else {
+    const double f1c = f.bx[o.c], f4c = f.by[o.c], f6c = f.bz[o.c];
+    b11p = f.bx[o.xp] + f1c; b11m = f.bx[o.xm] + f1c;
+    b22p = f.by[o.yp] + f4c; b22m = f.by[o.ym] + f4c;
+    b33p = f.bz[o.c + f.dkp] + f6c; b33m = f.bz[o.c + f.dkm] + f6c;
+    d = b11p + b11m + b22p + b22m + b33p + b33m;
+  }
+  s1 = b11p * p(1, 0) + b11m * p(-1, 0) + b22p * p(0, 1) + b22m * p(0, -1) + b33p * Kp[o.c] + b33m * Km[o.c];
+  const double ppk = p(1, 1), mpk = p(-1, 1), pmk = p(1, -1), mmk = p(-1, -1);
+  const double jpkp = Kp[o.yp], jmkp = Kp[o.ym], jpkm = Km[o.yp], jmkm = Km[o.ym];
+  const double ipkp = Kp[o.xp], imkp = Kp[o.xm], ipkm = Km[o.xp], imkm = Km[o.xm];
+  s2 = (ppk - mpk) * f.f2[o.yp] - (pmk - mmk) * f.f2[o.ym] + (ppk - pmk) * f.f2[o.xp] - (mpk - mmk) * f.f2[o.xm] +
+       (jpkp - jmkp) * f.f5[o.c + f.dkp] - (jpkm - jmkm) * f.f5[o.c + f.dkm] + (jpkp - jpkm) * f.f5[o.yp] -
+       (jmkp - jmkm) * f.f5[o.ym] + (ipkp - imkp) * f.f3[o.c + f.dkp] - (ipkm - imkm) * f.f3[o.c + f.dkm] +
+       (ipkp - ipkm) * f.f3[o.xp] - (imkp - imkm) * f.f3[o.xm];
+}
+template <bool PRE>
+__device__ __forceinline__ Fields fields64(const Face64& a, i64 n2, i64 plane, i64 dkp, i64 dkm) {
+  const i64 o = n2 * plane;
+  Fields f;
+  f.bx = a.bx + o; f.by = a.by + o; f.bz = a.bz + o;
+  f.f2 = a.f2 + o; f.f3 = a.f3 + o; f.f5 = a.f5 + o;
+  f.d = PRE ? a.d + o : nullptr;
+  f.dkp = dkp; f.dkm = dkm;
+  return f;
+}
+// the coefficient planes themselves
+Face64 raw64(const double* coef, i64 n3) {
+  return Face64{coef, coef + 3 * n3, coef + 5 * n3, coef + n3, coef + 2 * n3, coef + 4 * n3, nullptr, nullptr};
+}
+
+template <bool PRE>
 __global__ void __launch_bounds__(kRowThreads, 2) k_gs_rows(const double* __restrict__ src,
                                                             const double* __restrict__ nbr, double* __restrict__ dst,
-                                                            const double* __restrict__ rhs,
-                                                            const double* __restrict__ coef, int lgn, int ty,
+                                                            const double* __restrict__ rhs, Face64 co, int lgn, int ty,
                                                             double dx2x2, int kpar) {
   extern __shared__ double sp[];
   const int n = 1 << lgn, h = n >> 1, lgh = lgn - 1;
-  const i64 n2 = (i64)n << lgn, n3 = n2 << lgn;
+  const i64 n2 = (i64)n << lgn;
   const int y0 = blockIdx.x * ty, k = 2 * blockIdx.y + kpar;
   const int kp = wp(k, n), km = wm(k, n);
   const double* own = src + n2 * k;
@@ -65,13 +134,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_gs_rows(const double* __rest
   __syncthreads();
   const double* Kp = nbr + n2 * kp;
   const double* Km = nbr + n2 * km;
-  const double* f1 = coef + n2 * k;
-  const double* f2 = f1 + n3;
-  const double* f4 = f1 + 3 * n3;
-  const double* f3 = f1 + 2 * n3;
-  const double* f5 = f1 + 4 * n3;
-  const double* f6 = f1 + 5 * n3;
-  const i64 dkp = n2 * (kp - k), dkm = n2 * (km - k);
+  const Fields f = fields64<PRE>(co, n2, k, n2 * (kp - k), n2 * (km - k));
+  const double* rk = rhs + n2 * k;
+  const double* yk = PRE ? co.y + n2 * k : nullptr;
 #pragma unroll 1
   for (int q = 0; q < 4; ++q) {
     const int io = q >> 1;
@@ -81,29 +146,16 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_gs_rows(const double* __rest
       const int m = e & (h - 1), yl = q - 2 + 2 * (e >> lgh);  // row relative to y0
       const int x = 2 * m + io, xp = (x + 1) & (n - 1), xm = (x - 1) & (n - 1);
       const int y = (y0 + yl) & (n - 1), yp = (y + 1) & (n - 1), ym = (y - 1) & (n - 1);
-      const i64 r0 = (i64)y << lgn, rp = (i64)yp << lgn, rm = (i64)ym << lgn;
-      const i64 c = r0 + x, cxp = r0 + xp, cxm = r0 + xm, cyp = rp + x, cym = rm + x;
-      // face sums (twice the face coefficients) and the diagonal
-      const double f1c = f1[c], f4c = f4[c], f6c = f6[c];
-      const double b11p = f1[cxp] + f1c, b11m = f1[cxm] + f1c;
-      const double b22p = f4[cyp] + f4c, b22m = f4[cym] + f4c;
-      const double b33p = f6[c + dkp] + f6c, b33m = f6[c + dkm] + f6c;
-      const double d = b11p + b11m + b22p + b22m + b33p + b33m;
+      const i64 r0 = (i64)y << lgn;
+      const Nbr o{r0 + x, r0 + xp, r0 + xm, ((i64)yp << lgn) + x, ((i64)ym << lgn) + x};
       // phi of the plane: rows yl+2 .. yl+4 of the tile, x+-1 in the other half
       const double* s0 = sp + ((yl + 3) << lgn);
-      const double* sP = s0 + n;
-      const double* sM = s0 - n;
       const int oc = io * h + m, op = (xp & 1) * h + (xp >> 1), om = (xm & 1) * h + (xm >> 1);
-      const double s1 = b11p * s0[op] + b11m * s0[om] + b22p * sP[oc] + b22m * sM[oc] + b33p * Kp[c] + b33m * Km[c];
-      const double ppk = sP[op], mpk = sP[om], pmk = sM[op], mmk = sM[om];
-      const double jpkp = Kp[cyp], jmkp = Kp[cym], jpkm = Km[cyp], jmkm = Km[cym];
-      const double ipkp = Kp[cxp], imkp = Kp[cxm], ipkm = Km[cxp], imkm = Km[cxm];
-      const double s2 = (ppk - mpk) * f2[cyp] - (pmk - mmk) * f2[cym] + (ppk - pmk) * f2[cxp] - (mpk - mmk) * f2[cxm] +
-                        (jpkp - jmkp) * f5[c + dkp] - (jpkm - jmkm) * f5[c + dkm] + (jpkp - jpkm) * f5[cyp] -
-                        (jmkp - jmkm) * f5[cym] + (ipkp - imkp) * f3[c + dkp] - (ipkm - imkm) * f3[c + dkm] +
-                        (ipkp - ipkm) * f3[cxp] - (imkp - imkm) * f3[cxm];
-      const double num = __fma_rn(-0.5, s2, rhs[n2 * k + c] * dx2x2 - s1);
-      sp[((yl + 3) << lgn) + oc] = -(num / d);
+      double s1, s2, d;
+      sums64<PRE>(
+          f, o, [&](int dx, int dy) { return s0[dy * n + (dx > 0 ? op : dx < 0 ? om : oc)]; }, Kp, Km, s1, s2, d);
+      const double num = __fma_rn(-0.5, s2, rk[o.c] * dx2x2 - s1);
+      sp[((yl + 3) << lgn) + oc] = -(PRE ? div_by(num, d, yk[o.c]) : num / d);
     }
     __syncthreads();
   }
@@ -114,6 +166,65 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_gs_rows(const double* __rest
   }
 }
 
+// MODE 0: r = rhs - L[phi] (r may be null), max|r|; 1: r = L[phi], max|r| --
+// calcresid's operations (gauss1.f90:683-709) from the face sums.  One cell per
+// thread straight from global memory: the FP64 pipe takes ten times as long as
+// the loads.
+template <int MODE>
+__global__ void __launch_bounds__(256) k_op64(const double* __restrict__ phi, const double* __restrict__ rhs,
+                                              Face64 co, int lgn, double hdi2, double* __restrict__ r,
+                                              unsigned long long* maxbits) {
+  const int n = 1 << lgn;
+  const i64 n2 = (i64)n << lgn, t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  double v = 0.0;
+  if (t < n2 << lgn) {
+    const int x = (int)t & (n - 1), y = (int)(t >> lgn) & (n - 1), k = (int)(t >> (2 * lgn));
+    const int kp = wp(k, n), km = wm(k, n), xp = wp(x, n), xm = wm(x, n);
+    const i64 r0 = (i64)y << lgn, rp = (i64)wp(y, n) << lgn, rm = (i64)wm(y, n) << lgn;
+    const Nbr o{r0 + x, r0 + xp, r0 + xm, rp + x, rm + x};
+    const double* P = phi + n2 * k;
+    const double* rows[3] = {P + rm, P + r0, P + rp};
+    double s1, s2, d;
+    sums64<true>(
+        fields64<true>(co, n2, k, n2 * (kp - k), n2 * (km - k)), o,
+        [&](int dx, int dy) { return rows[dy + 1][dx > 0 ? xp : dx < 0 ? xm : x]; }, phi + n2 * kp, phi + n2 * km, s1,
+        s2, d);
+    // t1 + t2 + tdiag phi = half of (S1 + S2/2) - D phi
+    v = (__fma_rn(0.5, s2, s1) - d * P[o.c]) * hdi2;
+    if (MODE == 0) v = rhs[t] - v;
+    if (r) r[t] = v;
+    v = fabs(v);
+  }
+  if (maxbits) block_max_commit(v, maxbits);
+}
+
+// out = f + f one cell up along the axis
+__global__ void k_face_sum(const double* __restrict__ f, int n, int axis, double* __restrict__ out) {
+  const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x, n3 = (i64)n * n * n;
+  if (t >= n3) return;
+  int c[3];
+  cell_of(t, n, c[0], c[1], c[2]);
+  const i64 st = axis == 0 ? 1 : (axis == 1 ? (i64)n : (i64)n * n);
+  out[t] = f[c[axis] == n - 1 ? t - (n - 1) * st : t + st] + f[t];
+}
+// d = sum of the six face sums in relaxplane's order, y = 1 / d
+__global__ void k_face_diag(const double* __restrict__ bx, const double* __restrict__ by,
+                            const double* __restrict__ bz, int n, double* __restrict__ d, double* __restrict__ y) {
+  const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x, n3 = (i64)n * n * n;
+  if (t >= n3) return;
+  int i, j, k;
+  cell_of(t, n, i, j, k);
+  const double v = bx[t] + bx[IDX(wm(i, n), j, k, n)] + by[t] + by[IDX(i, wm(j, n), k, n)] + bz[t] +
+                   bz[IDX(i, j, wm(k, n), n)];
+  d[t] = v;
+  y[t] = 1.0 / v;
+}
+
+int lg(int n) {
+  int l = 0;
+  while ((1 << l) < n) ++l;
+  return l;
+}
 int rows_ty(int n) { return n == 32 ? 8 : (n == 64 || n > 512 ? 16 : 32); }
 
 // ---------------------------------------------------------------------------
@@ -128,8 +239,7 @@ int rows_ty(int n) { return n == 32 ? 8 : (n == 64 || n > 512 ? 16 : 32); }
 // what counts.  The products of an update (12 cross terms, 6 faces) each have
 // a lane of their own, and only the two sums, in the reference's order, are
 // serial.  The division uses the correctly rounded reciprocal of the diagonal
-// (formed once per launch): two corrected steps give the correctly rounded
-// quotient (Markstein 1990; the second step starts from a faithful quotient).
+// (formed once per launch, div_by).
 // Colour p = 4k + 2i + j reads, among the cells updated one phase before it,
 //   p = 1, 3, 5, 7: its y neighbours (two face products);
 //   p = 2, 6: its xy diagonals (the first four cross terms);
@@ -157,12 +267,17 @@ struct BoxGeom {
 __device__ __forceinline__ void bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
+// address of a shared variable in CTA `rank` of the cluster, and a store to it
+__device__ __forceinline__ unsigned mapa(unsigned addr, int rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_cluster(unsigned addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
 __device__ __forceinline__ void bar_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-__device__ __forceinline__ bool mid_exp(double x) {
-  const int e = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
-  return e > 623 && e < 1423;
 }
 
 template <int N>
@@ -243,11 +358,56 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
 #pragma unroll
     for (int p = 0; p < 8; ++p) fc[p] = face_coef(fterm, p);
   }
+  // Warp F's stores of an updated cell: itself and, when it lies on the box's
+  // surface, its copies in the neighbours' halos (faces and edges).  A colour
+  // lies on the lower side of an axis where its parity is 0, on the upper one
+  // where it is 1; ok[s] has a bit per colour for set s of axes.  CC = 8: the
+  // four groups of 8 lanes hold the same cells and share the seven stores (two
+  // at most per lane); CC = 32: a lane makes all of its own.
+  constexpr int NS = CC == 8 ? 2 : 6;
+  unsigned ok_[NS], base_[NS][G::GZ > 2 ? 2 : 1];
+  int shift_[CC == 8 ? 2 : 1][3];
+  const unsigned here = (unsigned)__cvta_generic_to_shared(sp);
+  auto axes_ok = [&](int set) {
+    unsigned m = 0;
+    for (int p = 0; p < 8; ++p) {
+      const bool sx = ((p >> 1) & 1) ? a == G::BX / 2 - 1 : a == 0;
+      const bool sy = (p & 1) ? b == G::BY / 2 - 1 : b == 0;
+      const bool sz = (p >> 2) ? d == G::BZ / 2 - 1 : d == 0;
+      if ((!(set & 1) || sx) && (!(set & 2) || sy) && (!(set & 4) || sz)) m |= 1u << p;
+    }
+    return m;
+  };
+  auto target = [&](int set, int uz) {  // the neighbour along the axes of the set (z: uz = -1 or 1)
+    const int r = (bx + (set & 1)) % G::GX + G::GX * ((by + ((set >> 1) & 1)) % G::GY +
+                                                     G::GY * ((bz + ((set >> 2) & 1) * (uz + G::GZ)) % G::GZ));
+    return mapa(here, r);
+  };
+  if (CC == 8) {
+    // sets by lane group: {own, xy}, {x, yz}, {y, xz}, {z, -}
+    const int g = lane >> 3;
+    const int set[2] = {g == 0 ? 0 : g == 1 ? 1 : g == 2 ? 2 : 4, g == 0 ? 3 : g == 1 ? 6 : 5};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      ok_[s] = (s == 1 && g == 3) ? 0u : axes_ok(set[s]);
+      base_[s][0] = target(set[s], 1);  // GX = GY = GZ = 1 or 2: either sign is the same box
+      shift_[s][0] = (set[s] & 1) ? G::BX : 0;
+      shift_[s][1] = (set[s] & 2) ? G::BY * SX : 0;
+      shift_[s][2] = (set[s] & 4) ? G::BZ * SXY : 0;
+    }
+  } else {
+    constexpr int sets[6] = {1, 2, 3, 4, 5, 6};
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      ok_[s] = axes_ok(sets[s]);
+      base_[s][0] = target(sets[s], -1);
+      if (G::GZ > 2) base_[s][G::GZ > 2 ? 1 : 0] = target(sets[s], 1);
+    }
+  }
   // warp F: diagonal, its reciprocal and the lower y face sum per colour
   double(&X2)[8] = xc;
   double(&yp)[8] = fc;
   double D[8], Y[8], ym[8];
-  unsigned ok = 0;
   if (warp == 0) {
 #pragma unroll
     for (int p = 0; p < 8; ++p) {
@@ -257,7 +417,6 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
       ym[p] = face_coef(3, p);
       D[p] = face_coef(0, p) + face_coef(1, p) + yp[p] + ym[p] + face_coef(4, p) + face_coef(5, p);
       Y[p] = 1.0 / D[p];
-      if (mid_exp(D[p])) ok |= 1u << p;
     }
   }
   if (tid == 0) stop = 0;
@@ -347,37 +506,25 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
           s1 = s1 + f[5][cell];
           s2 = sum2[p & 1][cell];
         }
-        const double num = __fma_rn(-0.5, s2, X2[p] - s1);
-        double v;
-        if ((ok >> p & 1u) && mid_exp(num)) {
-          const double y = Y[p], dd = D[p];
-          double q = num * y;
-          q = __fma_rn(__fma_rn(-dd, q, num), y, q);
-          q = __fma_rn(__fma_rn(-dd, q, num), y, q);
-          v = -q;
-        } else {
-          v = -(num / D[p]);
-        }
+        const double v = -div_by(__fma_rn(-0.5, s2, X2[p] - s1), D[p], Y[p]);
         if (N == 4) changed = changed || __double_as_longlong(v) != __double_as_longlong(sp[c]);
-        // the cell, and its copies in the neighbours' halos: faces and edges
         const int i = (p >> 1) & 1, j = p & 1, kz = p >> 2;
-        const int sx = i == 0 ? (a == 0 ? -1 : 0) : (a == G::BX / 2 - 1 ? 1 : 0);
-        const int sy = j == 0 ? (b == 0 ? -1 : 0) : (b == G::BY / 2 - 1 ? 1 : 0);
-        const int sz = kz == 0 ? (d == 0 ? -1 : 0) : (d == G::BZ / 2 - 1 ? 1 : 0);
-        auto push = [&](int ux, int uy, int uz) {
-          const int r = (bx + ux + G::GX) % G::GX +
-                        G::GX * ((by + uy + G::GY) % G::GY + G::GY * ((bz + uz + G::GZ) % G::GZ));
-          double* w = (G::CL == 1 || r == rank) ? sp : cl.map_shared_rank(sp, r);
-          w[c - ux * G::BX - uy * G::BY * SX - uz * G::BZ * SXY] = v;
-        };
-        if (CC == 32 || lane < 8) {
+        if (CC == 8) {
+#pragma unroll
+          for (int s = 0; s < 2; ++s)
+            if (ok_[s] >> p & 1u)
+              st_cluster(base_[s][0] + 8u * (c + (i ? -shift_[s][0] : shift_[s][0]) +
+                                             (j ? -shift_[s][1] : shift_[s][1]) + (kz ? -shift_[s][2] : shift_[s][2])),
+                         v);
+        } else {
+          constexpr int sets[6] = {1, 2, 3, 4, 5, 6};
           sp[c] = v;
-          if (sx) push(sx, 0, 0);
-          if (sy) push(0, sy, 0);
-          if (sz) push(0, 0, sz);
-          if (sx && sy) push(sx, sy, 0);
-          if (sy && sz) push(0, sy, sz);
-          if (sx && sz) push(sx, 0, sz);
+#pragma unroll
+          for (int s = 0; s < NS; ++s) {
+            const int off = ((sets[s] & 1) ? (i ? -G::BX : G::BX) : 0) + ((sets[s] & 2) ? (j ? -1 : 1) * G::BY * SX : 0) +
+                            ((sets[s] & 4) ? (kz ? -1 : 1) * G::BZ * SXY : 0);
+            if (ok_[s] >> p & 1u) st_cluster(base_[s][(sets[s] & 4) && G::GZ > 2 ? kz : 0] + 8u * (c + off), v);
+          }
         }
         if (N == 4 && p == 7) {
           const bool any = __any_sync(0xffffffffu, changed);
@@ -422,10 +569,10 @@ void box_launch(double* phi, const double* rhs, const double* coef, double dx2, 
 
 }  // namespace
 
-// nsweeps FP64 8-colour sweeps of phi on an n^3 grid; scratch: n^3 doubles
-// (n >= 32).  Returns the buffer that holds the swept field.
-double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
-                           double* scratch, cudaStream_t s) {
+namespace {
+// faces: the coefficients' face sums (null: the coefficient planes themselves)
+double* gs64_sweeps(double* phi, const double* rhs, const double* coef, const Face64* faces, int n, double dx,
+                    int nsweeps, double* scratch, cudaStream_t s) {
   if (nsweeps <= 0) return phi;
   const i64 h3 = (i64)(n / 2) * (n / 2) * (n / 2);
   const double dx2 = dx * dx;
@@ -438,24 +585,68 @@ double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, i
     count_launch();
     return phi;
   }
-  int lgn = 0;
-  while ((1 << lgn) < n) ++lgn;
-  const int ty = rows_ty(n), smem = (int)(sizeof(double) * (ty + 7) * n);
-  static std::atomic<unsigned long long> attr_done{0};
-  smem_attr_once(k_gs_rows, 8 * 23 * 1024, attr_done);  // the largest of any size
+  const int lgn = lg(n), ty = rows_ty(n), smem = (int)(sizeof(double) * (ty + 7) * n);
+  static std::atomic<unsigned long long> d0{0}, d1{0};
+  smem_attr_once(k_gs_rows<false>, 8 * 23 * 1024, d0);  // the largest of any size
+  smem_attr_once(k_gs_rows<true>, 8 * 23 * 1024, d1);
+  const Face64 f = faces ? *faces : raw64(coef, 8 * h3);
   // double buffer: a sweep reads a and leaves the swept field in b
   double *a = phi, *b = scratch;
   for (int sw = 0; sw < nsweeps; ++sw) {
     for (int kpar = 0; kpar < 2; ++kpar) {
+      const dim3 grid(n / ty, n / 2);
       prof_begin(KK_GS, s, 4 * h3, n);
-      k_gs_rows<<<dim3(n / ty, n / 2), kRowThreads, smem, s>>>(a, kpar == 0 ? a : b, b, rhs, coef, lgn, ty, 2.0 * dx2,
-                                                               kpar);
+      if (faces)
+        k_gs_rows<true><<<grid, kRowThreads, smem, s>>>(a, kpar == 0 ? a : b, b, rhs, f, lgn, ty, 2.0 * dx2, kpar);
+      else
+        k_gs_rows<false><<<grid, kRowThreads, smem, s>>>(a, kpar == 0 ? a : b, b, rhs, f, lgn, ty, 2.0 * dx2, kpar);
       prof_end(KK_GS, s, n);
       count_launch();
     }
     std::swap(a, b);
   }
   return a;
+}
+}  // namespace
+
+// nsweeps FP64 8-colour sweeps of phi on an n^3 grid; scratch: n^3 doubles
+// (n >= 32).  Returns the buffer that holds the swept field.
+double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
+                           double* scratch, cudaStream_t s) {
+  return gs64_sweeps(phi, rhs, coef, nullptr, n, dx, nsweeps, scratch, s);
+}
+double* launch_gs64_sweeps(double* phi, const double* rhs, const Face64& f, int n, double dx, int nsweeps,
+                           double* scratch, cudaStream_t s) {
+  return gs64_sweeps(phi, rhs, nullptr, &f, n, dx, nsweeps, scratch, s);
+}
+
+Face64 launch_faces64(double* coef, int n, double* s0, double* s1, cudaStream_t s) {
+  const i64 n3 = (i64)n * n * n;
+  const unsigned g = (unsigned)((n3 + 255) / 256);
+  // each pass frees the plane the next one writes
+  k_face_sum<<<g, 256, 0, s>>>(coef, n, 0, s0);
+  k_face_sum<<<g, 256, 0, s>>>(coef + 3 * n3, n, 1, coef);
+  k_face_sum<<<g, 256, 0, s>>>(coef + 5 * n3, n, 2, coef + 3 * n3);
+  k_face_diag<<<g, 256, 0, s>>>(s0, coef, coef + 3 * n3, n, coef + 5 * n3, s1);
+  count_launch(4);
+  return Face64{s0, coef, coef + 3 * n3, coef + n3, coef + 2 * n3, coef + 4 * n3, coef + 5 * n3, s1};
+}
+
+void launch_residual64(const double* phi, const double* rhs, const Face64& f, int n, double dx, double* r,
+                       unsigned long long* maxbits, cudaStream_t s) {
+  const i64 n3 = (i64)n * n * n;
+  prof_begin(KK_RESIDUAL, s, n3, n);
+  k_op64<0><<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(phi, rhs, f, lg(n), 0.5 * (1.0 / (dx * dx)), r, maxbits);
+  prof_end(KK_RESIDUAL, s, n);
+  count_launch();
+}
+void launch_apply64(const double* p, const Face64& f, int n, double dx, double* q, unsigned long long* qbits,
+                    cudaStream_t s) {
+  const i64 n3 = (i64)n * n * n;
+  prof_begin(KK_APPLY, s, n3, n);
+  k_op64<1><<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(p, nullptr, f, lg(n), 0.5 * (1.0 / (dx * dx)), q, qbits);
+  prof_end(KK_APPLY, s, n);
+  count_launch();
 }
 
 }  // namespace mmh

@@ -41,6 +41,22 @@ template <class T> T* launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int 
 // the FP64 sweeps of launch_gs_sweeps (mmh_gs64.cu)
 double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
                            double* scratch, cudaStream_t s);
+// The FP64 form's operator on grids of 32^3 and up: sums of coefficients 1, 4,
+// 6 at a cell and the next one along their axis (twice the upper face's
+// coefficient), coefficients 2, 3, 5, the sum of the six face sums (-2 times
+// the diagonal) and its reciprocal.
+struct Face64 {
+  const double *bx, *by, *bz, *f2, *f3, *f5, *d, *y;
+};
+// from the six coefficient planes, three of which it overwrites; s0, s1: n^3 each
+Face64 launch_faces64(double* coef, int n, double* s0, double* s1, cudaStream_t s);
+double* launch_gs64_sweeps(double* phi, const double* rhs, const Face64& f, int n, double dx, int nsweeps,
+                           double* scratch, cudaStream_t s);
+// launch_residual<double> and launch_apply<double> from the face sums (the same bits)
+void launch_residual64(const double* phi, const double* rhs, const Face64& f, int n, double dx, double* r,
+                       unsigned long long* maxbits, cudaStream_t s);
+void launch_apply64(const double* p, const Face64& f, int n, double dx, double* q, unsigned long long* qbits,
+                    cudaStream_t s);
 // FP32 plane-kernel tile autotuning: the shape pinned for every grid (-1:
 // timed per grid size and device), and the shape chosen for n (-1: none yet)
 constexpr int kGsShapes = 6;

@@ -106,6 +106,11 @@ struct mmh_ctx {
   // FP64 hierarchy; level 0 u = defp, rhs = tmp
   Hier<double> h64;
   std::vector<double*> defl, rhol;
+  // FP64 form: the operator of the levels from 32^3 up as face sums (made from
+  // the coefficient planes with each metric), and their two extra planes
+  std::vector<Face64> face;
+  std::vector<double*> face0, face1;
+  bool faces_at(int l) const { return cfg.precision == MMH_FP64 && nl[l] >= 32; }
   // FP32 hierarchy (mixed)
   Hier<float> h32;
   // flexible PCG vectors (solution, right-hand side, search direction, L p);
@@ -216,10 +221,21 @@ int relax_level(mmh_ctx* c, int l, T*& u, T*& r, int nrelax, int mode, unsigned 
   Hier<T>& H = hier<T>(c);
   int n = c->nl[l];
   T dx = T(double(1 << l));
-  if (launch_gs_sweeps<T>(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s, zero_init) != u) std::swap(u, r);
+  bool done = false;
+  if constexpr (std::is_same<T, double>::value) {
+    if (c->faces_at(l)) {
+      if (launch_gs64_sweeps(u, H.rhs[l], c->face[l], n, dx, nrelax, r, c->s) != u) std::swap(u, r);
+      done = true;
+    }
+  }
+  if (!done && launch_gs_sweeps<T>(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s, zero_init) != u) std::swap(u, r);
   if (mode == 0) return MMH_OK;
   if (maxslot) CK(cudaMemsetAsync(maxslot, 0, 8, c->s));
-  launch_residual<T>(u, H.rhs[l], H.coef[l], n, dx, mode == 3 ? r : (T*)nullptr, nullptr, maxslot, c->s);
+  T* res = mode == 3 ? r : nullptr;
+  if constexpr (std::is_same<T, double>::value) {
+    if (done) launch_residual64(u, H.rhs[l], c->face[l], n, dx, res, maxslot, c->s);
+  }
+  if (!done) launch_residual<T>(u, H.rhs[l], H.coef[l], n, dx, res, nullptr, maxslot, c->s);
   if (mode == 3) launch_restrict_resid<T>(r, n, special_plane(nrelax, n), H.rhs[l + 1], c->s);
   return MMH_OK;
 }
@@ -373,6 +389,7 @@ int build_levels(mmh_ctx* c, int l0) {
     launch_metric<double>(c->defl[l], c->rhol[l], n, double(1 << l), c->h64.coef[l], c->s,
                           c->cfg.precision == MMH_MIXED);
     if (c->cfg.precision == MMH_MIXED) launch_d2f(c->h64.coef[l], c->h32.coef[l], 6 * (i64)n * n * n, c->s);
+    if (c->faces_at(l)) c->face[l] = launch_faces64(c->h64.coef[l], n, c->face0[l], c->face1[l], c->s);
   }
   if (c->coarse_inv && c->nl[c->nlev - 1] == 4)
     launch_coarse_inverse(c->h64.coef[c->nlev - 1], double(1 << (c->nlev - 1)), c->coarse_inv, c->s);
@@ -433,6 +450,17 @@ int precond_replay(mmh_ctx* c, int l0) {
   return MMH_OK;
 }
 
+// r = b - L x and q = L p of the FP64 form on level l, max|.| into maxbits
+void residual64(mmh_ctx* c, int l, double dx, const double* x, const double* b, double* r,
+                unsigned long long* maxbits) {
+  if (c->faces_at(l)) launch_residual64(x, b, c->face[l], c->nl[l], dx, r, maxbits, c->s);
+  else launch_residual<double>(x, b, c->h64.coef[l], c->nl[l], dx, r, nullptr, maxbits, c->s);
+}
+void apply64(mmh_ctx* c, int l, double dx, const double* p, double* q, unsigned long long* qbits) {
+  if (c->faces_at(l)) launch_apply64(p, c->face[l], c->nl[l], dx, q, qbits, c->s);
+  else launch_apply<double>(p, c->h64.coef[l], c->nl[l], dx, q, qbits, c->s);
+}
+
 // Flexible preconditioned conjugate gradients on L x = b at level l0 in
 // precision T, one V-cycle per iteration as preconditioner, until
 // max|r| <= tol * bn (recurrence residual) or maxit iterations.  The residual
@@ -446,7 +474,7 @@ int pcg_core64(mmh_ctx* c, int l0, double dx, double* x, const double* b, double
   PcgDev* P = &c->sc->pcg;
   double* r = H.rhs[l0];
   CK(cudaMemsetAsync(P, 0, sizeof(PcgDev), c->s));
-  launch_residual<double>(x, b, H.coef[l0], n, dx, r, nullptr, &P->rbits, c->s);
+  residual64(c, l0, dx, x, b, r, &P->rbits);
   RET(pull_scal(c));
   const double rmax0 = bits_to_double(c->hsc->pcg.rbits);
   double rel = rmax0 / bn;
@@ -469,7 +497,7 @@ int pcg_core64(mmh_ctx* c, int l0, double dx, double* x, const double* b, double
     launch_pcg_scalar(P, 0, c->s);
     for (it = 1;; ++it) {
       CK(cudaMemsetAsync(&P->qbits, 0, 8, c->s));
-      launch_apply<double>(p, H.coef[l0], n, dx, q, &P->qbits, c->s);
+      apply64(c, l0, dx, p, q, &P->qbits);
       CK(cudaMemsetAsync(P->acc[1], 0, 16, c->s));
       launch_dot(p, q, n3, &P->pbits, &P->qbits, P->acc[1], c->s);
       launch_pcg_scalar(P, 1, c->s);
@@ -561,7 +589,7 @@ int true_residual(mmh_ctx* c, int l0, double dx, const double* x, const double* 
   if (c->cfg.precision == MMH_MIXED)
     launch_residual_fma(x, b, c->h64.coef[l0], n, dx, r32, &c->sc->resbits, c->s);
   else
-    launch_residual<double>(x, b, c->h64.coef[l0], n, dx, nullptr, r32, &c->sc->resbits, c->s);
+    residual64(c, l0, dx, x, b, nullptr, &c->sc->resbits);
   RET(pull_scal(c));
   *rmax = bits_to_double(c->hsc->resbits);
   return MMH_OK;
@@ -1478,9 +1506,6 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
     c->own_stream = true;
   }
   int rc = MMH_OK;
-  auto A = [&](auto** p, i64 count) {
-    if (rc == MMH_OK) rc = c->alloc(p, count);
-  };
   i64 n3 = c->n3;
   // Scratch that is dead while relaxing runs (finest-level multigrid scratch,
   // limiter and spectral buffers, PCG vectors) shares one allocation with the
@@ -1490,7 +1515,8 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
     void** p;
     size_t bytes;
   };
-  std::vector<Piece> shared;
+  std::vector<Piece> own, shared;
+  auto A = [&](auto** p, i64 count) { own.push_back({(void**)p, sizeof(**p) * (size_t)count}); };
   auto S = [&](auto** p, i64 count) { shared.push_back({(void**)p, sizeof(**p) * (size_t)count}); };
   A(&c->def, n3);
   A(&c->rho, n3);
@@ -1510,13 +1536,25 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
     if (l == 0) {
       S(&c->h64.coef[l], 6 * m3);
       S(&c->h64.r[l], m3);
-      c->defl[0] = c->def;
-      c->rhol[0] = c->rho;
     } else {
       A(&c->h64.coef[l], 6 * m3);
       A(&c->h64.r[l], m3);
       A(&c->defl[l], m3);
       A(&c->rhol[l], m3);
+    }
+  }
+  c->face.resize(c->nlev);
+  c->face0.resize(c->nlev);
+  c->face1.resize(c->nlev);
+  for (int l = 0; l < c->nlev; ++l) {
+    if (!c->faces_at(l)) continue;
+    i64 m3 = (i64)c->nl[l] * c->nl[l] * c->nl[l];
+    if (l == 0) {
+      S(&c->face0[l], m3);
+      S(&c->face1[l], m3);
+    } else {
+      A(&c->face0[l], m3);
+      A(&c->face1[l], m3);
     }
   }
   if (cfg->precision == MMH_MIXED) {
@@ -1554,19 +1592,32 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
   }
   S((double**)&c->Xc, 2 * (i64)(n / 2 + 1) * n * n);
   S((double**)&c->Z, 2 * (i64)(n / 2) * n * n);
+  if (cfg->precision == MMH_MIXED) A(&c->dotpart, 2 * kDotBlocks);
+  A(&c->sc, 1);
   {
+    // every buffer of the context in one allocation: some fifty calls to the
+    // allocator were most of what creating and destroying a small context cost
     const size_t align = 256;
-    size_t total = 0;
-    for (const Piece& q : shared) total += (q.bytes + align - 1) / align * align;
+    auto up = [&](size_t bytes) { return (bytes + align - 1) / align * align; };
+    size_t total = 0, sum = 0;
+    for (const Piece& q : shared) total += up(q.bytes);
+    for (const Piece& q : own) sum += up(q.bytes);
     const size_t relax_bytes = sizeof(double) * 18 * (size_t)n3;  // baj 7, cc 1, sd 6, faces 3, u1 1
     double* arena = nullptr;
-    A(&arena, (i64)((std::max(total, relax_bytes) + sizeof(double) - 1) / sizeof(double)));
+    rc = c->alloc(&arena, (i64)((up(std::max(total, relax_bytes)) + sum + sizeof(double) - 1) / sizeof(double)));
     if (rc == MMH_OK) {
       char* at = reinterpret_cast<char*>(arena);
       for (const Piece& q : shared) {
         *q.p = at;
-        at += (q.bytes + align - 1) / align * align;
+        at += up(q.bytes);
       }
+      at = reinterpret_cast<char*>(arena) + up(std::max(total, relax_bytes));
+      for (const Piece& q : own) {
+        *q.p = at;
+        at += up(q.bytes);
+      }
+      c->defl[0] = c->def;
+      c->rhol[0] = c->rho;
       c->baj = arena;
       c->cc = arena + 7 * n3;
       c->vt = arena + 8 * n3;  // half sums and differences of the relaxing fluxes
@@ -1574,8 +1625,6 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
       c->u1 = arena + 17 * n3;
     }
   }
-  if (cfg->precision == MMH_MIXED) A(&c->dotpart, 2 * kDotBlocks);
-  A(&c->sc, 1);
   if (rc == MMH_OK && cudaMallocHost((void**)&c->hsc, sizeof(Scal)) != cudaSuccess) rc = MMH_ERR_NOMEM;
   if (rc == MMH_OK && cudaMemsetAsync(c->sc, 0, sizeof(Scal), c->s) != cudaSuccess) rc = MMH_ERR_CUDA;
   if (rc == MMH_OK) {
