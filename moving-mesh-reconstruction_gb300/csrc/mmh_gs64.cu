@@ -248,8 +248,6 @@ int rows_ty(int n) { return n == 32 ? 8 : (n == 64 || n > 512 ? 16 : 32); }
 // products of phase p + 1 that do not depend on p and sum its cross terms
 // (warp S): a phase costs 13, 13, 20, 13 dependent FP64 instructions instead
 // of some 75 (64 cycles each).
-// A whole sweep that leaves every bit of the 4^3 grid unchanged ends the
-// sweeps: the remaining ones would repeat it.
 // Against one CTA with a thread per cell: 32 sweeps at 4^3 197 us (747), at
 // 8^3 323 us (771); 16 sweeps at 16^3 185 us (1508).
 // ---------------------------------------------------------------------------
@@ -290,7 +288,6 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
   __shared__ double cross[2][12][CC];  // signed cross products of a phase, by phase parity
   __shared__ double face[2][6][CC];    // face products x+ x- y+ y- z+ z-
   __shared__ double sum2[2][CC];       // S2 of a phase (of S1 for p = 2, 6), by phase parity
-  __shared__ int stop;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = G::CL == 1 ? 0 : (int)cl.block_rank();
   const int bx = rank % G::GX, by = (rank / G::GX) % G::GY, bz = rank / (G::GX * G::GY);
@@ -419,7 +416,6 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
       Y[p] = 1.0 / D[p];
     }
   }
-  if (tid == 0) stop = 0;
   // every CTA of the cluster runs and has its halo before the first store into it
   if (G::CL == 1) __syncthreads();
   else cl.sync();
@@ -469,7 +465,6 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
   };
   ahead(0);
   __syncthreads();
-  bool changed = false;
   for (int sw = 0; sw < nsweeps; ++sw) {
 #pragma unroll
     for (int p = 0; p < 8; ++p) {
@@ -507,7 +502,6 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
           s2 = sum2[p & 1][cell];
         }
         const double v = -div_by(__fma_rn(-0.5, s2, X2[p] - s1), D[p], Y[p]);
-        if (N == 4) changed = changed || __double_as_longlong(v) != __double_as_longlong(sp[c]);
         const int i = (p >> 1) & 1, j = p & 1, kz = p >> 2;
         if (CC == 8) {
 #pragma unroll
@@ -526,16 +520,10 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
             if (ok_[s] >> p & 1u) st_cluster(base_[s][(sets[s] & 4) && G::GZ > 2 ? kz : 0] + 8u * (c + off), v);
           }
         }
-        if (N == 4 && p == 7) {
-          const bool any = __any_sync(0xffffffffu, changed);
-          changed = false;
-          if (lane == 0) stop = any ? 0 : 1;
-        }
       }
       if (G::CL == 1) __syncthreads();
       else cl.sync();
     }
-    if (N == 4 && stop) break;
   }
   for (int e = tid; e < G::BX * G::BY * G::BZ; e += G::NT) {
     const int x = e % G::BX, y = (e / G::BX) % G::BY, z = e / (G::BX * G::BY);

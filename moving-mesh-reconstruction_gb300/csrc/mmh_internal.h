@@ -119,16 +119,16 @@ void launch_calcdefp_rhs(double* tmp, const double* rho, int n, double dtold, bo
 void launch_limiter_pass1(double* tmp, const double* def, const double* rho, int n, double dtold, double dtaumesh,
                           LimDev* st, uint8_t* maskx, uint8_t* maskc, cudaStream_t s);
 // the mixed form's pass 1: the same decisions and fluxes, FP32 screening and
-// FP64 only where a decision is close; detff = the float-float metric's det
-// of the same def
-void launch_limiter_pass1_mixed(double* tmp, const double* def, const double* rho, const double* detff, int n,
-                                double dtold, double dtaumesh, LimDev* st, uint8_t* maskx, uint8_t* maskc,
-                                cudaStream_t s);
+// FP64 only where a decision is close; defs = the split of def, detff = the
+// float-float metric's det of the same def
+void launch_limiter_pass1_mixed(double* tmp, const double* def, const float2* defs, const double* rho,
+                                const double* detff, int n, double dtold, double dtaumesh, LimDev* st, uint8_t* maskx,
+                                uint8_t* maskc, cudaStream_t s);
 void launch_limiter_mask(double* defplim, const double* def, const double* defp, int n, double dtold, LimDev* st,
                          uint8_t* mask, cudaStream_t s);
 // the same outputs, FP32 screening and FP64 only for the cells that may matter
-void launch_limiter_mask_mixed(double* defplim, const double* def, const double* defp, int n, double dtold, LimDev* st,
-                               uint8_t* mask, cudaStream_t s);
+void launch_limiter_mask_mixed(double* defplim, const double* def, const double* defp, const float2* defs,
+                               const float2* defps, int n, double dtold, LimDev* st, uint8_t* mask, cudaStream_t s);
 void launch_lim_reset(LimDev* st, cudaStream_t s);
 void launch_spec_tables(double* tab, int n, cudaStream_t s);
 void launch_spec_pack(const void* Xc, int n, void* Z, const LimDev* st, const double* tab, cudaStream_t s);
@@ -147,7 +147,8 @@ void launch_relax_dpv(const double* sd, const double* cc, int n, const double* u
                       double* gface, cudaStream_t s);
 // the mixed form's relaxing of the density (mmh_relax32.cu): FP32 fluxes, FP64
 // update; geo (n^3 float4), uf0, uf1 (n^3 floats) are scratch
-void launch_relax32(double* rho, const double* def, const double* defp, int n, double dt, float4* geo, float* uf0,
+// (defs, defps: the splits of def and defp)
+void launch_relax32(double* rho, const float2* defs, const float2* defps, int n, double dt, float4* geo, float* uf0,
                     float* uf1, cudaStream_t s);
 // u(nf,n^3) (float or double) <-> density; flag |= 1 when a component 2..nf is not zero
 void launch_extract_density_f(const float* u, int nf, i64 n3, double* rho, int* flag, cudaStream_t s);
@@ -202,8 +203,13 @@ void launch_residual_ff(const double* phi, const double* rhs, const double* coef
 // the finest level's metric straight into float-float pairs (coef, the layout
 // launch_ff_split makes) and their hi parts (coef32, FP32); det (may be null)
 // receives det(A) rounded to FP64
-void launch_metric_ff(const double* def, const double* rho, int n, double dx, double* coef, float* coef32,
+// (def, rho: their splits)
+void launch_metric_ff(const float2* def, const float2* rho, int n, double dx, double* coef, float* coef32,
                       double* det, cudaStream_t s);
+// float-float splits (hi, lo) of one or two fields (b may be null); def = def +
+// defp with the splits of both
+void launch_ff_split2(const double* a, float2* as, const double* b, float2* bs, i64 count, cudaStream_t s);
+void launch_add_split(double* def, const double* defp, float2* defs, float2* defps, i64 count, cudaStream_t s);
 
 // main.f90's iteration diagnostics: exact sums (def, def^2, defp^2, rho,
 // (rho-1)^2), ord_of-encoded extrema of rho, count of rho < 0, range flag

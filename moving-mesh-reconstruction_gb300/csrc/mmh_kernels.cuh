@@ -28,6 +28,9 @@ __device__ __forceinline__ int wp(int i, int n) { return i + 1 == n ? 0 : i + 1;
 __device__ __forceinline__ int wm(int i, int n) { return i == 0 ? n - 1 : i - 1; }
 __device__ __forceinline__ i64 IDX(int i, int j, int k, int n) { return (i64)i + (i64)n * ((i64)j + (i64)n * (i64)k); }
 
+// the same in 32 bits (n <= 1024: below 2^30)
+__device__ __forceinline__ int IDX32(int i, int j, int k, int n) { return i + n * (j + n * k); }
+
 template <class T> struct Vec16;
 template <> struct Vec16<float> { typedef float4 type; };
 template <> struct Vec16<double> { typedef double2 type; };

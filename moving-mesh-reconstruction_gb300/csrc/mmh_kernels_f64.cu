@@ -424,8 +424,8 @@ __global__ void k_limiter_pass1(double* __restrict__ tmp, const double* __restri
 
 // Pass 1 in the mixed form: the same decisions and fluxes as the FP64 pass,
 // with FP64 arithmetic only where a decision is close.  Every cell is first
-// screened in FP32 from its def samples truncated to floats (bit operations):
-// each sample is within 2^-23 |x| + 2^-126 of its double, so every entry of
+// screened in FP32 from its def samples truncated to floats, the high parts of
+// their float-float splits (defs): each sample is within 2^-23 |x| + 2^-126 of its double, so every entry of
 // C = I + Hess(def) is within E = 2^-18 max|sample| + 2^-20 (1 + sum |C_ij|)
 // of the FP64 one (about 4x the worst case of truncation and rounding), and
 // the Gershgorin bound g within 3E.  A cell with g - 3E above the FP64
@@ -438,6 +438,7 @@ __global__ void k_limiter_pass1(double* __restrict__ tmp, const double* __restri
 // exact.  The statistics of the screened cells come from detff (det min and
 // max) and rho^2 / det in float-float (rho2): not bit-matched.
 __global__ void __launch_bounds__(256) k_limiter_pass1_mixed(double* __restrict__ tmp, const double* __restrict__ def,
+                                                             const float2* __restrict__ defs,
                                                              const double* __restrict__ rho,
                                                              const double* __restrict__ detff, int n, double dtold,
                                                              double dtaumesh, double lim, double cmpmaxglobal,
@@ -461,12 +462,10 @@ __global__ void __launch_bounds__(256) k_limiter_pass1_mixed(double* __restrict_
     cell_of(t, n, i, j, km);
     const int k = wp(km, n);
     const int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), kq = wm(k, n);
-    bool ok = true;
-    float M = 0.0f;
+    unsigned mb = 0;  // bits of the largest |sample|; Inf and NaN lie above all others
     auto S = [&](int x, int y, int z) {
-      float f;
-      ok = f32_trunc_bits(def[IDX(x, y, z, n)], f) && ok;
-      M = fmaxf(M, fabsf(f));
+      const float f = defs[IDX32(x, y, z, n)].x;
+      mb = max(mb, abs_bits(f));
       return f;
     };
     const float c0 = S(i, j, k);
@@ -476,6 +475,8 @@ __global__ void __launch_bounds__(256) k_limiter_pass1_mixed(double* __restrict_
     const float hxy = ((S(ip, jp, k) - S(im, jp, k)) - (S(ip, jm, k) - S(im, jm, k))) * 0.25f;
     const float hyz = ((S(i, jp, kp) - S(i, jp, kq)) - (S(i, jm, kp) - S(i, jm, kq))) * 0.25f;
     const float hxz = ((S(ip, j, kp) - S(im, j, kp)) - (S(ip, j, kq) - S(im, j, kq))) * 0.25f;
+    const float M = __uint_as_float(mb);
+    bool ok = mb < 0x7f800000u;
     const float c11 = 1.0f + hxx, c22 = 1.0f + hyy, c33 = 1.0f + hzz;
     const float sc = 1.0f + fabsf(c11) + fabsf(c22) + fabsf(c33) + 2.0f * (fabsf(hxy) + fabsf(hyz) + fabsf(hxz));
     const float E = 3.814697265625e-6f * M + 9.5367431640625e-7f * sc;  // 2^-18 M + 2^-20 sc
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(256) k_limiter_pass1_mixed(double* __restrict_
                           c33 - fabsf(hxz) - fabsf(hyz));
     const bool gsure = g - 3.0f * E > gthr;
     // pass 1 evaluates the metric at (i, j, k = km + 1) for the cell (i, j, km)
-    const double det = detff[IDX(i, j, k, n)];
+    const double det = detff[IDX32(i, j, k, n)];
     float d32;
     ok = f32_trunc_bits(det, d32) && ok;
     const float Ed = 9.094947017729282e-13f * (1.0f + M) * sc * sc + 4.76837158203125e-6f * (1.0f + fabsf(d32));
@@ -547,15 +548,15 @@ void launch_limiter_pass1(double* tmp, const double* def, const double* rho, int
   k_limiter_pass1<<<grid_of(n3, kBlock), kBlock, 0, s>>>(tmp, def, rho, n, dtold, dtaumesh, 10.0, st, maskx, maskc);
   count_launch();
 }
-void launch_limiter_pass1_mixed(double* tmp, const double* def, const double* rho, const double* detff, int n,
-                                double dtold, double dtaumesh, LimDev* st, uint8_t* maskx, uint8_t* maskc,
+void launch_limiter_pass1_mixed(double* tmp, const double* def, const float2* defs, const double* rho,
+                                const double* detff, int n, double dtold, double dtaumesh, LimDev* st, uint8_t* maskx, uint8_t* maskc,
                                 cudaStream_t s) {
   i64 n3 = (i64)n * n * n;
   // a float at or above the FP64 shortcut's threshold 1/cmpmax + 1e-6
   const double thr = 1.0 / 10.0 + 1e-6;
   float gthr = (float)thr;
   if ((double)gthr < thr) gthr = nextafterf(gthr, 1.0f);
-  k_limiter_pass1_mixed<<<grid_of(n3, kBlock), kBlock, 0, s>>>(tmp, def, rho, detff, n, dtold, dtaumesh,
+  k_limiter_pass1_mixed<<<grid_of(n3, kBlock), kBlock, 0, s>>>(tmp, def, defs, rho, detff, n, dtold, dtaumesh,
                                                                1.0 / dtaumesh, 10.0, gthr, st, maskx, maskc);
   count_launch();
 }
@@ -693,7 +694,8 @@ void launch_limiter_mask(double* defplim, const double* def, const double* defp,
 // The final compression test in the mixed form: the same outputs as
 // k_limiter_mask, with FP64 arithmetic only for the cells that may matter.
 // The bounds lo and hi come from C in FP32, formed from the samples of def
-// and defp truncated to floats (bit operations): every entry is within E =
+// and defp truncated to floats (the high parts of their splits defs, defps):
+// every entry is within E =
 // 2^-18 (max|def sample| + |dtold| max|defp sample|) + 2^-20 (1 + sum|C_ij|)
 // of the FP64 one (about 4x the worst case of truncation and rounding), so
 // the smallest eigenvalue within 3E, by which lo and hi are widened.  The
@@ -701,7 +703,9 @@ void launch_limiter_mask(double* defplim, const double* def, const double* defp,
 // inv_tight = (1/cmpmax)(1 + 1e-12), formed on the host.
 __global__ void __launch_bounds__(256) k_limiter_mask_mixed(double* __restrict__ defplim,
                                                             const double* __restrict__ def,
-                                                            const double* __restrict__ defp, int n, double dtold,
+                                                            const double* __restrict__ defp,
+                                                            const float2* __restrict__ defs,
+                                                            const float2* __restrict__ defps, int n, double dtold,
                                                             double cmpmaxglobal, double inv_tight, LimDev* st,
                                                             uint8_t* __restrict__ mask) {
   __shared__ int s_list[256];
@@ -725,17 +729,15 @@ __global__ void __launch_bounds__(256) k_limiter_mask_mixed(double* __restrict__
     int i, j, k;
     cell_of(t, n, i, j, k);
     const int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
-    float Md = 0.0f, Mp = 0.0f;
+    unsigned mbd = 0, mbp = 0;  // bits of the largest |sample|; Inf and NaN lie above all others
     auto D = [&](int x, int y, int z) {
-      float f;
-      ok = f32_trunc_bits(def[IDX(x, y, z, n)], f) && ok;
-      Md = fmaxf(Md, fabsf(f));
+      const float f = defs[IDX32(x, y, z, n)].x;
+      mbd = max(mbd, abs_bits(f));
       return f;
     };
     auto P = [&](int x, int y, int z) {
-      float f;
-      ok = f32_trunc_bits(defp[IDX(x, y, z, n)], f) && ok;
-      Mp = fmaxf(Mp, fabsf(f));
+      const float f = defps[IDX32(x, y, z, n)].x;
+      mbp = max(mbp, abs_bits(f));
       return f;
     };
     const float pc = P(i, j, k), dc = D(i, j, k);
@@ -752,7 +754,8 @@ __global__ void __launch_bounds__(256) k_limiter_mask_mixed(double* __restrict__
     const float c23 = pyz + ((D(i, jp, kp) - D(i, jp, km)) - (D(i, jm, kp) - D(i, jm, km))) * 0.25f;
     const float c13 = pxz + ((D(ip, j, kp) - D(im, j, kp)) - (D(ip, j, km) - D(im, j, km))) * 0.25f;
     const float sc = 1.0f + fabsf(c11) + fabsf(c22) + fabsf(c33) + 2.0f * (fabsf(c12) + fabsf(c23) + fabsf(c13));
-    const float E = 3.814697265625e-6f * (Md + fabsf(dtf) * Mp) + 9.5367431640625e-7f * sc;  // 2^-18, 2^-20
+    ok = max(mbd, mbp) < 0x7f800000u;
+    const float E = 3.814697265625e-6f * (__uint_as_float(mbd) + fabsf(dtf) * __uint_as_float(mbp)) + 9.5367431640625e-7f * sc;  // 2^-18, 2^-20
     compression_bounds_f(c11, c12, c13, c22, c23, c33, lo, hi);
     lo -= 3.0f * E;
     hi += 3.0f * E;
@@ -798,10 +801,10 @@ __global__ void __launch_bounds__(256) k_limiter_mask_mixed(double* __restrict__
   r = block_u64(cm, s_buf, 1);
   if (threadIdx.x == 0) atomicMax(&st->cmax, r);
 }
-void launch_limiter_mask_mixed(double* defplim, const double* def, const double* defp, int n, double dtold, LimDev* st,
-                               uint8_t* mask, cudaStream_t s) {
+void launch_limiter_mask_mixed(double* defplim, const double* def, const double* defp, const float2* defs,
+                               const float2* defps, int n, double dtold, LimDev* st, uint8_t* mask, cudaStream_t s) {
   i64 n3 = (i64)n * n * n;
-  k_limiter_mask_mixed<<<grid_of(n3, kBlock), kBlock, 0, s>>>(defplim, def, defp, n, dtold, 10.0,
+  k_limiter_mask_mixed<<<grid_of(n3, kBlock), kBlock, 0, s>>>(defplim, def, defp, defs, defps, n, dtold, 10.0,
                                                               (1.0 / 10.0) * (1.0 + 1e-12), st, mask);
   count_launch();
 }
@@ -952,7 +955,7 @@ void launch_power_bins(const void* A, const void* B, int n, int nb, const double
 // / dx^2 and the coefficients about 48 significant bits otherwise.  det <=
 // 1e-5 takes the reference's fallback (unit cofactors, det = 1).  di2 =
 // 1/dx^2 is a power of two.
-__global__ void __launch_bounds__(256) k_metric_ff(const double* __restrict__ def, const double* __restrict__ rho,
+__global__ void __launch_bounds__(256) k_metric_ff(const float2* __restrict__ def, const float2* __restrict__ rho,
                                                    int n, float di2, float2* __restrict__ coef,
                                                    float* __restrict__ coef32, double* __restrict__ det_out) {
   const i64 n3 = (i64)n * n * n;
@@ -961,8 +964,9 @@ __global__ void __launch_bounds__(256) k_metric_ff(const double* __restrict__ de
   int i, j, k;
   cell_of(t, n, i, j, k);
   const int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
-#define D_(x, y, z) ff_of_bits(def[IDX(x, y, z, n)])
-  const FF c = ff_of_bits(def[t]);
+  auto pair = [](float2 v) { return FF{v.x, v.y}; };
+#define D_(x, y, z) pair(def[IDX32(x, y, z, n)])
+  const FF c = pair(def[t]);
   const FF pxx = ff_scale(ff_add(ff_diff(D_(ip, j, k), c), ff_diff(D_(im, j, k), c)), di2);
   const FF pyy = ff_scale(ff_add(ff_diff(D_(i, jp, k), c), ff_diff(D_(i, jm, k), c)), di2);
   const FF pzz = ff_scale(ff_add(ff_diff(D_(i, j, kp), c), ff_diff(D_(i, j, km), c)), di2);
@@ -996,7 +1000,7 @@ __global__ void __launch_bounds__(256) k_metric_ff(const double* __restrict__ de
     for (int bb = 0; bb < 3; ++bb)
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const FF v = ff_of_bits(rho[IDX(is[a], js[bb], ks[d], n)]);
+        const FF v = pair(rho[IDX32(is[a], js[bb], ks[d], n)]);
         const FF s2 = ff_two_sum(sh, v.hi);
         sh = s2.hi;
         se = se + (s2.lo + v.lo);
@@ -1014,13 +1018,45 @@ __global__ void __launch_bounds__(256) k_metric_ff(const double* __restrict__ de
   }
 }
 
-void launch_metric_ff(const double* def, const double* rho, int n, double dx, double* coef, float* coef32,
+void launch_metric_ff(const float2* def, const float2* rho, int n, double dx, double* coef, float* coef32,
                       double* det, cudaStream_t s) {
   const i64 n3 = (i64)n * n * n;
   prof_begin(KK_METRIC, s, n3, n);
   k_metric_ff<<<grid_of(n3, kBlock), kBlock, 0, s>>>(def, rho, n, (float)(1.0 / (dx * dx)), reinterpret_cast<float2*>(coef),
                                                      coef32, det);
   prof_end(KK_METRIC, s, n);
+  count_launch();
+}
+
+// float-float splits of two fields (b may be null)
+__global__ void k_ff_split2(const double* __restrict__ a, float2* __restrict__ as, const double* __restrict__ b,
+                            float2* __restrict__ bs, i64 count) {
+  const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const FF v = ff_of_bits(a[t]);
+  as[t] = make_float2(v.hi, v.lo);
+  if (b) {
+    const FF w = ff_of_bits(b[t]);
+    bs[t] = make_float2(w.hi, w.lo);
+  }
+}
+// def = def + defp, and the splits of both
+__global__ void k_add_split(double* __restrict__ def, const double* __restrict__ defp, float2* __restrict__ defs,
+                            float2* __restrict__ defps, i64 count) {
+  const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const double p = defp[t], d = def[t] + p;
+  def[t] = d;
+  const FF v = ff_of_bits(d), w = ff_of_bits(p);
+  defs[t] = make_float2(v.hi, v.lo);
+  defps[t] = make_float2(w.hi, w.lo);
+}
+void launch_ff_split2(const double* a, float2* as, const double* b, float2* bs, i64 count, cudaStream_t s) {
+  k_ff_split2<<<grid_of(count, kBlock), kBlock, 0, s>>>(a, as, b, bs, count);
+  count_launch();
+}
+void launch_add_split(double* def, const double* defp, float2* defs, float2* defps, i64 count, cudaStream_t s) {
+  k_add_split<<<grid_of(count, kBlock), kBlock, 0, s>>>(def, defp, defs, defps, count);
   count_launch();
 }
 
@@ -1067,11 +1103,11 @@ __global__ void __launch_bounds__(256) k_residual_ff(const float2* __restrict__ 
     cell_of(t, n, i, j, k);
     const int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
     auto P = [&](int a, int b, int c) {
-      float2 v = __ldg(phi + IDX(a, b, c, n));
+      float2 v = __ldg(phi + IDX32(a, b, c, n));
       return FF{v.x, v.y};
     };
     auto C = [&](int f, int a, int b, int c) {
-      float2 v = __ldg(coef + (i64)f * n3 + IDX(a, b, c, n));
+      float2 v = __ldg(coef + (i64)f * n3 + IDX32(a, b, c, n));
       return FF{v.x, v.y};
     };
     const FF pc = P(i, j, k);

@@ -53,8 +53,8 @@ __device__ __forceinline__ float wphalf32(float sm, float s0, float sp, float d0
 
 // Geometry of the step at every cell: geo = (alpha_x, alpha_y, alpha_z, c),
 // and the density rounded to FP32.
-__global__ void __launch_bounds__(256) k_relax32_geom(const double* __restrict__ rho, const double* __restrict__ def,
-                                                      const double* __restrict__ defp, int n,
+__global__ void __launch_bounds__(256) k_relax32_geom(const double* __restrict__ rho, const float2* __restrict__ def,
+                                                      const float2* __restrict__ defp, int n,
                                                       float4* __restrict__ geo, float* __restrict__ uf) {
   const i64 n3 = (i64)n * n * n;
   const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -63,10 +63,11 @@ __global__ void __launch_bounds__(256) k_relax32_geom(const double* __restrict__
   cell_of(t, n, i, j, k);
   const int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
   // second differences of def and central differences of defp from
-  // float-float splits of the samples (integer and FP32 operations; FP64
-  // runs at two operations per clock per SM on GB300), rounded once to FP32
-#define D_(x, y, z) ff_of_bits(def[IDX(x, y, z, n)])
-  const FF c0 = ff_of_bits(def[t]);
+  // float-float splits of the samples (FP64 runs at two operations per clock
+  // per SM on GB300), rounded once to FP32
+  auto pair = [](float2 v) { return FF{v.x, v.y}; };
+#define D_(x, y, z) pair(def[IDX32(x, y, z, n)])
+  const FF c0 = pair(def[t]);
   const float pxx = ff_sum_f(ff_diff(D_(ip, j, k), c0), ff_diff(D_(im, j, k), c0));
   const float pyy = ff_sum_f(ff_diff(D_(i, jp, k), c0), ff_diff(D_(i, jm, k), c0));
   const float pzz = ff_sum_f(ff_diff(D_(i, j, kp), c0), ff_diff(D_(i, j, km), c0));
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(256) k_relax32_geom(const double* __restrict__
   const float b22 = a11 * a33 - a13 * a13, b23 = a12 * a13 - a11 * a23, b33 = a11 * a22 - a12 * a12;
   const float det = a11 * b11 + a12 * b12 + a13 * b13;
   // -grad defp (central differences)
-#define P_(x, y, z) ff_of_bits(defp[IDX(x, y, z, n)])
+#define P_(x, y, z) pair(defp[IDX32(x, y, z, n)])
   const float gx = ff_diff_f(P_(im, j, k), P_(ip, j, k)) * 0.5f;
   const float gy = ff_diff_f(P_(i, jm, k), P_(i, jp, k)) * 0.5f;
   const float gz = ff_diff_f(P_(i, j, km), P_(i, j, kp)) * 0.5f;
@@ -160,11 +161,11 @@ __global__ void __launch_bounds__(256) k_relax32_stage(const float* __restrict__
 
 // The mixed form's relaxing of the density rho (in place): geo (n^3 float4),
 // uf0 and uf1 (n^3 floats each) are scratch.
-void launch_relax32(double* rho, const double* def, const double* defp, int n, double dt, float4* geo, float* uf0,
+void launch_relax32(double* rho, const float2* defs, const float2* defps, int n, double dt, float4* geo, float* uf0,
                     float* uf1, cudaStream_t s) {
   const i64 n3 = (i64)n * n * n;
   const unsigned g = (unsigned)((n3 + 255) / 256);
-  k_relax32_geom<<<g, 256, 0, s>>>(rho, def, defp, n, geo, uf0);
+  k_relax32_geom<<<g, 256, 0, s>>>(rho, defs, defps, n, geo, uf0);
   k_relax32_stage<true><<<g, 256, 0, s>>>(uf0, geo, n, rho, (float)(dt / 2.0), nullptr, uf1);
   k_relax32_stage<false><<<g, 256, 0, s>>>(uf1, geo, n, rho, (float)dt, rho, nullptr);
   count_launch(3);

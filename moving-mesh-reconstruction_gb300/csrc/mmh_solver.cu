@@ -153,6 +153,10 @@ struct mmh_ctx {
   bool u_zero = false;
   uint8_t* mask(int q) { return keep_masks ? masks + q * n3 : nullptr; }
 
+  // float-float splits of def and of rho or defp, in the spectral buffers
+  // (which only the FFT Poisson correction and the power spectra use)
+  float2* defs() { return reinterpret_cast<float2*>(Xc); }
+  float2* aux_split() { return reinterpret_cast<float2*>(Z); }
   double* defp() { return h64.u[0]; }
   double* tmp() { return h64.rhs[0]; }
 
@@ -382,7 +386,8 @@ int build_levels(mmh_ctx* c, int l0) {
     // (a solve on the coarsest level itself keeps FP64 coefficients: its exact
     // coarse solve is formed from them)
     if (l == l0 && l0 < c->nlev - 1 && ff_outer(c)) {
-      launch_metric_ff(c->defl[l], c->rhol[l], n, double(1 << l), c->h64.coef[l], c->h32.coef[l], c->det, c->s);
+      launch_ff_split2(c->defl[l], c->defs(), c->rhol[l], c->aux_split(), (i64)n * n * n, c->s);
+      launch_metric_ff(c->defs(), c->aux_split(), n, double(1 << l), c->h64.coef[l], c->h32.coef[l], c->det, c->s);
       c->coef_ff = true;
       continue;
     }
@@ -878,12 +883,15 @@ int calcdefp_dev(mmh_ctx* c, double dtold, double dtaumesh, uint8_t* mx, uint8_t
   smooth_step(c, tmp, c->scr);
   launch_lim_reset(&c->sc->lim, c->s);
   c->levels_ready = false;
+  bool def_split = false;  // defs() holds the split of def
   if (ff_outer(c) && c->nlev > 1) {
     // The float-float metric of def (which calcdefp does not change) is
     // built first: pass 1 screens its expansion test with its det.
     RET(build_levels(c, 0));
     c->levels_ready = true;
-    launch_limiter_pass1_mixed(c->scr, c->def, c->rho, c->det, n, dtold, dtaumesh, &c->sc->lim, mx, mc1, c->s);
+    launch_limiter_pass1_mixed(c->scr, c->def, c->defs(), c->rho, c->det, n, dtold, dtaumesh, &c->sc->lim, mx, mc1,
+                               c->s);
+    def_split = true;
   } else {
     launch_limiter_pass1(c->scr, c->def, c->rho, n, dtold, dtaumesh, &c->sc->lim, mx, mc1, c->s);
   }
@@ -895,10 +903,13 @@ int calcdefp_dev(mmh_ctx* c, double dtold, double dtaumesh, uint8_t* mx, uint8_t
   if (st != MMH_OK && st != MMH_ERR_DIVERGED) return st;
   smooth_step(c, defp, c->scr);
   smooth_step(c, c->scr, defp);
-  if (c->cfg.precision == MMH_MIXED)
-    launch_limiter_mask_mixed(c->defplim, c->def, defp, n, dtold, &c->sc->lim, mc2, c->s);
-  else
+  if (c->cfg.precision == MMH_MIXED) {
+    if (def_split) launch_ff_split2(defp, c->aux_split(), nullptr, nullptr, n3, c->s);
+    else launch_ff_split2(c->def, c->defs(), defp, c->aux_split(), n3, c->s);
+    launch_limiter_mask_mixed(c->defplim, c->def, defp, c->defs(), c->aux_split(), n, dtold, &c->sc->lim, mc2, c->s);
+  } else {
     launch_limiter_mask(c->defplim, c->def, defp, n, dtold, &c->sc->lim, mc2, c->s);
+  }
   // The FFT Poisson correction adds F^-1[F[defplim]/kernel], which is zero
   // when no cell was limited: its transforms run only when one was.
   RET(pull_scal(c));
@@ -910,13 +921,22 @@ int calcdefp_dev(mmh_ctx* c, double dtold, double dtaumesh, uint8_t* mx, uint8_t
   return st;
 }
 
-// relaxing(u, def, defp, cmax, dt, 5) on the resident density.
-int relaxing_dev(mmh_ctx* c, double dt) {
+// def = def + defp (main.f90:98); the mixed form's relaxing reads the splits
+// that come with it
+void add_defp(mmh_ctx* c) {
+  if (c->cfg.precision == MMH_MIXED) launch_add_split(c->def, c->defp(), c->defs(), c->aux_split(), c->n3, c->s);
+  else launch_add(c->def, c->defp(), c->n3, c->s);
+}
+
+// relaxing(u, def, defp, cmax, dt, 5) on the resident density.  split: add_defp
+// has just been called.
+int relaxing_dev(mmh_ctx* c, double dt, bool split = false) {
   Stage stage_("mmh relaxing");
   int n = c->n;
   if (c->cfg.precision == MMH_MIXED) {
+    if (!split) launch_ff_split2(c->def, c->defs(), c->defp(), c->aux_split(), c->n3, c->s);
     // FP32 fluxes, FP64 update (the relaxing buffers hold the FP32 scratch)
-    launch_relax32(c->rho, c->def, c->defp(), n, dt, reinterpret_cast<float4*>(c->baj), reinterpret_cast<float*>(c->cc),
+    launch_relax32(c->rho, c->defs(), c->aux_split(), n, dt, reinterpret_cast<float4*>(c->baj), reinterpret_cast<float*>(c->cc),
                    reinterpret_cast<float*>(c->u1), c->s);
     return MMH_OK;
   }
@@ -1218,8 +1238,8 @@ int iterate_adjoint_dev(mmh_ctx* c, int niter, int every, const double* wdef, co
     mmh_diag dd{};
     int st = calcdefp_dev(c, 1.0, 1.0, nullptr, nullptr, nullptr, &dd);
     if (st != MMH_OK) return st;
-    launch_add(c->def, defp, n3, c->s);
-    RET(relaxing_dev(c, 1.0));
+    add_defp(c);
+    RET(relaxing_dev(c, 1.0, true));
     if (d) *d = dd;
   }
   CK(cudaMemcpyAsync(fin, c->def, f, cudaMemcpyDeviceToDevice, c->s));
@@ -1246,8 +1266,8 @@ int iterate_adjoint_dev(mmh_ctx* c, int niter, int every, const double* wdef, co
       RET(calcdefp_fwd_keep(c, 1.0, 1.0, keep(k - k0), nullptr));
       CK(cudaMemcpyAsync(sk + 2 * n3, defp, f, cudaMemcpyDeviceToDevice, c->s));
       if (k + 1 < k1) {
-        launch_add(c->def, defp, n3, c->s);
-        RET(relaxing_dev(c, 1.0));
+        add_defp(c);
+        RET(relaxing_dev(c, 1.0, true));
       }
     }
     for (int k = k1 - 1; k >= k0; --k) {
@@ -1927,7 +1947,8 @@ int mmh_metric_ff_f64(mmh_ctx* c, const double* deformpot, const double* rho, do
   i64 n3 = (i64)n * n * n;
   RET(upload(c, deformpot, c->defl[l], n3));
   RET(upload(c, rho, c->rhol[l], n3));
-  launch_metric_ff(c->defl[l], c->rhol[l], n, dx, c->h64.coef[l], c->h32.coef[l], det ? c->det : nullptr, c->s);
+  launch_ff_split2(c->defl[l], c->defs(), c->rhol[l], c->aux_split(), n3, c->s);
+  launch_metric_ff(c->defs(), c->aux_split(), n, dx, c->h64.coef[l], c->h32.coef[l], det ? c->det : nullptr, c->s);
   launch_ff_join(c->h64.coef[l], 6 * n3, c->s);
   c->coef_ff = false;
   if (det) RET(download(c, c->det, det, n3));
@@ -2008,10 +2029,12 @@ int mmh_limiter_pass1_f64(mmh_ctx* c, double* tmp, const double* def, const doub
   if (c->cfg.precision == MMH_MIXED) {
     // the mixed form screens with the float-float metric's det (the metric
     // of level 0 is rebuilt by the next solve)
-    launch_metric_ff(c->def, c->rho, n, 1.0, c->h64.coef[0], c->h32.coef[0], c->det, c->s);
+    launch_ff_split2(c->def, c->defs(), c->rho, c->aux_split(), n3, c->s);
+    launch_metric_ff(c->defs(), c->aux_split(), n, 1.0, c->h64.coef[0], c->h32.coef[0], c->det, c->s);
     c->coef_ff = true;
     c->levels_ready = false;
-    launch_limiter_pass1_mixed(c->scr, c->def, c->rho, c->det, n, dtold, dtaumesh, &c->sc->lim, dm, dm + n3, c->s);
+    launch_limiter_pass1_mixed(c->scr, c->def, c->defs(), c->rho, c->det, n, dtold, dtaumesh, &c->sc->lim, dm, dm + n3,
+                               c->s);
   } else {
     launch_limiter_pass1(c->scr, c->def, c->rho, n, dtold, dtaumesh, &c->sc->lim, dm, dm + n3, c->s);
   }
@@ -2034,9 +2057,10 @@ int mmh_limiter_mask_f64(mmh_ctx* c, double* defplim, const double* def, const d
   uint8_t* dm = nullptr;
   CK(cudaMallocAsync((void**)&dm, n3, c->s));
   launch_lim_reset(&c->sc->lim, c->s);
-  if (c->cfg.precision == MMH_MIXED)
-    launch_limiter_mask_mixed(c->defplim, c->def, c->scr, n, dtold, &c->sc->lim, dm, c->s);
-  else
+  if (c->cfg.precision == MMH_MIXED) {
+    launch_ff_split2(c->def, c->defs(), c->scr, c->aux_split(), n3, c->s);
+    launch_limiter_mask_mixed(c->defplim, c->def, c->scr, c->defs(), c->aux_split(), n, dtold, &c->sc->lim, dm, c->s);
+  } else
     launch_limiter_mask(c->defplim, c->def, c->scr, n, dtold, &c->sc->lim, dm, c->s);
   RET(download(c, c->defplim, defplim, n3));
   if (mask) CK(cudaMemcpyAsync(mask, dm, n3, cudaMemcpyDeviceToHost, c->s));
@@ -2082,8 +2106,8 @@ int mmh_iterate(mmh_ctx* c, int niter, mmh_diag* d) {
     mmh_diag dd{};
     st = calcdefp_dev(c, 1.0, 1.0, c->mask(0), c->mask(1), c->mask(2), &dd);
     if (st != MMH_OK && st != MMH_ERR_DIVERGED) return st;
-    launch_add(c->def, c->defp(), c->n3, c->s);
-    RET(relaxing_dev(c, 1.0));
+    add_defp(c);
+    RET(relaxing_dev(c, 1.0, true));
     dd.status = st;
     if (d) *d = dd;
   }
