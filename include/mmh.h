@@ -235,6 +235,8 @@ int mmh_power_spectrum_f64(mmh_ctx* ctx, const double* a, const double* b, int n
  * distance; the reference would keep searching).  No context: the call
  * allocates and frees its own device memory on the current device. */
 int mmh_haloden(const float* x, long long np, int nf, int ng, float* den, float* raw, int* wp);
+/* the same with x(np,3): all x, then all y, then all z */
+int mmh_haloden_planes(const float* x, long long np, int nf, int ng, float* den, float* raw, int* wp);
 /* from1024to512.f90: ncoarse halvings of an ng^3 density by 2x2x2 block sums,
  * then scaled to mean 1 (the sum taken exactly, then rounded to 4 bytes). */
 int mmh_coarsen(const float* den, int ng, int ncoarse, float* out);

@@ -32,14 +32,20 @@ constexpr int kB = 256;
 constexpr int kHaloMaxRadius = 64;
 unsigned blocks_of(i64 count) { return (unsigned)((count + kB - 1) / kB); }
 
-// Fortran MODULO for reals: the exact remainder, moved into [0, p).
+// Fortran MODULO for reals: the exact remainder, moved into [0, p).  For |a| <
+// 2p the remainder is a itself or a -+ p, which is exact (Sterbenz); fmodf's
+// general reduction costs ten times that.
 __device__ __forceinline__ float fmodulo(float a, float p) {
-  float r = fmodf(a, p);
+  const float m = fabsf(a);
+  float r = m < p ? a : m < 2.0f * p ? copysignf(m - p, a) : fmodf(a, p);
   if (r != 0.0f && ((r < 0.0f) != (p < 0.0f))) r = r + p;
   return r;
 }
 
-// positions to grid units and cells (haloden.f90:87-108)
+// positions to grid units and cells (haloden.f90:87-108); x: a particle's three
+// components together, or with PLANES all particles' one component after the
+// other
+template <bool PLANES>
 __global__ void k_halo_cells(const float* __restrict__ x, i64 np, int nf, int ng, float* __restrict__ xp,
                              unsigned* __restrict__ cell, unsigned* __restrict__ ip_out, int* flag) {
   i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -47,7 +53,7 @@ __global__ void k_halo_cells(const float* __restrict__ x, i64 np, int nf, int ng
   int c[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    float v = fmodulo(x[3 * p + a], (float)nf);
+    float v = fmodulo(x[PLANES ? a * np + p : 3 * p + a], (float)nf);
     v = v * (float)ng / (float)nf;
     xp[3 * p + a] = v;
     c[a] = (int)floorf(v);
@@ -78,6 +84,8 @@ __global__ void k_halo_bounds(const unsigned* __restrict__ key, i64 np, int* __r
 // The shells grow to at most rmax cells; a cell with no particle within that
 // radius sets flag bit 4 (the reference's search would go on, and so would
 // its cost: (2r+1)^3 cells per empty cell).  Launched on cells [g0, g1).
+// r <= ng/2 + 1 cells from a cell lie at most one period away, so a wrap is a
+// comparison and a sum, and a row inside the shell has only its two ends.
 __global__ void k_halo_search(const float* __restrict__ xp, const unsigned* __restrict__ order,
                               const int* __restrict__ first, const int* __restrict__ last, int ng, int rmax,
                               i64 g0, i64 g1, int* __restrict__ choice, int* __restrict__ wp, int* flag) {
@@ -88,14 +96,14 @@ __global__ void k_halo_search(const float* __restrict__ xp, const unsigned* __re
   const float gx = (float)(i + 1) - 0.5f, gy = (float)(j + 1) - 0.5f, gz = (float)(k + 1) - 0.5f;
   const float h = (float)(ng / 2), fng = (float)ng;
   float r2min = (float)(1000 * ng * ng);
+  auto wrap = [&](int c) { return c < 0 ? c + ng : c >= ng ? c - ng : c; };
   int best = -1;
   for (int r = 1; r <= rmax && best < 0; ++r) {
     for (int dk = -r; dk <= r; ++dk)
       for (int dj = -r; dj <= r; ++dj)
-        for (int di = -r; di <= r; ++di) {
-          // cells inside the shell were empty at the previous radius
-          if (dk > -r && dk < r && dj > -r && dj < r && di > -r && di < r) continue;
-          int ii = ((i + di) % ng + ng) % ng, jj = ((j + dj) % ng + ng) % ng, kk = ((k + dk) % ng + ng) % ng;
+        // cells inside the shell were empty at the previous radius
+        for (int di = -r; di <= r; di += (dk > -r && dk < r && dj > -r && dj < r) ? 2 * r : 1) {
+          const int ii = wrap(i + di), jj = wrap(j + dj), kk = wrap(k + dk);
           i64 c = ii + (i64)ng * (jj + (i64)ng * kk);
           int f = first[c];
           if (f < 0) continue;
@@ -220,9 +228,8 @@ struct Carve {
 
 using namespace mmh;
 
-extern "C" {
-
-int mmh_haloden(const float* x, long long np, int nf, int ng, float* den, float* raw, int* wp) {
+namespace {
+int haloden_run(const float* x, bool planes, long long np, int nf, int ng, float* den, float* raw, int* wp) {
   if (!x || !den || np < 1 || nf < 1 || ng < 2 || ng > 1024) return MMH_ERR_ARG;
   if (np >= (1ll << 31)) return MMH_ERR_SIZE;
   const i64 ng3 = (i64)ng * ng * ng;
@@ -256,7 +263,8 @@ int mmh_haloden(const float* x, long long np, int nf, int ng, float* den, float*
   PK(cudaMemset(first, 0xff, sizeof(int) * ng3));
   PK(cudaMemset(acc, 0, 16));
   PK(cudaMemset(flag, 0, sizeof(int)));
-  k_halo_cells<<<blocks_of(np), kB>>>(dx, np, nf, ng, xp, key, ips, flag);
+  if (planes) k_halo_cells<true><<<blocks_of(np), kB>>>(dx, np, nf, ng, xp, key, ips, flag);
+  else k_halo_cells<false><<<blocks_of(np), kB>>>(dx, np, nf, ng, xp, key, ips, flag);
   count_launch();
   PK(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, key, skey, ips, order, (int)np, 0, bits));
   k_halo_bounds<<<blocks_of(np), kB>>>(skey, np, first, last);
@@ -287,6 +295,16 @@ int mmh_haloden(const float* x, long long np, int nf, int ng, float* den, float*
   if (raw) PK(cudaMemcpy(raw, draw, sizeof(float) * ng3, cudaMemcpyDeviceToHost));
   if (wp) PK(cudaMemcpy(wp, dwp, sizeof(int) * np, cudaMemcpyDeviceToHost));
   return MMH_OK;
+}
+}  // namespace
+
+extern "C" {
+
+int mmh_haloden(const float* x, long long np, int nf, int ng, float* den, float* raw, int* wp) {
+  return haloden_run(x, false, np, nf, ng, den, raw, wp);
+}
+int mmh_haloden_planes(const float* x, long long np, int nf, int ng, float* den, float* raw, int* wp) {
+  return haloden_run(x, true, np, nf, ng, den, raw, wp);
 }
 
 int mmh_coarsen(const float* den, int ng, int ncoarse, float* out) {

@@ -43,7 +43,7 @@ EXPORTS = (
     "mmh_outputs_f64", "mmh_outputs_dev", "mmh_state_dev", "mmh_profile_start", "mmh_profile_stop",
     "mmh_relax_noalloc_f64", "mmh_batch_run", "mmh_calcdefp_adjoint_f64",
     "mmh_relaxing_adjoint_f64", "mmh_iterate_adjoint_f64", "mmh_state_stats",
-    "mmh_power_spectrum_f64", "mmh_haloden", "mmh_coarsen",
+    "mmh_power_spectrum_f64", "mmh_haloden", "mmh_haloden_planes", "mmh_coarsen",
     "mmh_column_density", "mmh_gridfigure", "mmh_keep_masks", "mmh_masks", "mmh_gs_tile_pin", "mmh_gs_tile", "mmh_stencil_pin",
 )
 
@@ -68,14 +68,19 @@ def write_spectrum(path, k, p):
 def haloden(x, nf, ng):
     """Particle density assignment (haloden.f90) on the GPU: x (3, np) float32
     positions in fine-cell units.  Returns (den, raw, wp)."""
-    xc = np.ascontiguousarray(np.asarray(x, dtype=np.float32).T)  # component fastest
-    np_ = xc.shape[0]
+    xa = np.asarray(x, dtype=np.float32)
+    # rows of coordinates go to the GPU as they lie (transposing them on the
+    # host took longer than the kernels); other layouts component fastest
+    planes = xa.ndim == 2 and xa.shape[0] == 3 and xa.flags.c_contiguous
+    xc = xa if planes else np.ascontiguousarray(xa.T)
+    np_ = xa.shape[1] if planes else xc.shape[0]
     den = np.zeros((ng, ng, ng), dtype=np.float32, order="F")
     raw = np.zeros_like(den, order="F")
     wp = np.zeros(np_, dtype=np.int32)
     L = lib()
-    L.mmh_haloden.argtypes = [C.c_void_p, C.c_longlong, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
-    _chk(L.mmh_haloden(_p(xc), np_, int(nf), int(ng), _p(den), _p(raw), _p(wp)), "haloden")
+    f = L.mmh_haloden_planes if planes else L.mmh_haloden
+    f.argtypes = [C.c_void_p, C.c_longlong, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
+    _chk(f(_p(xc), np_, int(nf), int(ng), _p(den), _p(raw), _p(wp)), "haloden")
     return den, raw, wp
 
 
