@@ -99,40 +99,52 @@ __device__ __forceinline__ float block_sum_f32(float v, float* buf) {
   return t;
 }
 
-// Sum of the block sums of one dot product, rounded as its fixed-point form
-// (2^(E-96), 2^E > max|a| max|b|) holds it; valid in thread 0.  The sums are
-// other blocks': read past L1.
-__device__ __forceinline__ double dot_total(const double* part, double* buf, unsigned long long abits,
-                                            unsigned long long bbits) {
-  double s = 0.0;
-  for (int q = threadIdx.x; q < kDotBlocks; q += 256) s += __ldcg(part + q);
-  buf[threadIdx.x] = s;
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) buf[threadIdx.x] += buf[threadIdx.x + h];
-    __syncthreads();
-  }
-  const double v = buf[0];
-  __syncthreads();
-  const double ma = __longlong_as_double((long long)abits), mb = __longlong_as_double((long long)bbits);
-  if (!(ma > 0.0) || !(mb > 0.0) || !(fabs(v) < INFINITY)) return 0.0;
-  const int E = ilogb(ma) + ilogb(mb) + 2;
+// The value of one dot product from the sum v of its block sums, rounded as
+// its fixed-point form (2^(E-96), 2^E > max|a| max|b|) holds it.
+__device__ __forceinline__ double dot_rounded(double v, unsigned long long abits, unsigned long long bbits) {
+  const unsigned long long inf_bits = 0x7FF0000000000000ull;
+  if (abits == 0 || bbits == 0 || abits > inf_bits || bbits > inf_bits || abs_bits(v) >= inf_bits) return 0.0;
+  // the maxima are widened FP32 values: normal, so ilogb is the exponent field
+  const int E = (int)(abits >> 52) + (int)(bbits >> 52) - 2 * 1023 + 2;
   const __int128 fx = fx_bits(v, 96 - E);
   const unsigned long long acc[2] = {(unsigned long long)fx, (unsigned long long)((unsigned __int128)fx >> 64)};
   return fx_unscale(acc, E);
+}
+// The part of a thread in the sum of a product's block sums.  The sums are
+// other blocks': read past L1.
+__device__ __forceinline__ double dot_share(const double* part) {
+  double s = 0.0;
+#pragma unroll
+  for (int q = 0; q < (kDotBlocks + 255) / 256; ++q) {
+    const int e = threadIdx.x + 256 * q;
+    if (e < kDotBlocks) s += __ldcg(part + e);
+  }
+  return s;
+}
+// The sum of 256 shares by halving (t + 128, t + 64, ...), by one warp; valid
+// in lane 0.
+__device__ __forceinline__ double dot_halve(const double* buf) {
+  const int l = threadIdx.x & 31;
+  double v = ((buf[l] + buf[l + 128]) + (buf[l + 64] + buf[l + 192])) +
+             ((buf[l + 32] + buf[l + 160]) + (buf[l + 96] + buf[l + 224]));
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+  return v;
 }
 
 // One pass over the vectors and the scalar they give, by the block that ends
 // last.  STAGE 0, after the first cycle: p = z, rz = r.z; 1: alpha = rz / p.q
 // (a = p, b = q); 2: beta = -(alpha z.q) / rz, rz = r.z (a = z, b = q, c = r).
 // 0 and 2 also take max|z|.  Clears the maxima that are read here and reduced
-// into next.
+// into next.  The last block is what a small grid waits for: its two totals go
+// to a warp each, with FP64 instructions in one warp where 256 threads halving
+// in steps issued them in eight (64^3: 11 and 22 us for stages 1 and 2 so,
+// 9 and 16 now).
 template <int STAGE>
 __global__ void __launch_bounds__(256) k_pcg_dot(const float* __restrict__ a, const float* __restrict__ b,
                                                  const float* __restrict__ c, float* __restrict__ p, i64 count,
                                                  double* part, PcgDev* P) {
   __shared__ float buf[32], buf2[32];
-  __shared__ double dbuf[256];
+  __shared__ double dbuf[2][256], total[2];
   __shared__ int last;
   const i64 stride = (i64)gridDim.x * blockDim.x;
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -173,8 +185,19 @@ __global__ void __launch_bounds__(256) k_pcg_dot(const float* __restrict__ a, co
   __threadfence();
   const unsigned long long rb = __ldcg(&P->rbits), zb = __ldcg(&P->zbits), qb = __ldcg(&P->qbits),
                            pb = __ldcg(&P->pbits);
-  const double first = STAGE == 0 ? 0.0 : dot_total(part, dbuf, STAGE == 1 ? pb : zb, qb);
-  const double rz = STAGE == 1 ? 0.0 : dot_total(part + kDotBlocks, dbuf, rb, zb);
+  if (STAGE != 0) dbuf[0][threadIdx.x] = dot_share(part);
+  if (STAGE != 1) dbuf[1][threadIdx.x] = dot_share(part + kDotBlocks);
+  __syncthreads();
+  if (threadIdx.x < 64) {
+    const int w = threadIdx.x >> 5;
+    if (w == 0 ? STAGE != 0 : STAGE != 1) {
+      const double v = dot_halve(dbuf[w]);
+      if ((threadIdx.x & 31) == 0)
+        total[w] = w == 0 ? dot_rounded(v, STAGE == 1 ? pb : zb, qb) : dot_rounded(v, rb, zb);
+    }
+  }
+  __syncthreads();
+  const double first = STAGE == 0 ? 0.0 : total[0], rz = STAGE == 1 ? 0.0 : total[1];
   if (threadIdx.x == 0) {
     P->arrived = 0;
     if constexpr (STAGE == 1) {
