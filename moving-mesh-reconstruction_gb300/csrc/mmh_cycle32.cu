@@ -356,6 +356,22 @@ __device__ void cycle(const Me& me, int base, int cube, Shared* sh, float dx2, c
   sweeps<N>(me, base, dx2, a.nu2);
 }
 
+// Asynchronous copies of single words into shared memory.  A cycle on its own
+// (below a 64^3 level) reads 100 words per thread before it starts; through
+// registers they came a few at a time and took as long as half the cycle, so
+// all are in flight at once.
+__device__ __forceinline__ void cp_word(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(__cvta_generic_to_global(src))
+               : "memory");
+}
+__device__ __forceinline__ void cp_word(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(__cvta_generic_to_global(src))
+               : "memory");
+}
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // fields of a slab level from global memory
 template <int N>
 __device__ void load_coef(float* w, int rank, const float* coef) {
@@ -364,13 +380,13 @@ __device__ void load_coef(float* w, int rank, const float* coef) {
   for (int e = threadIdx.x; e < (S::PP + 2) * S::PL; e += kThreads) {
     const int d = e / S::PL, x = e % N, y = (e / N) % N, k = (rank * S::PP + d - 1) & (N - 1);
     const int g = k * S::PL + y * N + x, o = d * S::PL + at<N>(x, y);
-    w[S::F3 + o] = coef[2 * n3 + g];
-    w[S::F5 + o] = coef[4 * n3 + g];
-    w[S::F6 + o] = coef[5 * n3 + g];
+    cp_word(w + S::F3 + o, coef + 2 * n3 + g);
+    cp_word(w + S::F5 + o, coef + 4 * n3 + g);
+    cp_word(w + S::F6 + o, coef + 5 * n3 + g);
     if (d >= 1 && d <= S::PP) {
-      w[S::F1 + o - S::PL] = coef[g];
-      w[S::F2 + o - S::PL] = coef[n3 + g];
-      w[S::F4 + o - S::PL] = coef[3 * n3 + g];
+      cp_word(w + S::F1 + o - S::PL, coef + g);
+      cp_word(w + S::F2 + o - S::PL, coef + n3 + g);
+      cp_word(w + S::F4 + o - S::PL, coef + 3 * n3 + g);
     }
   }
 }
@@ -379,7 +395,7 @@ __device__ void load_rhs(float* w, int rank, const float* rhs) {
   typedef Slab<N> S;
   for (int e = threadIdx.x; e < S::PP * S::PL; e += kThreads) {
     const int q = e / S::PL, x = e % N, y = (e / N) % N;
-    w[S::RHS + q * S::PL + at<N>(x, y)] = rhs[(rank * S::PP + q) * S::PL + y * N + x];
+    cp_word(w + S::RHS + q * S::PL + at<N>(x, y), rhs + (rank * S::PP + q) * S::PL + y * N + x);
   }
 }
 
@@ -406,9 +422,9 @@ __device__ __forceinline__ Me setup(Shared*& sh, const CycleArgs& a, unsigned ch
     float* f = me.w + Layout<N>::CUBE + Cube8::F;
     for (int e = threadIdx.x; e < 6 * 512; e += kThreads) {
       const int x = e & 7, y = (e >> 3) & 7;
-      f[(e & ~63) + at<8>(x, y)] = a.coef[2][e];
+      cp_word(f + (e & ~63) + at<8>(x, y), a.coef[2] + e);
     }
-    for (int e = threadIdx.x; e < 64 * 64; e += kThreads) sh->M[(e & 63) * 64 + (e >> 6)] = a.M[e];
+    for (int e = threadIdx.x; e < 64 * 64; e += kThreads) cp_word(sh->M + (e & 63) * 64 + (e >> 6), a.M + e);
   }
   return me;
 }
@@ -422,6 +438,7 @@ __global__ void __launch_bounds__(kThreads) k_cycle32(CycleArgs a, const float* 
   Shared* sh;
   Me me = setup<N>(sh, a, raw);
   load_rhs<N>(me.w, me.rank, rhs);
+  cp_wait();  // visible to the CTA at the cycle's first barrier
   cycle<N>(me, 0, Layout<N>::CUBE, sh, a.dx2, a);
   for (int e = threadIdx.x; e < S::PP * S::PL; e += kThreads) {
     const int q = e / S::PL, x = e % N, y = (e / N) % N;
@@ -485,6 +502,7 @@ __global__ void __launch_bounds__(kThreads) k_solve32(CycleArgs a, float* __rest
   Shared* sh;
   Me me = setup<N>(sh, a, raw);
   load_rhs<N>(me.w, me.rank, rhs);
+  cp_wait();  // visible to the CTA at the cycle's first barrier
   float* w = me.w;
   float* r = w + S::RHS;
   const float* z = w + S::PHI + S::PL;
