@@ -49,21 +49,6 @@ namespace {
 // ---------------------------------------------------------------------------
 constexpr int kRowThreads = 256;
 
-__device__ __forceinline__ bool mid_exp(double x) {
-  const int e = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
-  return e > 623 && e < 1423;
-}
-// num / d with y the correctly rounded 1 / d: two corrected steps from num * y
-// (the first gives a faithful quotient, the second then the correctly rounded
-// one, Markstein 1990); away from the middle of the exponent range the
-// division itself.
-__device__ __forceinline__ double div_by(double num, double d, double y) {
-  if (!(mid_exp(d) && mid_exp(num))) return num / d;
-  double q = num * y;
-  q = __fma_rn(__fma_rn(-d, q, num), y, q);
-  return __fma_rn(__fma_rn(-d, q, num), y, q);
-}
-
 // Offsets of a cell's neighbours from its plane's first element
 struct Nbr {
   i64 c, xp, xm, yp, ym;

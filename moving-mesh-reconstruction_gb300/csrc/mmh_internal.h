@@ -29,9 +29,10 @@ template <class T> inline int kk(int base) { return base | (sizeof(T) == 4 ? KK_
 // Launchers, instantiated for double (mmh_kernels_f64.cu, no FMA contraction)
 // and float (mmh_kernels_f32.cu).
 // fast_div: one division per cell (the mixed form); false: the reference's
-// operations, bit for bit
+// operations, bit for bit.  det (may be null): launch_det's output as well
 template <class T>
-void launch_metric(const T* def, const T* rho, int n, T dx, T* coef, cudaStream_t s, bool fast_div = false);
+void launch_metric(const T* def, const T* rho, int n, T dx, T* coef, cudaStream_t s, bool fast_div = false,
+                   T* det = nullptr);
 void launch_residual_fma(const double* phi, const double* rhs, const double* coef, int n, double dx, float* r32,
                          unsigned long long* maxbits, cudaStream_t s);
 // nsweeps 8-colour sweeps of phi; returns the buffer that holds the swept
@@ -139,10 +140,12 @@ void launch_spec_unpack(const void* z, int n, double* out, const LimDev* st, cud
 void launch_fft_tables(double* tab, int n, cudaStream_t s);
 void launch_spectral_lines(const double* src, int n, double* grad, double* delta, const double* tab, double* T,
                            cudaStream_t s);
+// rcc (may be null): receives 1 / cc, and baj's first six planes the metric
+// times det, both for launch_relax_flux (which is then given it too)
 void launch_relax_stage1(const double* rho, const double* def, const double* defp, int n, double* baj, double* cc,
-                         double* sd, cudaStream_t s, bool fast_div = false);
+                         double* sd, cudaStream_t s, bool fast_div = false, double* rcc = nullptr);
 void launch_relax_flux(const double* u1, const double* defp, const double* baj, const double* cc, int n, double* sd,
-                       cudaStream_t s, bool fast_div = false);
+                       cudaStream_t s, bool fast_div = false, const double* rcc = nullptr);
 void launch_relax_dpv(const double* sd, const double* cc, int n, const double* ubase, double dt, double* out,
                       double* gface, cudaStream_t s);
 // the mixed form's relaxing of the density (mmh_relax32.cu): FP32 fluxes, FP64

@@ -193,12 +193,60 @@ __device__ __forceinline__ float from_bits(unsigned b) { return __uint_as_float(
 __device__ __forceinline__ double from_bits(unsigned long long b) { return __longlong_as_double((long long)b); }
 
 // ---------------------------------------------------------------------------
+// FP64 operations off the FP64 pipe.  One FP64 warp instruction occupies its SM
+// quarter for 64 cycles, an integer one for 1 to 2, so exact operations (a
+// scaling by a power of two, a sign) are done on the bits; values for which
+// they would not be exact take the operation itself in a function of its own:
+// inlined, the compiler would execute it always and select.
+// ---------------------------------------------------------------------------
+// biased binary exponent: 0 for zero and subnormals, 2047 for inf and NaN
+__device__ __forceinline__ int bexp(double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7ff); }
+static __device__ __noinline__ double slow_mul(double a, double b) { return a * b; }
+static __device__ __noinline__ double slow_div(double a, double b) { return a / b; }
+// x 2^-K with the same bits as the product
+template <int K>
+__device__ __forceinline__ double pow2_down(double x) {
+  const int e = bexp(x);
+  if (e > K && e < 2047) return __longlong_as_double(__double_as_longlong(x) - ((i64)K << 52));
+  if (abs_bits(x) == 0) return x;
+  return slow_mul(x, 1.0 / (1 << K));
+}
+__device__ __forceinline__ double half_of(double x) { return pow2_down<1>(x); }
+__device__ __forceinline__ float quarter_of(float x) { return x * 0.25f; }
+__device__ __forceinline__ double quarter_of(double x) { return pow2_down<2>(x); }
+__device__ __forceinline__ bool mid_exp(double x) {
+  const int e = bexp(x);
+  return e > 623 && e < 1423;
+}
+// num / d with y the correctly rounded 1 / d: two corrected steps from num * y
+// (the first gives a faithful quotient, the second then the correctly rounded
+// one, Markstein 1990); zero by its sign; away from the middle of the exponent
+// range the division itself.
+__device__ __forceinline__ double div_by(double num, double d, double y) {
+  if (mid_exp(d)) {
+    if (mid_exp(num)) {
+      double q = __dmul_rn(num, y);
+      q = __fma_rn(__fma_rn(-d, q, num), y, q);
+      return __fma_rn(__fma_rn(-d, q, num), y, q);
+    }
+    if (abs_bits(num) == 0)
+      return __longlong_as_double((__double_as_longlong(num) ^ __double_as_longlong(d)) & (i64)0x8000000000000000ull);
+  }
+  return slow_div(num, d);
+}
+
+// ---------------------------------------------------------------------------
 // Curvilinear metric (cbajraw, mmh/gauss1.f90:1107-1210, non-lsquare branch)
 // ---------------------------------------------------------------------------
 // FastDiv (the mixed form, which is not bit-matched): urg/det once, then six
-// multiplications instead of six divisions.
+// multiplications instead of six divisions.  The FP64 form is bound by the FP64
+// pipe: its seven divisions have two denominators and go by their reciprocals,
+// halvings and the products with di2 = 1 are left out, and det (before the
+// replacement below; may be null) is what k_det would compute again.  256^3:
+// 4.5 ms before, 4.0 now, and the 1.4 ms of k_det saved.
 template <class T, bool FastDiv = false>
-__global__ void k_metric(const T* __restrict__ def, const T* __restrict__ rho, int n, T di2, T* __restrict__ coef) {
+__global__ void k_metric(const T* __restrict__ def, const T* __restrict__ rho, int n, T di2, T* __restrict__ coef,
+                         T* __restrict__ det_out) {
   i64 n3 = (i64)n * n * n;
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n3) return;
@@ -206,14 +254,22 @@ __global__ void k_metric(const T* __restrict__ def, const T* __restrict__ rho, i
   cell_of(t, n, i, j, k);
   int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
   T c = def[t];
-  T phixx = (def[IDX(ip, j, k, n)] - T(2) * c + def[IDX(im, j, k, n)]) * di2;
-  T phiyy = (def[IDX(i, jp, k, n)] - T(2) * c + def[IDX(i, jm, k, n)]) * di2;
-  T phizz = (def[IDX(i, j, kp, n)] - T(2) * c + def[IDX(i, j, km, n)]) * di2;
-  T phixy = (def[IDX(ip, jp, k, n)] - def[IDX(im, jp, k, n)] - def[IDX(ip, jm, k, n)] + def[IDX(im, jm, k, n)]) * di2 * T(0.25);
-  T phiyz = (def[IDX(i, jp, kp, n)] - def[IDX(i, jp, km, n)] - def[IDX(i, jm, kp, n)] + def[IDX(i, jm, km, n)]) * di2 * T(0.25);
-  T phixz = (def[IDX(ip, j, kp, n)] - def[IDX(im, j, kp, n)] - def[IDX(ip, j, km, n)] + def[IDX(im, j, km, n)]) * di2 * T(0.25);
+  T phixx = (def[IDX(ip, j, k, n)] - T(2) * c + def[IDX(im, j, k, n)]);
+  T phiyy = (def[IDX(i, jp, k, n)] - T(2) * c + def[IDX(i, jm, k, n)]);
+  T phizz = (def[IDX(i, j, kp, n)] - T(2) * c + def[IDX(i, j, km, n)]);
+  T phixy = (def[IDX(ip, jp, k, n)] - def[IDX(im, jp, k, n)] - def[IDX(ip, jm, k, n)] + def[IDX(im, jm, k, n)]);
+  T phiyz = (def[IDX(i, jp, kp, n)] - def[IDX(i, jp, km, n)] - def[IDX(i, jm, kp, n)] + def[IDX(i, jm, km, n)]);
+  T phixz = (def[IDX(ip, j, kp, n)] - def[IDX(im, j, kp, n)] - def[IDX(ip, j, km, n)] + def[IDX(im, j, km, n)]);
+  if (di2 != T(1)) {
+    phixx *= di2; phiyy *= di2; phizz *= di2;
+    phixy *= di2; phiyz *= di2; phixz *= di2;
+  }
+  phixy = quarter_of(phixy);
+  phiyz = quarter_of(phiyz);
+  phixz = quarter_of(phixz);
   T a11 = T(1) + phixx, a12 = phixy, a13 = phixz, a22 = T(1) + phiyy, a23 = phiyz, a33 = T(1) + phizz;
   T det = a11 * a22 * a33 + T(2) * a12 * a13 * a23 - a13 * a13 * a22 - a11 * (a23 * a23) - a12 * a12 * a33;
+  if (det_out) det_out[t] = det;
   T b11 = (a22 * a33 - a23 * a23);
   T b12 = (a13 * a23 - a12 * a33);
   T b13 = (a12 * a23 - a13 * a22);
@@ -234,6 +290,17 @@ __global__ void k_metric(const T* __restrict__ def, const T* __restrict__ rho, i
         if (a == 0 && b == 0 && d == 0) continue;
         urg = urg + rho[IDX(is[a], js[b], ks[d], n)];
       }
+  if constexpr (std::is_same<T, double>::value && !FastDiv) {
+    urg = div_by(urg, 27.0, 1.0 / 27.0);
+    const double y = 1.0 / det;
+    coef[0 * n3 + t] = div_by(urg * b11, det, y);
+    coef[1 * n3 + t] = div_by(urg * b12, det, y);
+    coef[2 * n3 + t] = div_by(urg * b13, det, y);
+    coef[3 * n3 + t] = div_by(urg * b22, det, y);
+    coef[4 * n3 + t] = div_by(urg * b23, det, y);
+    coef[5 * n3 + t] = div_by(urg * b33, det, y);
+    return;
+  }
   urg = urg / T(27);
   if (FastDiv) {
     const T w = urg / det;
@@ -1220,12 +1287,19 @@ __global__ void k_det(const T* __restrict__ def, int n, T di2, T* __restrict__ d
   cell_of(t, n, i, j, k);
   int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
   T c = def[t];
-  T phixx = (def[IDX(ip, j, k, n)] - T(2) * c + def[IDX(im, j, k, n)]) * di2;
-  T phiyy = (def[IDX(i, jp, k, n)] - T(2) * c + def[IDX(i, jm, k, n)]) * di2;
-  T phizz = (def[IDX(i, j, kp, n)] - T(2) * c + def[IDX(i, j, km, n)]) * di2;
-  T phixy = (def[IDX(ip, jp, k, n)] - def[IDX(im, jp, k, n)] - def[IDX(ip, jm, k, n)] + def[IDX(im, jm, k, n)]) * di2 * T(0.25);
-  T phiyz = (def[IDX(i, jp, kp, n)] - def[IDX(i, jp, km, n)] - def[IDX(i, jm, kp, n)] + def[IDX(i, jm, km, n)]) * di2 * T(0.25);
-  T phixz = (def[IDX(ip, j, kp, n)] - def[IDX(im, j, kp, n)] - def[IDX(ip, j, km, n)] + def[IDX(im, j, km, n)]) * di2 * T(0.25);
+  T phixx = (def[IDX(ip, j, k, n)] - T(2) * c + def[IDX(im, j, k, n)]);
+  T phiyy = (def[IDX(i, jp, k, n)] - T(2) * c + def[IDX(i, jm, k, n)]);
+  T phizz = (def[IDX(i, j, kp, n)] - T(2) * c + def[IDX(i, j, km, n)]);
+  T phixy = (def[IDX(ip, jp, k, n)] - def[IDX(im, jp, k, n)] - def[IDX(ip, jm, k, n)] + def[IDX(im, jm, k, n)]);
+  T phiyz = (def[IDX(i, jp, kp, n)] - def[IDX(i, jp, km, n)] - def[IDX(i, jm, kp, n)] + def[IDX(i, jm, km, n)]);
+  T phixz = (def[IDX(ip, j, kp, n)] - def[IDX(im, j, kp, n)] - def[IDX(ip, j, km, n)] + def[IDX(im, j, km, n)]);
+  if (di2 != T(1)) {
+    phixx *= di2; phiyy *= di2; phizz *= di2;
+    phixy *= di2; phiyz *= di2; phixz *= di2;
+  }
+  phixy = quarter_of(phixy);
+  phiyz = quarter_of(phiyz);
+  phixz = quarter_of(phixz);
   T a11 = T(1) + phixx, a12 = phixy, a13 = phixz, a22 = T(1) + phiyy, a23 = phiyz, a33 = T(1) + phizz;
   det[t] = (a11 * a22 * a33 + T(2) * a12 * a13 * a23 - a13 * a13 * a22 - a11 * (a23 * a23) - a12 * a12 * a33);
 }

@@ -12,12 +12,12 @@ namespace mmh {
 // Limiter metric: cof(A)/det and det of A = I + Hess(def) at unit spacing
 // (limiter.f90:268-286, relaxing.f90:876-901).
 struct LimM {
-  double b11, b12, b13, b22, b23, b33, det;
+  double b11, b12, b13, b22, b23, b33, det, y;
   double phixx, phiyy, phizz, phixy, phiyz, phixz;
 };
 
 // FastDiv (the mixed form, which is not bit-matched): the six divisions by
-// det become one reciprocal and six multiplications.
+// det become one reciprocal and six multiplications; y = 1/det otherwise.
 template <bool FastDiv = false>
 __device__ __forceinline__ LimM lim_metric(const double* __restrict__ def, int n, int i, int j, int k) {
   int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
@@ -26,9 +26,9 @@ __device__ __forceinline__ LimM lim_metric(const double* __restrict__ def, int n
   m.phixx = (def[IDX(ip, j, k, n)] - 2.0 * c + def[IDX(im, j, k, n)]);
   m.phiyy = (def[IDX(i, jp, k, n)] - 2.0 * c + def[IDX(i, jm, k, n)]);
   m.phizz = (def[IDX(i, j, kp, n)] - 2.0 * c + def[IDX(i, j, km, n)]);
-  m.phixy = (def[IDX(ip, jp, k, n)] - def[IDX(im, jp, k, n)] - def[IDX(ip, jm, k, n)] + def[IDX(im, jm, k, n)]) * 0.25;
-  m.phiyz = (def[IDX(i, jp, kp, n)] - def[IDX(i, jp, km, n)] - def[IDX(i, jm, kp, n)] + def[IDX(i, jm, km, n)]) * 0.25;
-  m.phixz = (def[IDX(ip, j, kp, n)] - def[IDX(im, j, kp, n)] - def[IDX(ip, j, km, n)] + def[IDX(im, j, km, n)]) * 0.25;
+  m.phixy = quarter_of(def[IDX(ip, jp, k, n)] - def[IDX(im, jp, k, n)] - def[IDX(ip, jm, k, n)] + def[IDX(im, jm, k, n)]);
+  m.phiyz = quarter_of(def[IDX(i, jp, kp, n)] - def[IDX(i, jp, km, n)] - def[IDX(i, jm, kp, n)] + def[IDX(i, jm, km, n)]);
+  m.phixz = quarter_of(def[IDX(ip, j, kp, n)] - def[IDX(im, j, kp, n)] - def[IDX(ip, j, km, n)] + def[IDX(im, j, km, n)]);
   double a11 = 1.0 + m.phixx, a12 = m.phixy, a13 = m.phixz, a22 = 1.0 + m.phiyy, a23 = m.phiyz, a33 = 1.0 + m.phizz;
   double det = a11 * a22 * a33 + 2.0 * a12 * a13 * a23 - a13 * a13 * a22 - a11 * (a23 * a23) - a12 * a12 * a33;
   m.det = det;
@@ -41,12 +41,14 @@ __device__ __forceinline__ LimM lim_metric(const double* __restrict__ def, int n
     m.b23 = (a12 * a13 - a11 * a23) * r;
     m.b33 = (a11 * a22 - a12 * a12) * r;
   } else {
-    m.b11 = (a22 * a33 - a23 * a23) / det;
-    m.b12 = (a13 * a23 - a12 * a33) / det;
-    m.b13 = (a12 * a23 - a13 * a22) / det;
-    m.b22 = (a11 * a33 - a13 * a13) / det;
-    m.b23 = (a12 * a13 - a11 * a23) / det;
-    m.b33 = (a11 * a22 - a12 * a12) / det;
+    const double y = 1.0 / det;
+    m.b11 = div_by(a22 * a33 - a23 * a23, det, y);
+    m.b12 = div_by(a13 * a23 - a12 * a33, det, y);
+    m.b13 = div_by(a12 * a23 - a13 * a22, det, y);
+    m.b22 = div_by(a11 * a33 - a13 * a13, det, y);
+    m.b23 = div_by(a12 * a13 - a11 * a23, det, y);
+    m.b33 = div_by(a11 * a22 - a12 * a12, det, y);
+    m.y = y;
   }
   return m;
 }
@@ -60,9 +62,9 @@ __device__ __forceinline__ LimM lim_hess_det(const double* __restrict__ def, int
   m.phixx = (def[IDX(ip, j, k, n)] - 2.0 * c + def[IDX(im, j, k, n)]);
   m.phiyy = (def[IDX(i, jp, k, n)] - 2.0 * c + def[IDX(i, jm, k, n)]);
   m.phizz = (def[IDX(i, j, kp, n)] - 2.0 * c + def[IDX(i, j, km, n)]);
-  m.phixy = (def[IDX(ip, jp, k, n)] - def[IDX(im, jp, k, n)] - def[IDX(ip, jm, k, n)] + def[IDX(im, jm, k, n)]) * 0.25;
-  m.phiyz = (def[IDX(i, jp, kp, n)] - def[IDX(i, jp, km, n)] - def[IDX(i, jm, kp, n)] + def[IDX(i, jm, km, n)]) * 0.25;
-  m.phixz = (def[IDX(ip, j, kp, n)] - def[IDX(im, j, kp, n)] - def[IDX(ip, j, km, n)] + def[IDX(im, j, km, n)]) * 0.25;
+  m.phixy = quarter_of(def[IDX(ip, jp, k, n)] - def[IDX(im, jp, k, n)] - def[IDX(ip, jm, k, n)] + def[IDX(im, jm, k, n)]);
+  m.phiyz = quarter_of(def[IDX(i, jp, kp, n)] - def[IDX(i, jp, km, n)] - def[IDX(i, jm, kp, n)] + def[IDX(i, jm, km, n)]);
+  m.phixz = quarter_of(def[IDX(ip, j, kp, n)] - def[IDX(im, j, kp, n)] - def[IDX(ip, j, km, n)] + def[IDX(im, j, km, n)]);
   double a11 = 1.0 + m.phixx, a12 = m.phixy, a13 = m.phixz, a22 = 1.0 + m.phiyy, a23 = m.phiyz, a33 = 1.0 + m.phizz;
   m.det = a11 * a22 * a33 + 2.0 * a12 * a13 * a23 - a13 * a13 * a22 - a11 * (a23 * a23) - a12 * a12 * a33;
   m.b11 = m.b12 = m.b13 = m.b22 = m.b23 = m.b33 = 0.0;

@@ -374,7 +374,8 @@ bool ff_outer(const mmh_ctx* c) {
 // Build the coarse geometry (restricted def and density) and the metric of
 // every level from l0 down (FP64; FP32 copies for the mixed form, whose
 // finest level's metric is formed as float-float pairs when its outer loop
-// keeps them).
+// keeps them).  The FP64 form and the float-float metric leave det(A) of the
+// finest level in c->det.
 int build_levels(mmh_ctx* c, int l0) {
   for (int l = l0 + 1; l < c->nlev; ++l) {
     launch_restrict27<double>(c->defl[l - 1], c->nl[l - 1], c->defl[l], c->s);
@@ -392,7 +393,7 @@ int build_levels(mmh_ctx* c, int l0) {
       continue;
     }
     launch_metric<double>(c->defl[l], c->rhol[l], n, double(1 << l), c->h64.coef[l], c->s,
-                          c->cfg.precision == MMH_MIXED);
+                          c->cfg.precision == MMH_MIXED, l == l0 && c->cfg.precision == MMH_FP64 ? c->det : nullptr);
     if (c->cfg.precision == MMH_MIXED) launch_d2f(c->h64.coef[l], c->h32.coef[l], 6 * (i64)n * n * n, c->s);
     if (c->faces_at(l)) c->face[l] = launch_faces64(c->h64.coef[l], n, c->face0[l], c->face1[l], c->s);
   }
@@ -717,9 +718,10 @@ int multigrid_level(mmh_ctx* c, int l0, double dx, mmh_diag* d) {
   int n = c->nl[l0];
   i64 n3 = (i64)n * n * n;
   CK(cudaMemsetAsync(c->sc, 0, offsetof(Scal, lim), c->s));
-  // The mixed form's float-float metric also gives det(A) for rgzerosum, so
-  // the metric goes first there (it does not depend on rhs or u).
-  const bool det_from_metric = ff_outer(c) && l0 < c->nlev - 1 && dx == double(1 << l0);
+  // The float-float metric and the FP64 form's also give det(A) for
+  // rgzerosum, so the metric goes first there (it does not depend on rhs or u).
+  const bool det_from_metric =
+      (ff_outer(c) ? l0 < c->nlev - 1 : c->cfg.precision == MMH_FP64) && dx == double(1 << l0);
   const bool ready = c->levels_ready && l0 == 0;
   c->levels_ready = false;
   if (det_from_metric && !ready) RET(build_levels(c, l0));
@@ -940,9 +942,10 @@ int relaxing_dev(mmh_ctx* c, double dt, bool split = false) {
                    reinterpret_cast<float*>(c->u1), c->s);
     return MMH_OK;
   }
-  launch_relax_stage1(c->rho, c->def, c->defp(), n, c->baj, c->cc, c->vt, c->s);
+  double* rcc = c->tmp();  // 1 / cc
+  launch_relax_stage1(c->rho, c->def, c->defp(), n, c->baj, c->cc, c->vt, c->s, false, rcc);
   launch_relax_dpv(c->vt, c->cc, n, c->rho, dt / 2.0, c->u1, c->gface, c->s);
-  launch_relax_flux(c->u1, c->defp(), c->baj, c->cc, n, c->vt, c->s);
+  launch_relax_flux(c->u1, c->defp(), c->baj, c->cc, n, c->vt, c->s, false, rcc);
   launch_relax_dpv(c->vt, c->cc, n, c->rho, dt, c->rho, c->gface, c->s);
   return MMH_OK;
 }
