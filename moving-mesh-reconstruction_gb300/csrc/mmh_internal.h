@@ -252,8 +252,10 @@ void launch_adj_limiter(const double* def, const double* defps, const double* pw
                         double dtold, double* abar, cudaStream_t s);
 void launch_adj_axpy(const double* a, double sc, const double* b, double* out, i64 n3, cudaStream_t s);
 void launch_adj_alpha(const double* baj, const double* defp, const double* cc, int n, double* alpha, cudaStream_t s);
+// fa (7 n^3) and cb (n^3): scratch
 void launch_adj_dpv(const double* sd, const double* cc, const double* alpha, const double* x, const double* rbar,
-                    double scale, int n, double* xbar, double* alphabar, double* cbar, cudaStream_t s);
+                    double scale, int n, double* xbar, double* alphabar, double* cbar, double* fa, double* cb,
+                    cudaStream_t s);
 void launch_adj_relax_geom(const double* def, const double* defp, const double* cc, const double* alphabar,
                            const double* cbar, int n, double* abar, double* pdbar, cudaStream_t s);
 void launch_adj_grad_t(const double* pdbar, int n, double* out, int add, cudaStream_t s);

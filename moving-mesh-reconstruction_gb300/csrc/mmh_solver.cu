@@ -1168,8 +1168,8 @@ int relaxing_adjoint_dev(mmh_ctx* c, double dt, const double* ubar, double* gu, 
   launch_relax_flux(c->u1, defp, c->baj, c->cc, n, sd1, c->s, fast);
   // stage 2 (u' = u - dt R(u1)), then stage 1 (u1 = u - dt/2 R(u))
   CK(cudaMemsetAsync(alphabar, 0, sizeof(double) * 4 * n3, c->s));
-  launch_adj_dpv(sd1, c->cc, alpha, c->u1, ubar, -dt, n, u1bar, alphabar, cbar, c->s);
-  launch_adj_dpv(sd0, c->cc, alpha, c->rho, u1bar, -dt / 2.0, n, xbar, alphabar, cbar, c->s);
+  launch_adj_dpv(sd1, c->cc, alpha, c->u1, ubar, -dt, n, u1bar, alphabar, cbar, c->baj, c->gface, c->s);
+  launch_adj_dpv(sd0, c->cc, alpha, c->rho, u1bar, -dt / 2.0, n, xbar, alphabar, cbar, c->baj, c->gface, c->s);
   CK(cudaMemcpyAsync(gu, ubar, sizeof(double) * n3, cudaMemcpyDeviceToDevice, c->s));
   launch_add(gu, u1bar, n3, c->s);
   launch_add(gu, xbar, n3, c->s);
