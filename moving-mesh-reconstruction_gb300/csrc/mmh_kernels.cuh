@@ -193,6 +193,52 @@ __device__ __forceinline__ float from_bits(unsigned b) { return __uint_as_float(
 __device__ __forceinline__ double from_bits(unsigned long long b) { return __longlong_as_double((long long)b); }
 
 // ---------------------------------------------------------------------------
+// Launches of the kernels that an iteration runs by the hundred.  They begin
+// with pdl_begin and are launched by launch or launch_cluster with programmatic
+// stream serialisation: their blocks may be placed while the kernel before
+// drains, and then wait until it has completed and its stores are visible.
+// Nothing comes before the wait, so the order of a stream is what it was; what
+// goes is part of the gap between two kernels (1.5 us: four iterations at 32^3 in
+// the mixed form 4.6 ms, 4.2 so).  Not for kernels inside the captured cycles nor
+// for those with much shared memory: FP64 solves became 3 to 8% slower, a batch
+// of realisations on several streams 11%.
+//   A kernel without pdl_begin must not be launched this way, and a kernel with
+// it takes no __restrict__ parameters and uses no __ldg: its inputs may still
+// be written while its first blocks wait, which non-coherent loads do not
+// allow.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// cluster: CTAs per cluster along x (0: none)
+template <class... P, class... A>
+void launch_cluster(void (*kernel)(P...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                    A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 1;
+  if (cluster) {
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  cfg.attrs = at;
+  cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  launch_cluster(kernel, 0, grid, block, smem, s, std::forward<A>(args)...);
+}
+
+// ---------------------------------------------------------------------------
 // FP64 operations off the FP64 pipe.  One FP64 warp instruction occupies its SM
 // quarter for 64 cycles, an integer one for 1 to 2, so exact operations (a
 // scaling by a power of two, a sign) are done on the bits; values for which
@@ -1201,7 +1247,8 @@ __device__ __forceinline__ T smooth27(const T* __restrict__ a, int n, int i, int
 }
 
 template <class T>
-__global__ void k_restrict27(const T* __restrict__ fine, int n, T* __restrict__ coarse) {
+__global__ void k_restrict27(const T* fine, int n, T* coarse) {
+  pdl_begin();
   int nh = n >> 1;
   i64 tot = (i64)nh * nh * nh;
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1265,7 +1312,8 @@ __global__ void k_prolong_add_blk(T* __restrict__ u, const T* __restrict__ uh, i
 
 // Exact sum of a[0..count) into acc (lo, hi); flag |= 1 on a term out of range.
 template <class T>
-__global__ void k_fxsum(const T* __restrict__ a, i64 count, unsigned long long* acc, int* flag) {
+__global__ void k_fxsum(const T* a, i64 count, unsigned long long* acc, int* flag) {
+  pdl_begin();
   __int128 s = 0;
   bool bad = false;
   for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (i64)gridDim.x * blockDim.x) {
@@ -1279,7 +1327,8 @@ __global__ void k_fxsum(const T* __restrict__ a, i64 count, unsigned long long* 
 
 // det of I + Hess(def)/dx^2 without the tangle fallback (rgzerosum gauss1.f90:1390-1402)
 template <class T>
-__global__ void k_det(const T* __restrict__ def, int n, T di2, T* __restrict__ det) {
+__global__ void k_det(const T* def, int n, T di2, T* det) {
+  pdl_begin();
   i64 n3 = (i64)n * n * n;
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n3) return;
@@ -1317,7 +1366,8 @@ __global__ void k_sub_mean(T* __restrict__ a, i64 count, const double* __restric
 
 // rhs = rhs - dfact * det, dfact rounded to T (rgzerosum)
 template <class T>
-__global__ void k_sub_dfact(T* __restrict__ a, const T* __restrict__ det, i64 count, const double* __restrict__ ratio) {
+__global__ void k_sub_dfact(T* a, const T* det, i64 count, const double* ratio) {
+  pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   T dfact = (T)(*ratio);
@@ -1325,7 +1375,8 @@ __global__ void k_sub_dfact(T* __restrict__ a, const T* __restrict__ det, i64 co
 }
 
 template <class T>
-__global__ void k_fill(T* __restrict__ a, i64 count, T v) {
+__global__ void k_fill(T* a, i64 count, T v) {
+  pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < count) a[t] = v;
 }
@@ -1338,8 +1389,9 @@ __global__ void k_zero_if(T* __restrict__ a, i64 count, const int* __restrict__ 
   if (t < count) a[t] = T(0);
 }
 template <class T>
-__global__ void k_sub_mean_unless(T* __restrict__ a, i64 count, const double* __restrict__ mean,
-                                  const int* __restrict__ flag) {
+__global__ void k_sub_mean_unless(T* a, i64 count, const double* mean,
+                                  const int* flag) {
+  pdl_begin();
   if (*flag != 0) return;
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;

@@ -104,17 +104,19 @@ MMH_INSTANTIATE(double)
 // scalar helpers
 // ---------------------------------------------------------------------------
 __global__ void k_fx_mean(const unsigned long long* acc, double count, double* out) {
+  pdl_begin();
   *out = fx_to(acc[0], acc[1]) / count;
 }
 __global__ void k_fx_ratio(const unsigned long long* num, const unsigned long long* den, double* out) {
+  pdl_begin();
   *out = fx_to(num[0], num[1]) / fx_to(den[0], den[1]);
 }
 void launch_fx_mean(const unsigned long long* acc, double count, double* out, cudaStream_t s) {
-  k_fx_mean<<<1, 1, 0, s>>>(acc, count, out);
+  launch(k_fx_mean, 1, 1, 0, s, acc, count, out);
   count_launch();
 }
 void launch_fx_ratio(const unsigned long long* num, const unsigned long long* den, double* out, cudaStream_t s) {
-  k_fx_ratio<<<1, 1, 0, s>>>(num, den, out);
+  launch(k_fx_ratio, 1, 1, 0, s, num, den, out);
   count_launch();
 }
 
@@ -132,7 +134,8 @@ void launch_guard(const unsigned long long* r1bits, const unsigned long long* er
   count_launch();
 }
 
-__global__ void k_d2f(const double* __restrict__ a, float* __restrict__ b, i64 count) {
+__global__ void k_d2f(const double* a, float* b, i64 count) {
+  pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < count) b[t] = (float)a[t];
 }
@@ -149,7 +152,7 @@ __global__ void k_add(double* __restrict__ a, const double* __restrict__ b, i64 
   if (t < count) a[t] = a[t] + b[t];
 }
 void launch_d2f(const double* a, float* b, i64 count, cudaStream_t s) {
-  k_d2f<<<grid_of(count, kBlock), kBlock, 0, s>>>(a, b, count);
+  launch(k_d2f, grid_of(count, kBlock), kBlock, 0, s, a, b, count);
   count_launch();
 }
 void launch_f2d(const float* a, double* b, i64 count, cudaStream_t s) {
@@ -177,8 +180,9 @@ constexpr int kCoarseN = 64;
 // whole matrix is bound by its FP64 pipe (5000 cycles per step): 344 us per
 // metric, this form 63 us.  The same operations per entry, so the same bits.
 constexpr int kInvCtas = 16;
-__global__ void __launch_bounds__(256) k_coarse_inverse(const double* __restrict__ coef, double di2,
-                                                        double* __restrict__ M) {
+__global__ void __launch_bounds__(256) k_coarse_inverse(const double* coef, double di2,
+                                                        double* M) {
+  pdl_begin();
   constexpr int N = kCoarseN;
   __shared__ double unit[N][N];
   __shared__ double diag[N], rowbuf[2][N], colp[2][4];
@@ -248,17 +252,7 @@ __global__ void __launch_bounds__(64) k_coarse_apply(const float* __restrict__ r
 void launch_coarse_inverse(const double* coef, double dx, double* M, cudaStream_t s) {
   static std::atomic<unsigned long long> attr_done{0};
   func_attr_once(k_coarse_inverse, cudaFuncAttributeNonPortableClusterSizeAllowed, 1, attr_done);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kInvCtas);
-  cfg.blockDim = dim3(256);
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kInvCtas;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_coarse_inverse, coef, 1.0 / (dx * dx), M);
+  launch_cluster(k_coarse_inverse, kInvCtas, kInvCtas, 256, 0, s, coef, 1.0 / (dx * dx), M);
   count_launch();
 }
 void launch_coarse_apply(const float* r, const double* M, float* z, cudaStream_t s) {
@@ -282,8 +276,9 @@ void launch_add(double* a, const double* b, i64 count, cudaStream_t s) {
 // form multiplies by 1 / (30 dtold) instead of dividing twice (an FP64
 // division is some ten FP64-pipe operations): within 2 ulp.
 template <bool MIXED>
-__global__ void k_calcdefp_rhs(double* __restrict__ tmp, const double* __restrict__ rho, i64 n3, double dtold,
+__global__ void k_calcdefp_rhs(double* tmp, const double* rho, i64 n3, double dtold,
                                double rcp) {
+  pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n3) return;
   double t1 = 1.0 - rho[t];
@@ -293,16 +288,16 @@ __global__ void k_calcdefp_rhs(double* __restrict__ tmp, const double* __restric
     t1 = t1 * rcp;
   } else {
     t1 = div_by(t1, 30.0, 1.0 / 30.0);
-    if (dtold != 1.0) t1 = t1 / dtold;
+    if (dtold != 1.0) t1 = slow_div(t1, dtold);
   }
   tmp[t] = t1;
 }
 void launch_calcdefp_rhs(double* tmp, const double* rho, int n, double dtold, bool mixed, cudaStream_t s) {
   i64 n3 = (i64)n * n * n;
   if (mixed)
-    k_calcdefp_rhs<true><<<grid_of(n3, kBlock), kBlock, 0, s>>>(tmp, rho, n3, dtold, 1.0 / (30.0 * dtold));
+    launch(k_calcdefp_rhs<true>, grid_of(n3, kBlock), kBlock, 0, s, tmp, rho, n3, dtold, 1.0 / (30.0 * dtold));
   else
-    k_calcdefp_rhs<false><<<grid_of(n3, kBlock), kBlock, 0, s>>>(tmp, rho, n3, dtold, 0.0);
+    launch(k_calcdefp_rhs<false>, grid_of(n3, kBlock), kBlock, 0, s, tmp, rho, n3, dtold, 0.0);
   count_launch();
 }
 
@@ -405,6 +400,9 @@ __device__ __forceinline__ void pass1_commit(LimDev* st, unsigned long long nexp
   fx_block_commit(r2, st->rho2);
 }
 
+// Pass-1 flux limiter for a density-only state (u(2:5) = 0, so the
+// momentum-flux divergence is zero): limiter.f90:238-381.  The flux of cell
+// (i,j,km) is tested with the metric of plane k = km+1.
 __global__ void k_limiter_pass1(double* __restrict__ tmp, const double* __restrict__ def,
                                 const double* __restrict__ rho, int n, double dtold, double lim,
                                 double cmpmaxglobal, double gthr, LimDev* st, uint8_t* __restrict__ maskx,
@@ -831,6 +829,7 @@ void launch_limiter_mask_mixed(double* defplim, const double* def, const double*
 }
 
 __global__ void k_lim_reset(LimDev* st) {
+  pdl_begin();
   st->nexpand = 0;
   st->ncompress = 0;
   st->detmax = ord_of(0.0);
@@ -1050,8 +1049,9 @@ void launch_metric_ff(const float2* def, const float2* rho, int n, double dx, do
 }
 
 // float-float splits of two fields (b may be null)
-__global__ void k_ff_split2(const double* __restrict__ a, float2* __restrict__ as, const double* __restrict__ b,
-                            float2* __restrict__ bs, i64 count) {
+__global__ void k_ff_split2(const double* a, float2* as, const double* b,
+                            float2* bs, i64 count) {
+  pdl_begin();
   const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const FF v = ff_of_bits(a[t]);
@@ -1062,8 +1062,9 @@ __global__ void k_ff_split2(const double* __restrict__ a, float2* __restrict__ a
   }
 }
 // def = def + defp, and the splits of both
-__global__ void k_add_split(double* __restrict__ def, const double* __restrict__ defp, float2* __restrict__ defs,
-                            float2* __restrict__ defps, i64 count) {
+__global__ void k_add_split(double* def, const double* defp, float2* defs,
+                            float2* defps, i64 count) {
+  pdl_begin();
   const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const double p = defp[t], d = def[t] + p;
@@ -1073,36 +1074,40 @@ __global__ void k_add_split(double* __restrict__ def, const double* __restrict__
   defps[t] = make_float2(w.hi, w.lo);
 }
 void launch_ff_split2(const double* a, float2* as, const double* b, float2* bs, i64 count, cudaStream_t s) {
-  k_ff_split2<<<grid_of(count, kBlock), kBlock, 0, s>>>(a, as, b, bs, count);
+  launch(k_ff_split2, grid_of(count, kBlock), kBlock, 0, s, a, as, b, bs, count);
   count_launch();
 }
 void launch_add_split(double* def, const double* defp, float2* defs, float2* defps, i64 count, cudaStream_t s) {
-  k_add_split<<<grid_of(count, kBlock), kBlock, 0, s>>>(def, defp, defs, defps, count);
+  launch(k_add_split, grid_of(count, kBlock), kBlock, 0, s, def, defp, defs, defps, count);
   count_launch();
 }
 
 // in place: doubles -> (hi, lo) pairs in the same 8 bytes, and back
-__global__ void k_ff_split(double* __restrict__ a, i64 count) {
+__global__ void k_ff_split(double* a, i64 count) {
+  pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   FF v = ff_of_bits(a[t]);
   reinterpret_cast<float2*>(a)[t] = make_float2(v.hi, v.lo);
 }
-__global__ void k_ff_join(double* __restrict__ a, i64 count) {
+__global__ void k_ff_join(double* a, i64 count) {
+  pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   float2 v = reinterpret_cast<const float2*>(a)[t];
   a[t] = (double)v.x + (double)v.y;
 }
 // x += e (float) ; x -= mean (double)
-__global__ void k_ff_add_f(float2* __restrict__ x, const float* __restrict__ e, i64 count) {
+__global__ void k_ff_add_f(float2* x, const float* e, i64 count) {
+  pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   float2 v = x[t];
   FF r = ff_add({v.x, v.y}, {e[t], 0.0f});
   x[t] = make_float2(r.hi, r.lo);
 }
-__global__ void k_ff_sub_mean(float2* __restrict__ x, const double* __restrict__ mean, i64 count) {
+__global__ void k_ff_sub_mean(float2* x, const double* mean, i64 count) {
+  pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   float2 v = x[t];
@@ -1167,8 +1172,9 @@ __global__ void __launch_bounds__(256) k_residual_ff(const float2* __restrict__ 
 // The outer residual of a zero guess, b itself, as the inner solve's FP32
 // right-hand side: what k_residual_ff gives for phi = 0 (b split into a
 // float-float pair and rounded, hi + lo), with max |r| into maxbits.
-__global__ void k_ff_rhs32(const double* __restrict__ b, i64 count, float* __restrict__ r32,
+__global__ void k_ff_rhs32(const double* b, i64 count, float* r32,
                            unsigned long long* maxbits) {
+  pdl_begin();
   const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   float m = 0.0f;
   if (t < count) {
@@ -1180,23 +1186,23 @@ __global__ void k_ff_rhs32(const double* __restrict__ b, i64 count, float* __res
   block_max_commit(m, maxbits);
 }
 void launch_ff_rhs32(const double* b, i64 count, float* r32, unsigned long long* maxbits, cudaStream_t s) {
-  k_ff_rhs32<<<grid_of(count, kBlock), kBlock, 0, s>>>(b, count, r32, maxbits);
+  launch(k_ff_rhs32, grid_of(count, kBlock), kBlock, 0, s, b, count, r32, maxbits);
   count_launch();
 }
 void launch_ff_split(double* a, i64 count, cudaStream_t s) {
-  k_ff_split<<<grid_of(count, kBlock), kBlock, 0, s>>>(a, count);
+  launch(k_ff_split, grid_of(count, kBlock), kBlock, 0, s, a, count);
   count_launch();
 }
 void launch_ff_join(double* a, i64 count, cudaStream_t s) {
-  k_ff_join<<<grid_of(count, kBlock), kBlock, 0, s>>>(a, count);
+  launch(k_ff_join, grid_of(count, kBlock), kBlock, 0, s, a, count);
   count_launch();
 }
 void launch_ff_add_f(double* x, const float* e, i64 count, cudaStream_t s) {
-  k_ff_add_f<<<grid_of(count, kBlock), kBlock, 0, s>>>(reinterpret_cast<float2*>(x), e, count);
+  launch(k_ff_add_f, grid_of(count, kBlock), kBlock, 0, s, reinterpret_cast<float2*>(x), e, count);
   count_launch();
 }
 void launch_ff_sub_mean(double* x, const double* mean, i64 count, cudaStream_t s) {
-  k_ff_sub_mean<<<grid_of(count, kBlock), kBlock, 0, s>>>(reinterpret_cast<float2*>(x), mean, count);
+  launch(k_ff_sub_mean, grid_of(count, kBlock), kBlock, 0, s, reinterpret_cast<float2*>(x), mean, count);
   count_launch();
 }
 void launch_residual_ff(const double* phi, const double* rhs, const double* coef, int n, double dx, float* r32,
@@ -1217,7 +1223,8 @@ void launch_residual_ff(const double* phi, const double* rhs, const double* coef
 // power of two is exact and commutes with rounding, so the result has the
 // bits of three passes of (in[-1] + in[+1]) / 4 + in / 2.
 template <bool LAST>
-__global__ void k_smooth_axis(const double* __restrict__ in, int n, int axis, double* __restrict__ out) {
+__global__ void k_smooth_axis(const double* in, int n, int axis, double* out) {
+  pdl_begin();
   const i64 n3 = (i64)n * n * n;
   const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n3) return;
@@ -1234,14 +1241,14 @@ __global__ void k_smooth_axis(const double* __restrict__ in, int n, int axis, do
 // overwritten.
 void launch_smooth_sep(double* in, int n, double* out, cudaStream_t s) {
   const i64 n3 = (i64)n * n * n;
-  k_smooth_axis<false><<<grid_of(n3, kBlock), kBlock, 0, s>>>(in, n, 0, out);
-  k_smooth_axis<false><<<grid_of(n3, kBlock), kBlock, 0, s>>>(out, n, 1, in);
-  k_smooth_axis<true><<<grid_of(n3, kBlock), kBlock, 0, s>>>(in, n, 2, out);
+  launch(k_smooth_axis<false>, grid_of(n3, kBlock), kBlock, 0, s, in, n, 0, out);
+  launch(k_smooth_axis<false>, grid_of(n3, kBlock), kBlock, 0, s, out, n, 1, in);
+  launch(k_smooth_axis<true>, grid_of(n3, kBlock), kBlock, 0, s, in, n, 2, out);
   count_launch(3);
 }
 
 void launch_lim_reset(LimDev* st, cudaStream_t s) {
-  k_lim_reset<<<1, 1, 0, s>>>(st);
+  launch(k_lim_reset, 1, 1, 0, s, st);
   count_launch();
 }
 
@@ -1277,6 +1284,10 @@ void launch_spec_tables(double* tab, int n, cudaStream_t s) {
   count_launch();
 }
 
+// FFT Poisson correction, stage 1: from the e^{-i} half spectrum Xc = D2Z(x),
+// build the packed complex input Z' of the reference's inverse real FFT applied
+// to X_NR / symbol, X_NR = conj(Xc) the e^{+i} spectrum and the symbol that of
+// the 7-point Laplacian (limiter.f90:561-576).
 __global__ void k_spec_pack(const double2* __restrict__ Xc, int n, double2* __restrict__ Z, const LimDev* st,
                             const double* __restrict__ tab) {
   if (st->ncompress == 0) return;
@@ -1309,6 +1320,8 @@ void launch_spec_pack(const void* Xc, int n, void* Z, const LimDev* st, const do
   count_launch();
 }
 
+// Stage 2: out += 2/n^3 * (real samples held pairwise by z).  Both are skipped
+// when no cell was limited.
 __global__ void k_spec_unpack(const double2* __restrict__ z, int n, double* __restrict__ out, const LimDev* st) {
   if (st->ncompress == 0) return;
   i64 tot = (i64)(n / 2) * n * n;

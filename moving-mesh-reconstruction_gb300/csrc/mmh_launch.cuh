@@ -239,7 +239,7 @@ template <class T>
 void launch_restrict27(const T* fine, int n, T* coarse, cudaStream_t s) {
   i64 h3 = (i64)(n / 2) * (n / 2) * (n / 2);
   prof_begin(kk<T>(KK_RESTRICT), s, h3, n);
-  k_restrict27<T><<<grid_of(h3, kBlock), kBlock, 0, s>>>(fine, n, coarse);
+  launch(k_restrict27<T>, grid_of(h3, kBlock), kBlock, 0, s, fine, n, coarse);
   prof_end(kk<T>(KK_RESTRICT), s, n);
   count_launch();
 }
@@ -267,7 +267,7 @@ void launch_fxsum(const T* a, i64 count, unsigned long long* acc, int* flag, cud
   i64 blocks = (count + kBlock - 1) / kBlock;
   if (blocks > 152 * 16) blocks = 152 * 16;
   if (blocks < 1) blocks = 1;
-  k_fxsum<T><<<(unsigned)blocks, kBlock, 0, s>>>(a, count, acc, flag);
+  launch(k_fxsum<T>, (unsigned)blocks, kBlock, 0, s, a, count, acc, flag);
   count_launch();
 }
 
@@ -275,7 +275,7 @@ template <class T>
 void launch_det(const T* def, int n, T dx, T* det, cudaStream_t s) {
   i64 n3 = (i64)n * n * n;
   T di2 = T(1) / (dx * dx);
-  k_det<T><<<grid_of(n3, kBlock), kBlock, 0, s>>>(def, n, di2, det);
+  launch(k_det<T>, grid_of(n3, kBlock), kBlock, 0, s, def, n, di2, det);
   count_launch();
 }
 
@@ -287,18 +287,19 @@ void launch_sub_mean(T* a, i64 count, const double* mean, cudaStream_t s) {
 
 template <class T>
 void launch_sub_dfact(T* a, const T* det, i64 count, const double* ratio, cudaStream_t s) {
-  k_sub_dfact<T><<<grid_of(count, kBlock), kBlock, 0, s>>>(a, det, count, ratio);
+  launch(k_sub_dfact<T>, grid_of(count, kBlock), kBlock, 0, s, a, det, count, ratio);
   count_launch();
 }
 
 template <class T>
 void launch_fill(T* a, i64 count, T v, cudaStream_t s) {
-  k_fill<T><<<grid_of(count, kBlock), kBlock, 0, s>>>(a, count, v);
+  launch(k_fill<T>, grid_of(count, kBlock), kBlock, 0, s, a, count, v);
   count_launch();
 }
 
 template <class T>
-__global__ void k_absmax(const T* __restrict__ a, i64 count, unsigned long long* maxbits) {
+__global__ void k_absmax(const T* a, i64 count, unsigned long long* maxbits) {
+  pdl_begin();
   decltype(abs_bits(T(0))) m = 0;
   for (i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (i64)gridDim.x * blockDim.x) {
     auto v = abs_bits(a[t]);
@@ -312,7 +313,7 @@ void launch_absmax(const T* a, i64 count, unsigned long long* maxbits, cudaStrea
   i64 blocks = (count + kBlock - 1) / kBlock;
   if (blocks > 152 * 16) blocks = 152 * 16;
   if (blocks < 1) blocks = 1;
-  k_absmax<T><<<(unsigned)blocks, kBlock, 0, s>>>(a, count, maxbits);
+  launch(k_absmax<T>, (unsigned)blocks, kBlock, 0, s, a, count, maxbits);
   count_launch();
 }
 
@@ -324,19 +325,20 @@ void launch_zero_if(T* a, i64 count, const int* flag, cudaStream_t s) {
 
 template <class T>
 void launch_sub_mean_unless(T* a, i64 count, const double* mean, const int* flag, cudaStream_t s) {
-  k_sub_mean_unless<T><<<grid_of(count, kBlock), kBlock, 0, s>>>(a, count, mean, flag);
+  launch(k_sub_mean_unless<T>, grid_of(count, kBlock), kBlock, 0, s, a, count, mean, flag);
   count_launch();
 }
 
 template <class T>
 __global__ void k_usum_flag(const unsigned long long* acc, int* flag) {
+  pdl_begin();
   T s = (T)fx_to(acc[0], acc[1]);
   *flag = (s > T(1.e-2)) ? 0 : 1;  // 0: run zerosum, 1: skip (flag semantics of k_sub_mean_unless)
 }
 
 template <class T>
 void launch_usum_flag(const unsigned long long* acc, int* flag, cudaStream_t s) {
-  k_usum_flag<T><<<1, 1, 0, s>>>(acc, flag);
+  launch(k_usum_flag<T>, 1, 1, 0, s, acc, flag);
   count_launch();
 }
 

@@ -100,40 +100,4 @@ struct LimDev {
   int pad;
 };
 
-// Pass-1 flux limiter for a density-only state (u(2:5) = 0, so the
-// momentum-flux divergence is zero): limiter.f90:238-381.  The flux of cell
-// (i,j,km) is tested with the metric of plane k = km+1.
-__global__ void k_limiter_pass1(double* __restrict__ tmp, const double* __restrict__ def,
-                                const double* __restrict__ rho, int n, double dtold, double dtaumesh,
-                                double cmpmaxglobal, LimDev* st, uint8_t* __restrict__ maskx,
-                                uint8_t* __restrict__ maskc);
-
-// Compression test on I + dtold*Hess(defp) + Hess(def) (limiter.f90:425-533).
-__global__ void k_limiter_mask(double* __restrict__ defplim, const double* __restrict__ def,
-                               const double* __restrict__ defp, int n, double dtold, double cmpmaxglobal, LimDev* st,
-                               uint8_t* __restrict__ mask);
-
-// calcdefp RHS: tmp = clip(1 - rho, +-2)/30/dtold (limiter.f90:134-169)
-__global__ void k_calcdefp_rhs(double* __restrict__ tmp, const double* __restrict__ rho, i64 n3, double dtold);
-
-// FFT Poisson correction, stage 1: from the e^{-i} half spectrum Xc = D2Z(x),
-// build the packed complex input Z' of the reference's inverse real FFT applied
-// to X_NR / symbol, X_NR = conj(Xc) the e^{+i} spectrum and the symbol that of
-// the 7-point Laplacian (limiter.f90:561-576).
-__global__ void k_spec_pack(const double2* __restrict__ Xc, int n, double2* __restrict__ Z, const LimDev* st,
-                            const double* __restrict__ tab);
-// Stage 2: out += 2/n^3 * (real samples held pairwise by z).  Both are skipped
-// when no cell was limited.
-__global__ void k_spec_unpack(const double2* __restrict__ z, int n, double* __restrict__ out, const LimDev* st);
-
-// relaxing-TVD (relaxing.f90) for the density component.
-__global__ void k_relax_stage1(const double* __restrict__ rho, const double* __restrict__ def,
-                               const double* __restrict__ defp, int n, double* __restrict__ baj,
-                               double* __restrict__ cc, double* __restrict__ vt);
-__global__ void k_relax_flux(const double* __restrict__ u1, const double* __restrict__ defp,
-                             const double* __restrict__ baj, int n, double* __restrict__ vt);
-__global__ void k_relax_dpv(const double* __restrict__ u, const double* __restrict__ vt,
-                            const double* __restrict__ cc, int n, const double* __restrict__ ubase, double dt,
-                            double* __restrict__ out);
-
 }  // namespace mmh
