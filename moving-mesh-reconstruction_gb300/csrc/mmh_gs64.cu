@@ -233,7 +233,7 @@ int rows_ty(int n) { return n == 32 ? 8 : (n == 64 || n > 512 ? 16 : 32); }
 // products of phase p + 1 that do not depend on p and sum its cross terms
 // (warp S): a phase costs 13, 13, 20, 13 dependent FP64 instructions instead
 // of some 75 (64 cycles each).
-// Against one CTA with a thread per cell: 32 sweeps at 4^3 197 us (747), at
+// Against one CTA with a thread per cell: 32 sweeps at 4^3 185 us (747), at
 // 8^3 323 us (771); 16 sweeps at 16^3 185 us (1508).
 // ---------------------------------------------------------------------------
 template <int N>
@@ -489,12 +489,16 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
         const double v = -div_by(__fma_rn(-0.5, s2, X2[p] - s1), D[p], Y[p]);
         const int i = (p >> 1) & 1, j = p & 1, kz = p >> 2;
         if (CC == 8) {
+          // the box itself (and, alone, its own neighbour) by a plain store: a
+          // cluster store to the own CTA takes the way between SMs too
 #pragma unroll
           for (int s = 0; s < 2; ++s)
-            if (ok_[s] >> p & 1u)
-              st_cluster(base_[s][0] + 8u * (c + (i ? -shift_[s][0] : shift_[s][0]) +
-                                             (j ? -shift_[s][1] : shift_[s][1]) + (kz ? -shift_[s][2] : shift_[s][2])),
-                         v);
+            if (ok_[s] >> p & 1u) {
+              const int e = c + (i ? -shift_[s][0] : shift_[s][0]) + (j ? -shift_[s][1] : shift_[s][1]) +
+                            (kz ? -shift_[s][2] : shift_[s][2]);
+              if (G::CL == 1 || (s == 0 && lane < 8)) sp[e] = v;
+              else st_cluster(base_[s][0] + 8u * e, v);
+            }
         } else {
           constexpr int sets[6] = {1, 2, 3, 4, 5, 6};
           sp[c] = v;
