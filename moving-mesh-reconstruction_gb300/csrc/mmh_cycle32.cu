@@ -16,8 +16,9 @@
 // single cells of the density by 1e-7.
 //
 // What bounds it now is shared-memory latency per colour phase and, on the
-// 4^3 level, the FP64 pipe (64 dependent additions of 64 cycles).  Measured: a
-// 32^3 inner solve 43 us per iteration (250 us as launches).
+// 4^3 level, the FP64 pipe (2048 cycles for the 4096 products; summed one by one
+// per row they were a chain of 4096).  Measured: a 32^3 inner solve of
+// five iterations 194 us (250 us an iteration as launches).
 #include <cooperative_groups.h>
 
 #include "mmh_kernels.cuh"
@@ -59,7 +60,7 @@ struct CycleArgs {
 struct Shared {
   double M[64 * 64];      // inverse of the 4^3 operator, transposed (first CTA)
   double b4[64], wsum[2];
-  double prod[2][8][64];  // products of 8 columns of M with b4
+  double part[4][64];     // quarters of the rows' sums
   double slot[3][128];     // block sums of the dot products p.q, z.q, r.z
   double smax[kCta];
   float warp[64];
@@ -254,8 +255,7 @@ __device__ void cube_cycle(float* w, Shared* sh, float dx2, int nu1, int nu2, in
   }
   __syncthreads();
   // z = M (r - mean r) on the 4^3 cells, FP64, with the operations of
-  // k_coarse_apply: a row's 64 products are summed one by one.  The first two
-  // warps hold the rows' sums; all form the products, 8 columns ahead.
+  // k_coarse_apply: four threads share a row, 16 fused multiply-adds each.
   if (tid < 64) {
     const int X = tid & 3, Y = (tid >> 2) & 3, K = tid >> 4;
     const float* r = w + C::R;
@@ -268,25 +268,17 @@ __device__ void cube_cycle(float* w, Shared* sh, float dx2, int nu1, int nu2, in
     sh->b4[tid] = __dsub_rn(v, __dadd_rn(sh->wsum[0], sh->wsum[1]) / 64);
   }
   __syncthreads();
-  auto products = [&](int chunk, int first, int count) {
-    for (int e = tid - first; e < 512; e += count) {
-      const int j = chunk * 8 + (e >> 6), row = e & 63;
-      sh->prod[chunk & 1][e >> 6][row] = __dmul_rn(sh->M[j * 64 + row], sh->b4[j]);
-    }
-  };
-  products(0, 0, kThreads);
-  __syncthreads();
-  double acc = 0.0;
-  for (int chunk = 0; chunk < 8; ++chunk) {
-    if (tid < 64) {
+  {
+    const int row = tid & 63, q = tid >> 6;
+    double acc = 0.0;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc = __dadd_rn(acc, sh->prod[chunk & 1][j][tid]);
-    } else if (chunk < 7) {
-      products(chunk + 1, 64, kThreads - 64);
-    }
-    __syncthreads();
+    for (int j = 16 * q; j < 16 * q + 16; ++j) acc = __fma_rn(sh->M[j * 64 + row], sh->b4[j], acc);
+    sh->part[q][row] = acc;
   }
-  if (tid < 64) sh->z4[(tid >> 4) * 16 + at<4>(tid & 3, (tid >> 2) & 3)] = (float)acc;
+  __syncthreads();
+  if (tid < 64)
+    sh->z4[(tid >> 4) * 16 + at<4>(tid & 3, (tid >> 2) & 3)] =
+        (float)__dadd_rn(__dadd_rn(sh->part[0][tid], sh->part[1][tid]), __dadd_rn(sh->part[2][tid], sh->part[3][tid]));
   __syncthreads();
   for (int e = tid; e < 512; e += kThreads) {
     const int k = e >> 6, x = e & 7, y = (e >> 3) & 7;

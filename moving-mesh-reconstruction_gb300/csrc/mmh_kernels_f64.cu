@@ -229,24 +229,27 @@ __global__ void __launch_bounds__(256) k_coarse_inverse(const double* coef, doub
   M[i * N + j] = a;
 }
 
-// z = M (r - mean r) on the 64 cells: one CTA of 64 threads, FP64 sums.
-__global__ void __launch_bounds__(64) k_coarse_apply(const float* __restrict__ r, const double* __restrict__ M,
-                                                     float* __restrict__ z) {
+// z = M (r - mean r) on the 64 cells in FP64, M symmetric: one CTA, four threads
+// per row (the operations of mmh_cycle32.cu).
+__global__ void __launch_bounds__(256) k_coarse_apply(const float* __restrict__ r, const double* __restrict__ M,
+                                                      float* __restrict__ z) {
   constexpr int N = kCoarseN;
-  __shared__ double b[N];
+  __shared__ double b[N], part[4][N];
   __shared__ double wsum[2];
-  const int tid = threadIdx.x;
-  double v = (double)r[tid];
+  const int tid = threadIdx.x, row = tid & 63, q = tid >> 6;
+  const double v = (double)r[row];
   double sv = v;
   for (int d = 16; d > 0; d >>= 1) sv += __shfl_down_sync(0xffffffffu, sv, d);
-  if ((tid & 31) == 0) wsum[tid >> 5] = sv;
+  if (tid < N && (tid & 31) == 0) wsum[tid >> 5] = sv;
   __syncthreads();
-  b[tid] = v - (wsum[0] + wsum[1]) / N;
+  if (tid < N) b[tid] = v - (wsum[0] + wsum[1]) / N;
   __syncthreads();
   double acc = 0.0;
-#pragma unroll 8
-  for (int j = 0; j < N; ++j) acc += M[tid * N + j] * b[j];
-  z[tid] = (float)acc;
+#pragma unroll
+  for (int j = 16 * q; j < 16 * q + 16; ++j) acc = __fma_rn(M[row * N + j], b[j], acc);
+  part[q][row] = acc;
+  __syncthreads();
+  if (tid < N) z[tid] = (float)((part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]));
 }
 
 void launch_coarse_inverse(const double* coef, double dx, double* M, cudaStream_t s) {
@@ -256,7 +259,7 @@ void launch_coarse_inverse(const double* coef, double dx, double* M, cudaStream_
   count_launch();
 }
 void launch_coarse_apply(const float* r, const double* M, float* z, cudaStream_t s) {
-  k_coarse_apply<<<1, kCoarseN, 0, s>>>(r, M, z);
+  k_coarse_apply<<<1, 4 * kCoarseN, 0, s>>>(r, M, z);
   count_launch();
 }
 
