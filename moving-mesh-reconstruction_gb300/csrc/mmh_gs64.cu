@@ -139,7 +139,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_gs_rows(const double* __rest
       double s1, s2, d;
       sums64<PRE>(
           f, o, [&](int dx, int dy) { return s0[dy * n + (dx > 0 ? op : dx < 0 ? om : oc)]; }, Kp, Km, s1, s2, d);
-      const double num = __fma_rn(-0.5, s2, rk[o.c] * dx2x2 - s1);
+      // Face64 comes with the levels' own spacings, powers of two: rhs 2dx2 is exact
+      const double lead = PRE ? __fma_rn(rk[o.c], dx2x2, -s1) : rk[o.c] * dx2x2 - s1;
+      const double num = __fma_rn(-0.5, s2, lead);
       sp[((yl + 3) << lgn) + oc] = -(PRE ? div_by(num, d, yk[o.c]) : num / d);
     }
     __syncthreads();

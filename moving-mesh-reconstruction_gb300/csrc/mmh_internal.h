@@ -82,6 +82,12 @@ template <class T> void launch_absmax(const T* a, i64 count, unsigned long long*
 // divergence guard: flag = relaxerr > r1*margin && r1 > floor (bits are maxbits words)
 void launch_guard(const unsigned long long* r1bits, const unsigned long long* errbits, double margin, double floor_,
                   int* flag, int* guards, cudaStream_t s);
+// launch_fxsum, launch_fx_mean and launch_sub_mean of a field of at most 4096
+// cells in one launch; the second with launch_guard, zeroing the field if it holds
+void launch_zerosum_small(double* a, i64 count, int* bad, cudaStream_t s);
+void launch_zerosum_small(double* a, i64 count, int* bad, const unsigned long long* r1bits,
+                          const unsigned long long* errbits, double margin, double floor_, int* flag, int* guards,
+                          cudaStream_t s);
 template <class T> void launch_zero_if(T* a, i64 count, const int* flag, cudaStream_t s);
 template <class T> void launch_sub_mean_unless(T* a, i64 count, const double* mean, const int* flag, cudaStream_t s);
 // zerosum helpers: mean = fx(acc)/count ; usum flag = (T)fx(acc) > 1e-2

@@ -134,6 +134,63 @@ void launch_guard(const unsigned long long* r1bits, const unsigned long long* er
   count_launch();
 }
 
+// zerosum of a field of at most 4096 cells, and with GUARD the divergence guard
+// (k_guard; the field is zeroed where it holds) in one block: the exact sum has
+// no order, so the bits are those of k_fxsum, k_fx_mean and k_sub_mean.  On the
+// levels of 16^3 and below these are launches, not work: 4 (6 with the guard) a
+// level and cycle.
+template <bool GUARD>
+__global__ void __launch_bounds__(512) k_zerosum_small(double* __restrict__ a, int count, int* bad,
+                                                       const unsigned long long* r1bits,
+                                                       const unsigned long long* errbits, double margin, double floor_,
+                                                       int* flag, int* guards) {
+  __shared__ unsigned long long s_acc[2];
+  __shared__ double s_mean;
+  __shared__ int s_zero;
+  if (threadIdx.x < 2) s_acc[threadIdx.x] = 0;
+  __syncthreads();
+  double v[8];
+  __int128 s = 0;
+  bool out = false;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int t = threadIdx.x + 512 * q;
+    v[q] = t < count ? a[t] : 0.0;
+    if (!(fabs(v[q]) < 4294967296.0)) out = true;
+    else s += fx_of(v[q]);
+  }
+  if (out) atomicOr(bad, 1);
+  fx_block_commit(s, s_acc);
+  if (threadIdx.x == 0) {
+    s_mean = fx_to(s_acc[0], s_acc[1]) / (double)count;
+    s_zero = 0;
+    if (GUARD) {
+      const double r1 = from_bits(*r1bits), err = from_bits(*errbits);
+      const int g = (err > r1 * margin && r1 > floor_) ? 1 : 0;
+      *flag = s_zero = g;
+      if (g) *guards += 1;
+    }
+  }
+  __syncthreads();
+  const double mean = s_mean;
+  const bool zero = GUARD && s_zero;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int t = threadIdx.x + 512 * q;
+    if (t < count) a[t] = zero ? 0.0 : v[q] - mean;
+  }
+}
+void launch_zerosum_small(double* a, i64 count, int* bad, cudaStream_t s) {
+  k_zerosum_small<false><<<1, 512, 0, s>>>(a, (int)count, bad, nullptr, nullptr, 0.0, 0.0, nullptr, nullptr);
+  count_launch();
+}
+void launch_zerosum_small(double* a, i64 count, int* bad, const unsigned long long* r1bits,
+                          const unsigned long long* errbits, double margin, double floor_, int* flag, int* guards,
+                          cudaStream_t s) {
+  k_zerosum_small<true><<<1, 512, 0, s>>>(a, (int)count, bad, r1bits, errbits, margin, floor_, flag, guards);
+  count_launch();
+}
+
 __global__ void k_d2f(const double* a, float* b, i64 count) {
   pdl_begin();
   i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;

@@ -177,6 +177,12 @@ namespace {
 // ---------------------------------------------------------------------------
 template <class T>
 int zerosum(mmh_ctx* c, T* a, i64 count) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (count <= 4096) {
+      launch_zerosum_small(a, count, &c->sc->bad, c->s);
+      return MMH_OK;
+    }
+  }
   CK(cudaMemsetAsync(c->sc->acc[0], 0, 16, c->s));
   launch_fxsum<T>(a, count, c->sc->acc[0], &c->sc->bad, c->s);
   launch_fx_mean(c->sc->acc[0], (double)count, &c->sc->mean, c->s);
@@ -255,6 +261,13 @@ int guard_or_zerosum(mmh_ctx* c, int l, T* u, double margin, double floor_, bool
   // products with them, and the outer loop removes the solution's mean.
   if (!guard && std::is_same<T, float>::value && c->cfg.schedule == MMH_SCHED_TOL) return MMH_OK;
   if (!guard) return zerosum<T>(c, u, n3);
+  if constexpr (std::is_same<T, double>::value) {
+    if (n3 <= 4096) {
+      launch_zerosum_small(u, n3, &c->sc->bad, &c->sc->r1bits[l], &c->sc->errbits[l], margin, floor_, &c->sc->gflag[l],
+                           &c->sc->guards, c->s);
+      return MMH_OK;
+    }
+  }
   launch_guard(&c->sc->r1bits[l], &c->sc->errbits[l], margin, floor_, &c->sc->gflag[l], &c->sc->guards, c->s);
   CK(cudaMemsetAsync(c->sc->acc[3], 0, 16, c->s));
   launch_fxsum<T>(u, n3, c->sc->acc[3], &c->sc->bad, c->s);

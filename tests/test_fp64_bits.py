@@ -62,3 +62,26 @@ def test_pass1(mmh, oracle, fields, kind, dtold, dtaumesh):
         mxg, mcg, dg = ctx.limiter_pass1(tg, d, np.asfortranarray(u[0]), dtold, dtaumesh)
     assert same(tg, to) and np.array_equal(mxo, mxg) and np.array_equal(mco, mcg)
     assert do["nexpand"] == dg["nexpand"] and do["detmin"] == dg["detmin"]
+
+
+@pytest.mark.parametrize("kind", ("smooth", "zero", "tiny", "subnormal", "rough", "huge"))
+@pytest.mark.parametrize("n", [8, 32])
+def test_smooth(mmh, oracle, n, kind):
+    a = potential(n, kind, 11)
+    if kind == "huge":
+        a = np.asfortranarray(a * 1e217)  # sums beyond the scaled form's range
+    g = a.copy(order="F")
+    with mmh.Context(n) as ctx:
+        ctx.nsmooth(g)
+        assert same(ctx.restrict(a), oracle.restrict(a))
+    assert same(g, oracle.nsmooth(a))
+
+
+@pytest.mark.parametrize("n", [4, 8, 16])
+def test_zerosum_small(mmh, oracle, n):
+    a = np.asfortranarray(np.random.default_rng(n).standard_normal((n, n, n)))
+    g = a.copy(order="F")
+    with mmh.Context(max(n, 8)) as ctx:
+        ctx.zerosum(g)
+    oracle.zerosum(a)
+    assert same(g, a)
