@@ -313,14 +313,14 @@ __device__ __forceinline__ double mm_branch(double a, double b, double& da, doub
     db = ub;
     return v;
   }
-  const bool pa = __double_as_longlong(a) >= 0 || ax == 0, pb = __double_as_longlong(b) >= 0 || ay == 0;
+  const bool pa = __double2hiint(a) >= 0 || ax == 0, pb = __double2hiint(b) >= 0 || ay == 0;
   const double l15 = 1.5 * from_bits(lob);
   const bool low = abs_bits(l15) <= hib;
   const double w = pa != pb ? 0.0 : low ? 1.5 : 1.0, v = pa != pb ? 0.0 : low ? l15 : from_bits(hib);
   const bool first = low ? ax <= ay : ax >= ay;
   da = first ? w : 0.0;
   db = first ? 0.0 : w;
-  return pa ? v : -v;
+  return pa ? v : neg_of(v);
 }
 
 // the cells t + o along an axis, periodic (|o| < n)

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_gs_rows(const double* __rest
       // Face64 comes with the levels' own spacings, powers of two: rhs 2dx2 is exact
       const double lead = PRE ? __fma_rn(rk[o.c], dx2x2, -s1) : rk[o.c] * dx2x2 - s1;
       const double num = __fma_rn(-0.5, s2, lead);
-      sp[((yl + 3) << lgn) + oc] = -(PRE ? div_by(num, d, yk[o.c]) : num / d);
+      sp[((yl + 3) << lgn) + oc] = neg_of(PRE ? div_by(num, d, yk[o.c]) : num / d);
     }
     __syncthreads();
   }
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
           s1 = s1 + f[5][cell];
           s2 = sum2[p & 1][cell];
         }
-        const double v = -div_by(__fma_rn(-0.5, s2, X2[p] - s1), D[p], Y[p]);
+        const double v = neg_of(div_by(__fma_rn(-0.5, s2, X2[p] - s1), D[p], Y[p]));
         const int i = (p >> 1) & 1, j = p & 1, kz = p >> 2;
         if (CC == 8) {
           // the box itself (and, alone, its own neighbour) by a plain store: a

@@ -186,11 +186,19 @@ __device__ __forceinline__ void block_max_commit(float v, unsigned long long* ou
   block_max_commit_bits(w, out);
 }
 __device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+// The bits of doubles go by their halves: of masks, flips and tests on the whole
+// word the compiler makes fabs, negations and comparisons again, which are
+// FP64-pipe operations.
 __device__ __forceinline__ unsigned long long abs_bits(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  return (unsigned long long)((unsigned)__double2hiint(x) & 0x7FFFFFFFu) << 32 | (unsigned)__double2loint(x);
 }
 __device__ __forceinline__ float from_bits(unsigned b) { return __uint_as_float(b); }
-__device__ __forceinline__ double from_bits(unsigned long long b) { return __longlong_as_double((long long)b); }
+__device__ __forceinline__ double from_bits(unsigned long long b) {
+  return __hiloint2double((int)(b >> 32), (int)(unsigned)b);
+}
+__device__ __forceinline__ double neg_of(double x) {
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000u, __double2loint(x));
+}
 
 // ---------------------------------------------------------------------------
 // Launches of the kernels that an iteration runs by the hundred.  They begin
@@ -246,14 +254,14 @@ void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream
 // inlined, the compiler would execute it always and select.
 // ---------------------------------------------------------------------------
 // biased binary exponent: 0 for zero and subnormals, 2047 for inf and NaN
-__device__ __forceinline__ int bexp(double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7ff); }
+__device__ __forceinline__ int bexp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 static __device__ __noinline__ double slow_mul(double a, double b) { return a * b; }
 static __device__ __noinline__ double slow_div(double a, double b) { return a / b; }
 // x 2^-K with the same bits as the product
 template <int K>
 __device__ __forceinline__ double pow2_down(double x) {
   const int e = bexp(x);
-  if (e > K && e < 2047) return __longlong_as_double(__double_as_longlong(x) - ((i64)K << 52));
+  if (e > K && e < 2047) return __hiloint2double(__double2hiint(x) - (K << 20), __double2loint(x));
   if (abs_bits(x) == 0) return x;
   return slow_mul(x, 1.0 / (1 << K));
 }
@@ -276,7 +284,7 @@ __device__ __forceinline__ double div_by(double num, double d, double y) {
       return __fma_rn(__fma_rn(-d, q, num), y, q);
     }
     if (abs_bits(num) == 0)
-      return __longlong_as_double((__double_as_longlong(num) ^ __double_as_longlong(d)) & (i64)0x8000000000000000ull);
+      return __hiloint2double((__double2hiint(num) ^ __double2hiint(d)) & (int)0x80000000u, 0);
   }
   return slow_div(num, d);
 }

@@ -1419,7 +1419,7 @@ static __device__ __noinline__ double slow_sub(double a, double b) { return a - 
 // z - x for a zero z (or a NaN one): -x by its sign bit, but for zeros and NaN
 __device__ __forceinline__ double zero_minus(double z, double x) {
   const unsigned long long b = abs_bits(x);
-  if (abs_bits(z) == 0 && b != 0 && b <= 0x7FF0000000000000ull) return -x;
+  if (abs_bits(z) == 0 && b != 0 && b <= 0x7FF0000000000000ull) return neg_of(x);
   return slow_sub(z, x);
 }
 // MIN/MAX as the restatement evaluates them (std::min / std::max: a
@@ -1644,8 +1644,8 @@ __device__ __forceinline__ double minmod(double a, double b) {
     const double hi = from_bits(hib), l15 = 1.5 * from_bits(lob);  // finite or +inf
     const double mm = abs_bits(l15) <= hib ? l15 : hi;
     if (bexp(mm) < 2046) {
-      const bool pa = (__double_as_longlong(a) >= 0) || ax == 0, pb = (__double_as_longlong(b) >= 0) || ay == 0;
-      return pa != pb ? 0.0 : (pa ? mm : -mm);
+      const bool pa = __double2hiint(a) >= 0 || ax == 0, pb = __double2hiint(b) >= 0 || ay == 0;
+      return pa != pb ? 0.0 : (pa ? mm : neg_of(mm));
     }
   }
   return minmod_written(a, b);
