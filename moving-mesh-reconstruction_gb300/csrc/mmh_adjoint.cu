@@ -144,13 +144,14 @@ __global__ void k_adj_metric(const double* __restrict__ def, const double* __res
     double uxp = u[xp], uxm = u[xm], uyp = u[yp], uym = u[ym], uzp = u[zp], uzm = u[zm];
     double w = -urg[t];
     // adjoint of C_f: -urg G_f, then of cof_f / det
-    double g11 = w * 0.5 * ((lc - lxp) * (uxp - uc) + (lc - lxm) * (uxm - uc)) / det;
-    double g22 = w * 0.5 * ((lc - lyp) * (uyp - uc) + (lc - lym) * (uym - uc)) / det;
-    double g33 = w * 0.5 * ((lc - lzp) * (uzp - uc) + (lc - lzm) * (uzm - uc)) / det;
-    double g12 = w * 0.25 * ((lym - lyp) * (uxp - uxm) + (lxm - lxp) * (uyp - uym)) / det;
-    double g13 = w * 0.25 * ((lzm - lzp) * (uxp - uxm) + (lxm - lxp) * (uzp - uzm)) / det;
-    double g23 = w * 0.25 * ((lzm - lzp) * (uyp - uym) + (lym - lyp) * (uzp - uzm)) / det;
-    detb -= (g11 * b11 + g12 * b12 + g13 * b13 + g22 * b22 + g23 * b23 + g33 * b33) / det;
+    const double rdet = 1.0 / det;
+    double g11 = div_by(w * 0.5 * ((lc - lxp) * (uxp - uc) + (lc - lxm) * (uxm - uc)), det, rdet);
+    double g22 = div_by(w * 0.5 * ((lc - lyp) * (uyp - uc) + (lc - lym) * (uym - uc)), det, rdet);
+    double g33 = div_by(w * 0.5 * ((lc - lzp) * (uzp - uc) + (lc - lzm) * (uzm - uc)), det, rdet);
+    double g12 = div_by(w * 0.25 * ((lym - lyp) * (uxp - uxm) + (lxm - lxp) * (uyp - uym)), det, rdet);
+    double g13 = div_by(w * 0.25 * ((lzm - lzp) * (uxp - uxm) + (lxm - lxp) * (uzp - uzm)), det, rdet);
+    double g23 = div_by(w * 0.25 * ((lzm - lzp) * (uyp - uym) + (lym - lyp) * (uzp - uzm)), det, rdet);
+    detb -= div_by(g11 * b11 + g12 * b12 + g13 * b13 + g22 * b22 + g23 * b23 + g33 * b33, det, rdet);
     c11 = g11; c12 = g12; c13 = g13; c22 = g22; c23 = g23; c33 = g33;
   }
   adj_cofdet(a11, a12, a13, a22, a23, a33, b11, b12, b13, b22, b23, b33, detb, c11, c12, c13, c22, c23, c33, abar,
@@ -379,9 +380,10 @@ __global__ void k_adj_alpha(const double* __restrict__ baj, const double* __rest
   double b11 = baj[t], b12 = baj[n3 + t], b13 = baj[2 * n3 + t], b22 = baj[3 * n3 + t], b23 = baj[4 * n3 + t],
          b33 = baj[5 * n3 + t];
   double c = cc[t];
-  alpha[t] = (b11 * v1 + b12 * v2 + b13 * v3) / c;
-  alpha[n3 + t] = (b12 * v1 + b22 * v2 + b23 * v3) / c;
-  alpha[2 * n3 + t] = (b13 * v1 + b23 * v2 + b33 * v3) / c;
+  const double yc = 1.0 / c;
+  alpha[t] = div_by(b11 * v1 + b12 * v2 + b13 * v3, c, yc);
+  alpha[n3 + t] = div_by(b12 * v1 + b22 * v2 + b23 * v3, c, yc);
+  alpha[2 * n3 + t] = div_by(b13 * v1 + b23 * v2 + b33 * v3, c, yc);
 }
 
 // Adjoint of one dpv evaluation x -> scale * R(x) against rbar: xbar = the
@@ -448,7 +450,8 @@ __global__ void k_adj_relax_geom(const double* __restrict__ def, const double* _
   double ab[3] = {alphabar[t], alphabar[n3 + t], alphabar[2 * n3 + t]};
   // alpha_a = vv_a / c, c = |vv_as|
   double cb = cbar[t] - (ab[0] * vv[0] + ab[1] * vv[1] + ab[2] * vv[2]) / (c * c);
-  double vb[3] = {ab[0] / c, ab[1] / c, ab[2] / c};
+  const double yc = 1.0 / c;
+  double vb[3] = {div_by(ab[0], c, yc), div_by(ab[1], c, yc), div_by(ab[2], c, yc)};
   vb[as] += cb * (vv[as] > 0.0 ? 1.0 : (vv[as] < 0.0 ? -1.0 : 0.0));
   // vv = b v, v = -pd; b = cof / det
   double g11 = vb[0] * v1, g22 = vb[1] * v2, g33 = vb[2] * v3;
@@ -460,8 +463,13 @@ __global__ void k_adj_relax_geom(const double* __restrict__ def, const double* _
   double det = m.det;
   double c11 = a22 * a33 - a23 * a23, c12 = a13 * a23 - a12 * a33, c13 = a12 * a23 - a13 * a22;
   double c22 = a11 * a33 - a13 * a13, c23 = a12 * a13 - a11 * a23, c33 = a11 * a22 - a12 * a12;
-  g11 /= det; g12 /= det; g13 /= det; g22 /= det; g23 /= det; g33 /= det;
-  double detb = -(g11 * c11 + g12 * c12 + g13 * c13 + g22 * c22 + g23 * c23 + g33 * c33) / det;
+  g11 = div_by(g11, det, m.y);
+  g12 = div_by(g12, det, m.y);
+  g13 = div_by(g13, det, m.y);
+  g22 = div_by(g22, det, m.y);
+  g23 = div_by(g23, det, m.y);
+  g33 = div_by(g33, det, m.y);
+  double detb = div_by(neg_of(g11 * c11 + g12 * c12 + g13 * c13 + g22 * c22 + g23 * c23 + g33 * c33), det, m.y);
   adj_cofdet(a11, a12, a13, a22, a23, a33, c11, c12, c13, c22, c23, c33, detb, g11, g12, g13, g22, g23, g33, abar,
              t, n3);
 }

@@ -13,7 +13,7 @@
 //     and every warp instruction has 32 (16 at n = 32) useful lanes;
 //   - the FP64 form's solver keeps, with each metric, the face sums, the
 //     diagonal and its reciprocal (Face64) in place of three coefficient
-//     planes: 54 FP64 instructions per update instead of 69, 51 per residual;
+//     planes: 53 FP64 instructions per update instead of 69, 52 per residual;
 //   - powers of two are folded (scaling is exact and commutes with rounding):
 //     with S1 = 2 t1, S2 = 4 t2, D = -2 tdiag formed from unhalved face sums,
 //     phi = (rhs dx2 - t1 - t2) / tdiag = -(((rhs 2dx2) - S1) - S2/2) / D;
@@ -44,8 +44,8 @@ namespace {
 // fit shared memory (1024^3) or would leave SMs without a CTA (64^3), 8 at
 // 32^3.  Per half sweep, against the form it replaces (from 64^3 up a 32 x 8
 // tile with 1.75 updates per cell counting idle lanes, at 32^3 four
-// one-colour launches): 256^3 1.26 ms (2.25), 128^3 0.187 ms (0.30), 64^3
-// 33.5 us (48), 32^3 14.4 us (38).
+// one-colour launches): 256^3 0.99 ms (2.25), 128^3 0.148 ms (0.30), 64^3
+// 29.3 us (48), 32^3 14.3 us (38).
 // ---------------------------------------------------------------------------
 constexpr int kRowThreads = 256;
 
@@ -235,7 +235,7 @@ int rows_ty(int n) { return n == 32 ? 8 : (n == 64 || n > 512 ? 16 : 32); }
 // products of phase p + 1 that do not depend on p and sum its cross terms
 // (warp S): a phase costs 13, 13, 20, 13 dependent FP64 instructions instead
 // of some 75 (64 cycles each).
-// Against one CTA with a thread per cell: 32 sweeps at 4^3 185 us (747), at
+// Against one CTA with a thread per cell: 32 sweeps at 4^3 183 us (747), at
 // 8^3 323 us (771); 16 sweeps at 16^3 185 us (1508).
 // ---------------------------------------------------------------------------
 template <int N>

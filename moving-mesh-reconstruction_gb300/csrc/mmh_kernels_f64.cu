@@ -1449,7 +1449,7 @@ __device__ __forceinline__ void store_sd(double* __restrict__ sd, i64 n3, i64 t,
 // by det, by det again and by c become one reciprocal each and products.  The
 // other form divides by the reciprocals of det and c (the same bits), and with
 // rcc leaves 1 / c and the metric times det for k_relax_flux.  Bound by the
-// FP64 pipe: 256^3 6.6 ms with a division each, now 5.8 ms.
+// FP64 pipe: 256^3 6.6 ms with a division each, now 5.0 ms.
 template <bool FastDiv>
 __global__ void k_relax_stage1(const double* __restrict__ rho, const double* __restrict__ def,
                                const double* __restrict__ defp, int n, double* __restrict__ baj,
@@ -1561,7 +1561,7 @@ void launch_relax_stage1(const double* rho, const double* def, const double* def
 
 // flux of the half-step state u1 with the metric of stage 1 (relaxing.f90:
 // 970-988), as the half sums and differences of store_sd.  With rcc: stage 1's
-// products of the metric with det and its 1 / c (256^3 2.4 ms, 2.9 ms with a
+// products of the metric with det and its 1 / c (256^3 2.0 ms, 2.9 ms with a
 // division each).
 template <bool FastDiv>
 __global__ void k_relax_flux(const double* __restrict__ u1, const double* __restrict__ defp,
@@ -1670,7 +1670,7 @@ __device__ __forceinline__ double wphalf_sd(double sm, double s0, double sp, dou
 // and the lower face of each cell; the lower face is the upper face of the
 // neighbour below, computed from the same operands in the same order, so each
 // face is evaluated once here instead of once from each side.
-// 33 FP64 instructions per cell (256^3: 2.0 ms; 2.6 ms while the slow paths
+// 33 FP64 instructions per cell (256^3: 1.06 ms; 2.6 ms while the slow paths
 // of minmod and the halvings were inlined, and so executed).
 __global__ void k_relax_faces(const double* __restrict__ sd, const double* __restrict__ cc, int n,
                               double* __restrict__ g) {
