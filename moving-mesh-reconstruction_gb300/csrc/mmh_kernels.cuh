@@ -211,9 +211,9 @@ __device__ __forceinline__ double neg_of(double x) {
 // for those with much shared memory: FP64 solves became 3 to 8% slower, a batch
 // of realisations on several streams 11%.
 //   A kernel without pdl_begin must not be launched this way, and a kernel with
-// it takes no __restrict__ parameters and uses no __ldg: its inputs may still
-// be written while its first blocks wait, which non-coherent loads do not
-// allow.
+// it, and what it inlines, takes no __restrict__ parameters and uses no __ldg:
+// its inputs may still be written while its first blocks wait, which
+// non-coherent loads do not allow.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -418,7 +418,7 @@ __device__ __forceinline__ float gs_div(float a, float b) { return __fdividef(a,
 
 // Gather the stencil of cell (i,j,k) from global memory.
 template <class T>
-__device__ __forceinline__ void op_terms(const T* __restrict__ phi, const T* __restrict__ coef, int n, i64 n3, int i,
+__device__ __forceinline__ void op_terms(const T* phi, const T* coef, int n, i64 n3, int i,
                                          int j, int k, T& tdiag, T& t1, T& t2) {
   int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
   const T* f1 = coef;
@@ -1245,7 +1245,7 @@ static __device__ __noinline__ double smooth27_written(double c, double f, doubl
 // 27-point full weighting [1/4,1/2,1/4]^3 (restrict mgutil.f90:74-118 at the
 // odd fine points, nsmooth limiter.f90:677-781 at every point).
 template <class T>
-__device__ __forceinline__ T smooth27(const T* __restrict__ a, int n, int i, int j, int k) {
+__device__ __forceinline__ T smooth27(const T* a, int n, int i, int j, int k) {
   int ip = wp(i, n), im = wm(i, n), jp = wp(j, n), jm = wm(j, n), kp = wp(k, n), km = wm(k, n);
 #define A_(x, y, z) a[IDX(x, y, z, n)]
   const T c = A_(i, j, k);
