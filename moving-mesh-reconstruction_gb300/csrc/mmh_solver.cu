@@ -281,10 +281,11 @@ int vcycle_fp64(mmh_ctx* c, int l);
 
 // Whether the FP32 levels from l down run as one launch (mmh_cycle32.cu): the
 // 32^3 and 16^3 levels of a cycle without guards and with the exact 4^3 solve.
+// While the timing hooks are armed they run launch by launch (the same bits).
 bool cycle32_at(const mmh_ctx* c, int l) {
   const int n = c->nl[l];
-  return (n == 32 || n == 16) && c->coarse_inv && c->nl[c->nlev - 1] == 4 && c->cfg.schedule == MMH_SCHED_TOL &&
-         !c->cfg.precond_guards;
+  return (n == 32 || n == 16) && !prof_armed() && c->coarse_inv && c->nl[c->nlev - 1] == 4 &&
+         c->cfg.schedule == MMH_SCHED_TOL && !c->cfg.precond_guards;
 }
 
 // the special restriction planes of the levels from n down (n, n/2, n/4)
