@@ -177,7 +177,8 @@ int mmh_iterate(mmh_ctx* ctx, int niter, mmh_diag* diag);
 /* Copy the state back to the host (either pointer may be NULL). */
 int mmh_store_f64(mmh_ctx* ctx, double* def, double* u, int nfluid);
 /* Spectral outputs of the current def to the host: grad(n,n,n,3), delta(n,n,n)
- * (either may be NULL).  mmh/main.f90:131-179 */
+ * (either may be NULL).  A cell of def that is not finite makes every value of
+ * them NaN, here and in the two calls above.  mmh/main.f90:131-179 */
 int mmh_outputs_f64(mmh_ctx* ctx, double* grad, double* delta);
 /* Same to device memory: d_grad (3 n^3 doubles), d_delta (n^3 doubles). */
 int mmh_outputs_dev(mmh_ctx* ctx, double* d_grad, double* d_delta);

@@ -142,10 +142,11 @@ void launch_spec_pack(const void* Xc, int n, void* Z, const LimDev* st, const do
 void launch_spec_unpack(const void* z, int n, double* out, const LimDev* st, cudaStream_t s);
 // spectral outputs line by line (mmh_spectral.cu): grad (3 n^3) and delta (n^3)
 // of src, either may be null; tab: 4 n doubles made once by launch_fft_tables;
-// T: scratch of 2 n^2 doubles
+// T: scratch of 2 n^2 doubles; bad: one word.  A cell of src that is not finite
+// makes every value NaN, as a three-dimensional transform would.
 void launch_fft_tables(double* tab, int n, cudaStream_t s);
 void launch_spectral_lines(const double* src, int n, double* grad, double* delta, const double* tab, double* T,
-                           cudaStream_t s);
+                           unsigned* bad, cudaStream_t s);
 // rcc (may be null): receives 1 / cc, and baj's first six planes the metric
 // times det, both for launch_relax_flux (which is then given it too)
 void launch_relax_stage1(const double* rho, const double* def, const double* defp, int n, double* baj, double* cc,

@@ -967,12 +967,14 @@ int relaxing_dev(mmh_ctx* c, double dt, bool split = false) {
 // spectral outputs of src into device buffers (grad: 3 planes of n^3)
 int spectral_outputs(mmh_ctx* c, const double* src, double* d_grad, double* d_delta) {
   Stage stage_("mmh spectral outputs");
+  const i64 n = c->n;
   if (!c->linetab) {
-    const i64 n = c->n;
-    RET(c->alloc(&c->linetab, 4 * n + 2 * n * n));  // tables, then the alternating sums
+    RET(c->alloc(&c->linetab, 4 * n + 2 * n * n + 1));  // tables, the alternating sums, the word for non-finite cells
     launch_fft_tables(c->linetab, c->n, c->s);
   }
-  launch_spectral_lines(src, c->n, d_grad, d_delta, c->linetab, c->linetab + 4 * (i64)c->n, c->s);
+  double* sums = c->linetab + 4 * n;
+  launch_spectral_lines(src, c->n, d_grad, d_delta, c->linetab, sums, reinterpret_cast<unsigned*>(sums + 2 * n * n),
+                        c->s);
   CK(cudaGetLastError());
   return MMH_OK;
 }

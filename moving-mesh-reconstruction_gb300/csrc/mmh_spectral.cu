@@ -137,6 +137,11 @@ struct LineArgs {
   const double* w;       // y, z: pi / n times the ky (kz) = n/2 operator's result
   const double* tab;
   int axis;
+  // A cell that is not finite would reach its own lines only, where the
+  // three-dimensional transform carries it into every value: the x pass sets
+  // *bad when a line's sum is not finite, the z pass then leaves NaN everywhere.
+  unsigned* bad;
+  double* all;  // z: the displacement's three planes (null: not wanted)
 };
 
 template <int N>
@@ -154,6 +159,15 @@ __global__ void __launch_bounds__(Fft<N>::NT) k_lines(LineArgs a) {
   const i64 js = a.axis == kAxisY ? N : a.axis == kAxisZ ? n2 : 1;
   const i64 ls = along_x ? 2 * N : 2, io = along_x ? N : 1;
   const i64 base = (i64)blockIdx.x * LC * ls + (a.axis == kAxisZ ? (i64)N * blockIdx.y : n2 * blockIdx.y);
+  if (a.axis == kAxisZ && *a.bad) {
+    const double nan = __hiloint2double(0x7ff80000, 0);
+    for (int t = tid; t < 2 * LC * N; t += NT) {
+      const i64 c = base + t % (2 * LC) + t / (2 * LC) * n2;
+      for (int ax = 0; ax < 3 && a.all; ++ax) a.all[ax * n2 * N + c] = nan;
+      if (a.delta) a.delta[c] = nan;
+    }
+    return;
+  }
   const double2* tw = reinterpret_cast<const double2*>(a.tab);
   const double* kd = a.tab + 2 * N;
   const double* ks = a.tab + 3 * N;
@@ -208,6 +222,8 @@ __global__ void __launch_bounds__(Fft<N>::NT) k_lines(LineArgs a) {
   __syncthreads();
   if constexpr (F::S >= 2) in_place(A, std::integral_constant<int, F::R1>(), F::R0);
   if constexpr (F::S >= 3) in_place(A, std::integral_constant<int, F::R2>(), F::R0 * F::R1);
+  // a line's sum is its k = 0 value
+  if (a.axis == kAxisX && tid < LC && max(bexp(A[tid * P].x), bexp(A[tid * P].y)) == 2047) *a.bad = 1;
 
   // inverse of m(l, k) (a multiplied spectrum with real and imaginary parts
   // exchanged, which turns the forward transform into the inverse), emitted
@@ -301,21 +317,24 @@ __global__ void __launch_bounds__(Fft<N>::NT) k_lines(LineArgs a) {
 }
 
 template <int N>
-void lines_run(const double* src, double* grad, double* delta, const double* tab, double* T, cudaStream_t s) {
+void lines_run(const double* src, double* grad, double* delta, const double* tab, double* T, unsigned* bad,
+               cudaStream_t s) {
   typedef Fft<N> F;
   constexpr int smem = 2 * F::LC * (N + 1) * (int)sizeof(double2);
   static std::atomic<unsigned long long> done{0};
   smem_attr_once(k_lines<N>, smem, done);
   const i64 n2 = (i64)N * N, n3 = n2 * N;
   const dim3 grid(N / 2 / F::LC, N);
+  cudaMemsetAsync(bad, 0, sizeof(unsigned), s);
   if (grad) {
     k_altsum<<<dim3((unsigned)((n2 + 127) / 128), 2), 128, 0, s>>>(src, N, T);
     // both T fields, in place: a CTA has read its lines before it writes them
-    k_lines<N><<<dim3(N / F::LC, 1), F::NT, smem, s>>>(LineArgs{T, T, nullptr, nullptr, tab, kHilbert});
+    k_lines<N><<<dim3(N / F::LC, 1), F::NT, smem, s>>>(LineArgs{T, T, nullptr, nullptr, tab, kHilbert, nullptr, nullptr});
     count_launch(2);
   }
   for (int ax = 0; ax < 3; ++ax) {
-    const LineArgs a{src, grad ? grad + ax * n3 : nullptr, delta, ax == 0 ? nullptr : T + (ax - 1) * n2, tab, ax};
+    const LineArgs a{src, grad ? grad + ax * n3 : nullptr, delta, ax == 0 ? nullptr : T + (ax - 1) * n2, tab, ax, bad,
+                     grad};
     k_lines<N><<<grid, F::NT, smem, s>>>(a);
     count_launch();
   }
@@ -329,16 +348,16 @@ void launch_fft_tables(double* tab, int n, cudaStream_t s) {
 }
 
 void launch_spectral_lines(const double* src, int n, double* grad, double* delta, const double* tab, double* T,
-                           cudaStream_t s) {
+                           unsigned* bad, cudaStream_t s) {
   switch (n) {
-    case 8: lines_run<8>(src, grad, delta, tab, T, s); break;
-    case 16: lines_run<16>(src, grad, delta, tab, T, s); break;
-    case 32: lines_run<32>(src, grad, delta, tab, T, s); break;
-    case 64: lines_run<64>(src, grad, delta, tab, T, s); break;
-    case 128: lines_run<128>(src, grad, delta, tab, T, s); break;
-    case 256: lines_run<256>(src, grad, delta, tab, T, s); break;
-    case 512: lines_run<512>(src, grad, delta, tab, T, s); break;
-    default: lines_run<1024>(src, grad, delta, tab, T, s); break;
+    case 8: lines_run<8>(src, grad, delta, tab, T, bad, s); break;
+    case 16: lines_run<16>(src, grad, delta, tab, T, bad, s); break;
+    case 32: lines_run<32>(src, grad, delta, tab, T, bad, s); break;
+    case 64: lines_run<64>(src, grad, delta, tab, T, bad, s); break;
+    case 128: lines_run<128>(src, grad, delta, tab, T, bad, s); break;
+    case 256: lines_run<256>(src, grad, delta, tab, T, bad, s); break;
+    case 512: lines_run<512>(src, grad, delta, tab, T, bad, s); break;
+    default: lines_run<1024>(src, grad, delta, tab, T, bad, s); break;
   }
 }
 
