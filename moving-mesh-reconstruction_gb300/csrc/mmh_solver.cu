@@ -951,9 +951,12 @@ int relaxing_dev(mmh_ctx* c, double dt, bool split = false) {
   int n = c->n;
   if (c->cfg.precision == MMH_MIXED) {
     if (!split) launch_ff_split2(c->def, c->defs(), c->defp(), c->aux_split(), c->n3, c->s);
-    // FP32 fluxes, FP64 update (the relaxing buffers hold the FP32 scratch)
-    launch_relax32(c->rho, c->defs(), c->aux_split(), n, dt, reinterpret_cast<float4*>(c->baj), reinterpret_cast<float*>(c->cc),
-                   reinterpret_cast<float*>(c->u1), c->s);
+    // FP32 fluxes, FP64 update.  The scratch (half of the finest coefficient
+    // planes, which hold nothing between solves) is not the relaxing buffers:
+    // those overlap the spectral buffers, where the splits are.
+    double* g = c->h64.coef[0];
+    float* uf = reinterpret_cast<float*>(g + 2 * c->n3);
+    launch_relax32(c->rho, c->defs(), c->aux_split(), n, dt, reinterpret_cast<float4*>(g), uf, uf + c->n3, c->s);
     return MMH_OK;
   }
   double* rcc = c->tmp();  // 1 / cc
@@ -1546,10 +1549,12 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
   }
   int rc = MMH_OK;
   i64 n3 = c->n3;
-  // Scratch that is dead while relaxing runs (finest-level multigrid scratch,
-  // limiter and spectral buffers, PCG vectors) shares one allocation with the
-  // relaxing buffers, which are dead whenever that scratch is in use: this
-  // takes 18 fields off the footprint (1024^3 fits on one GPU).
+  // Scratch that is dead while the FP64 relaxing and its adjoint run
+  // (finest-level multigrid scratch, limiter and spectral buffers, PCG vectors)
+  // shares one allocation with their buffers (baj to u1), which are dead
+  // whenever that scratch is in use: this takes 18 fields off the footprint
+  // (1024^3 fits on one GPU).  The mixed form's relaxing reads the splits in the
+  // spectral buffers and so keeps off baj to u1 (relaxing_dev).
   struct Piece {
     void** p;
     size_t bytes;
