@@ -364,9 +364,10 @@ int mmh_gs_tile(int n, int* tx, int* ty);
  * The event pool grows with the launches timed; mmh_profile_stop returns
  * MMH_ERR_NOMEM (with the figures of the launches it did time) when a launch
  * went untimed because no event could be created.  While armed, the
- * preconditioner cycle runs launch by launch instead of from its CUDA graph,
- * and so do the mixed form's levels of 32^3 and below, which otherwise are one
- * launch per cycle or per inner solve (the same bits). */
+ * preconditioner cycle runs launch by launch instead of from its CUDA graph.
+ * The mixed form's levels of 32^3 and below are one launch per cycle or per
+ * inner solve; they too run launch by launch (the same bits) while an FP32 kind
+ * is armed for every grid or for one of theirs. */
 #define MMH_K_GS 1
 #define MMH_K_RESIDUAL 2
 #define MMH_K_RESTRICT_RESID 3

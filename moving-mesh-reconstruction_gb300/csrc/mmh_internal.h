@@ -22,6 +22,8 @@ enum KernelKind {
 void prof_begin(int kind, cudaStream_t s, i64 cells, int n);
 void prof_end(int kind, cudaStream_t s, int n);
 int prof_start(int kind);
+// an armed FP32 kind times launches on levels of n^3 or below
+bool prof_armed_f32(int n);
 bool prof_armed();  // timing hooks armed: launches must stay individual (no graph replay)
 int prof_stop(int* launches, double* ms, long long* cells);
 template <class T> inline int kk(int base) { return base | (sizeof(T) == 4 ? KK_F32 : 0); }

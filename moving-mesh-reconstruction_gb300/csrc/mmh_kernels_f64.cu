@@ -34,6 +34,7 @@ Prof g_prof;
 }  // namespace
 
 bool prof_armed() { return g_prof.kind != 0; }
+bool prof_armed_f32(int n) { return (g_prof.kind & KK_F32) && (g_prof.kind >> 12) <= n; }
 
 // Events are created in chunks as launches are timed (the pool grows with the
 // launch count: a 512^3 reconstruction times ~2400 finest-level launches).

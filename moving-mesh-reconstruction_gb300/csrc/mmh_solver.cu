@@ -281,10 +281,10 @@ int vcycle_fp64(mmh_ctx* c, int l);
 
 // Whether the FP32 levels from l down run as one launch (mmh_cycle32.cu): the
 // 32^3 and 16^3 levels of a cycle without guards and with the exact 4^3 solve.
-// While the timing hooks are armed they run launch by launch (the same bits).
+// While an FP32 kind is armed there they run launch by launch (the same bits).
 bool cycle32_at(const mmh_ctx* c, int l) {
   const int n = c->nl[l];
-  return (n == 32 || n == 16) && !prof_armed() && c->coarse_inv && c->nl[c->nlev - 1] == 4 &&
+  return (n == 32 || n == 16) && !prof_armed_f32(n) && c->coarse_inv && c->nl[c->nlev - 1] == 4 &&
          c->cfg.schedule == MMH_SCHED_TOL && !c->cfg.precond_guards;
 }
 
