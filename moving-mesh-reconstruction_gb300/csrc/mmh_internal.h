@@ -37,11 +37,11 @@ void launch_metric(const T* def, const T* rho, int n, T dx, T* coef, cudaStream_
                    T* det = nullptr);
 void launch_residual_fma(const double* phi, const double* rhs, const double* coef, int n, double dx, float* r32,
                          unsigned long long* maxbits, cudaStream_t s);
-// nsweeps 8-colour sweeps of phi; returns the buffer that holds the swept
-// field, phi or scratch (the other one is then free)
+// nsweeps FP32 8-colour sweeps of phi (T = float); returns the buffer that holds
+// the swept field, phi or scratch (the other one is then free)
 template <class T> T* launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch,
                                        cudaStream_t s, bool zero_init = false);
-// the FP64 sweeps of launch_gs_sweeps (mmh_gs64.cu)
+// the same in FP64 (mmh_gs64.cu)
 double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
                            double* scratch, cudaStream_t s);
 // The FP64 form's operator on grids of 32^3 and up: sums of coefficients 1, 4,

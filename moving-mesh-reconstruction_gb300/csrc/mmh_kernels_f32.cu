@@ -77,6 +77,8 @@ int gs_tile_chosen(int n, int* tx, int* ty) {
 }
 
 MMH_INSTANTIATE(float)
+template float* launch_gs_sweeps<float>(float*, const float*, const float*, int, float, int, float*, cudaStream_t,
+                                        bool);
 MMH_INSTANTIATE_PCG(float)
 
 // Dot products of FP32 vectors for the mixed form's inner solve, whose

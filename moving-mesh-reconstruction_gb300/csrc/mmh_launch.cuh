@@ -101,14 +101,15 @@ inline bool gs_shape_fits(int v, int n) {
 int gs_tile_choice(int n, const float* phi, const float* rhs, const float* coef, float dx2, float* scratch,
                    cudaStream_t s);
 
-// nsweeps FP32 8-colour Gauss-Seidel sweeps.  Grids of 64^3 and up run one fused
-// launch per half sweep (all in-plane colours of every plane of one parity);
-// smaller grids run one launch per colour.
-// zero_init: phi holds no field yet and the sweeps start from zero (grids of 64^3 and up run the first sweep in place without reading phi;
-// elsewhere phi is zeroed first).
+// nsweeps FP32 8-colour Gauss-Seidel sweeps (T = float).  Grids of 64^3 and up
+// run one fused launch per half sweep (all in-plane colours of every plane of
+// one parity); smaller grids run one launch per colour.
+// zero_init: phi holds no field yet and the sweeps start from zero (grids of
+// 64^3 and up run the first sweep in place without reading phi; elsewhere phi
+// is zeroed first).
 template <class T>
-T* launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
-                      bool zero_init) {
+T* launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
+                    bool zero_init) {
   i64 h3 = (i64)(n / 2) * (n / 2) * (n / 2);
   T dx2 = dx * dx;
   int sw0 = 0;
@@ -177,17 +178,6 @@ T* launch_gs32_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nswe
           count_launch();
         }
   return phi;
-}
-
-template <class T>
-T* launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch, cudaStream_t s,
-                    bool zero_init) {
-  if constexpr (std::is_same<T, double>::value) {
-    if (zero_init) launch_fill<double>(phi, (i64)n * n * n, 0.0, s);
-    return launch_gs64_sweeps(phi, rhs, coef, n, dx, nsweeps, scratch, s);
-  } else {
-    return launch_gs32_sweeps<T>(phi, rhs, coef, n, dx, nsweeps, scratch, s, zero_init);
-  }
 }
 
 // The marching FP32 stencil (k_stencil_march) for grids of 64 and up, unless
@@ -344,7 +334,6 @@ void launch_usum_flag(const unsigned long long* acc, int* flag, cudaStream_t s) 
 
 #define MMH_INSTANTIATE(T)                                                                                          \
   template void launch_metric<T>(const T*, const T*, int, T, T*, cudaStream_t, bool, T*);                         \
-  template T* launch_gs_sweeps<T>(T*, const T*, const T*, int, T, int, T*, cudaStream_t, bool);                         \
   template void launch_residual<T>(const T*, const T*, const T*, int, T, T*, float*, unsigned long long*,          \
                                    cudaStream_t);                                                                   \
   template void launch_restrict_resid<T>(const T*, int, int, T*, cudaStream_t);                                   \

@@ -70,7 +70,7 @@ extern "C" int mmh_relax_noalloc_f64(const double* d_deformpot, const double* d_
   double* buf = scratch + 6 * n3;         // n^3: Gauss-Seidel double buffer
   unsigned long long* maxw = reinterpret_cast<unsigned long long*>(scratch + 7 * kMaxN3);
   launch_metric<double>(d_deformpot, d_rho, n, dx, coef, s);
-  if (launch_gs_sweeps<double>(d_arr, d_rhs, coef, n, dx, nrelax, buf, s) != d_arr &&
+  if (launch_gs64_sweeps(d_arr, d_rhs, coef, n, dx, nrelax, buf, s) != d_arr &&
       cudaMemcpyAsync(d_arr, buf, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return MMH_ERR_CUDA;
   if (cudaGetLastError() != cudaSuccess) return MMH_ERR_CUDA;

@@ -88,19 +88,17 @@ template <class T>
 void launch_apply(const T* p, const T* coef, int n, T dx, T* q, unsigned long long* qbits, cudaStream_t s) {
   i64 n3 = (i64)n * n * n;
   prof_begin(kk<T>(KK_APPLY), s, n3, n);
+  // (the FP64 form's grids of 32^3 and up take launch_apply64)
   bool done = false;
   if constexpr (std::is_same<T, float>::value) {
-    if (use_march(n)) {
+    done = n >= 32;
+    if (use_march(n))
       launch_stencil_march<1>(p, nullptr, coef, n, T(1) / (dx * dx), q, qbits, s);
-      done = true;
-    }
+    else if (done)
+      k_stencil_plane<T, 1><<<dim3(n / 32, n / 16, n), 256, 0, s>>>(p, nullptr, coef, n, T(1) / (dx * dx), q, nullptr,
+                                                                   qbits);
   }
-  if (done) {
-  } else if (n >= 32)
-    k_stencil_plane<T, 1><<<dim3(n / 32, n / 16, n), 256, 0, s>>>(p, nullptr, coef, n, T(1) / (dx * dx), q, nullptr,
-                                                                 qbits);
-  else
-    k_apply<T><<<grid_of(n3, kBlock), kBlock, 0, s>>>(p, coef, n, T(1) / (dx * dx), q, qbits);
+  if (!done) k_apply<T><<<grid_of(n3, kBlock), kBlock, 0, s>>>(p, coef, n, T(1) / (dx * dx), q, qbits);
   prof_end(kk<T>(KK_APPLY), s, n);
   count_launch();
 }

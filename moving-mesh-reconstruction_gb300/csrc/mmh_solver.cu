@@ -220,6 +220,17 @@ Hier<double>& hier<double>(mmh_ctx* c) { return c->h64; }
 template <>
 Hier<float>& hier<float>(mmh_ctx* c) { return c->h32; }
 
+// r = b - L x and q = L p of the FP64 form on level l, max|.| into maxbits
+void residual64(mmh_ctx* c, int l, double dx, const double* x, const double* b, double* r,
+                unsigned long long* maxbits) {
+  if (c->faces_at(l)) launch_residual64(x, b, c->face[l], c->nl[l], dx, r, maxbits, c->s);
+  else launch_residual<double>(x, b, c->h64.coef[l], c->nl[l], dx, r, nullptr, maxbits, c->s);
+}
+void apply64(mmh_ctx* c, int l, double dx, const double* p, double* q, unsigned long long* qbits) {
+  if (c->faces_at(l)) launch_apply64(p, c->face[l], c->nl[l], dx, q, qbits, c->s);
+  else launch_apply<double>(p, c->h64.coef[l], c->nl[l], dx, q, qbits, c->s);
+}
+
 // relax(): nrelax 8-colour sweeps of the field in u, then residual (mode 3:
 // full weighting into rhs[l+1] and max norm; mode 2: max norm only; mode 0:
 // none) into *maxslot (null: no norm).  The sweeps go back and forth between u
@@ -231,21 +242,21 @@ int relax_level(mmh_ctx* c, int l, T*& u, T*& r, int nrelax, int mode, unsigned 
   Hier<T>& H = hier<T>(c);
   int n = c->nl[l];
   T dx = T(double(1 << l));
-  bool done = false;
+  T* swept;
   if constexpr (std::is_same<T, double>::value) {
-    if (c->faces_at(l)) {
-      if (launch_gs64_sweeps(u, H.rhs[l], c->face[l], n, dx, nrelax, r, c->s) != u) std::swap(u, r);
-      done = true;
-    }
+    swept = c->faces_at(l) ? launch_gs64_sweeps(u, H.rhs[l], c->face[l], n, dx, nrelax, r, c->s)
+                           : launch_gs64_sweeps(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s);
+  } else {
+    swept = launch_gs_sweeps<T>(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s, zero_init);
   }
-  if (!done && launch_gs_sweeps<T>(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s, zero_init) != u) std::swap(u, r);
+  if (swept != u) std::swap(u, r);
   if (mode == 0) return MMH_OK;
   if (maxslot) CK(cudaMemsetAsync(maxslot, 0, 8, c->s));
   T* res = mode == 3 ? r : nullptr;
-  if constexpr (std::is_same<T, double>::value) {
-    if (done) launch_residual64(u, H.rhs[l], c->face[l], n, dx, res, maxslot, c->s);
-  }
-  if (!done) launch_residual<T>(u, H.rhs[l], H.coef[l], n, dx, res, nullptr, maxslot, c->s);
+  if constexpr (std::is_same<T, double>::value)
+    residual64(c, l, dx, u, H.rhs[l], res, maxslot);
+  else
+    launch_residual<T>(u, H.rhs[l], H.coef[l], n, dx, res, nullptr, maxslot, c->s);
   if (mode == 3) launch_restrict_resid<T>(r, n, special_plane(nrelax, n), H.rhs[l + 1], c->s);
   return MMH_OK;
 }
@@ -470,17 +481,6 @@ int precond_replay(mmh_ctx* c, int l0) {
   return MMH_OK;
 }
 
-// r = b - L x and q = L p of the FP64 form on level l, max|.| into maxbits
-void residual64(mmh_ctx* c, int l, double dx, const double* x, const double* b, double* r,
-                unsigned long long* maxbits) {
-  if (c->faces_at(l)) launch_residual64(x, b, c->face[l], c->nl[l], dx, r, maxbits, c->s);
-  else launch_residual<double>(x, b, c->h64.coef[l], c->nl[l], dx, r, nullptr, maxbits, c->s);
-}
-void apply64(mmh_ctx* c, int l, double dx, const double* p, double* q, unsigned long long* qbits) {
-  if (c->faces_at(l)) launch_apply64(p, c->face[l], c->nl[l], dx, q, qbits, c->s);
-  else launch_apply<double>(p, c->h64.coef[l], c->nl[l], dx, q, qbits, c->s);
-}
-
 // Flexible preconditioned conjugate gradients on L x = b at level l0 in
 // precision T, one V-cycle per iteration as preconditioner, until
 // max|r| <= tol * bn (recurrence residual) or maxit iterations.  The residual
@@ -600,14 +600,15 @@ int pcg_core32(mmh_ctx* c, int l0, double dx, float* x, float* p, float* q, doub
   return status;
 }
 
-// FP64 true residual of x against b at level l0: max|b - L x| (also copied
-// to FP32 in r32 when given).  The mixed form evaluates it with fused
-// multiply-adds; the FP64 form keeps the reference's separate roundings.
+// FP64 true residual of x against b at level l0: max|b - L x|.  The mixed form
+// evaluates it with fused multiply-adds and can copy it to FP32 (r32); the FP64
+// form keeps the reference's separate roundings and takes no r32.
 int true_residual(mmh_ctx* c, int l0, double dx, const double* x, const double* b, float* r32, double* rmax) {
-  int n = c->nl[l0];
+  const bool mixed = c->cfg.precision == MMH_MIXED;
+  if (r32 && !mixed) return MMH_ERR_ARG;
   CK(cudaMemsetAsync(&c->sc->resbits, 0, 8, c->s));
-  if (c->cfg.precision == MMH_MIXED)
-    launch_residual_fma(x, b, c->h64.coef[l0], n, dx, r32, &c->sc->resbits, c->s);
+  if (mixed)
+    launch_residual_fma(x, b, c->h64.coef[l0], c->nl[l0], dx, r32, &c->sc->resbits, c->s);
   else
     residual64(c, l0, dx, x, b, nullptr, &c->sc->resbits);
   RET(pull_scal(c));
@@ -1935,7 +1936,7 @@ int mmh_relax_f64(mmh_ctx* c, double* arr, double* resid, const double* rhs, con
   }
   launch_metric<double>(c->defl[l], c->rhol[l], n, dx, c->h64.coef[l], c->s);
   double *du = c->h64.u[l], *dr = c->h64.r[l];
-  if (launch_gs_sweeps<double>(du, c->h64.rhs[l], c->h64.coef[l], n, dx, nrelax, dr, c->s) != du) std::swap(du, dr);
+  if (launch_gs64_sweeps(du, c->h64.rhs[l], c->h64.coef[l], n, dx, nrelax, dr, c->s) != du) std::swap(du, dr);
   CK(cudaMemsetAsync(c->sc->errbits, 0, 8, c->s));
   if (ir != 0) {
     launch_residual<double>(du, c->h64.rhs[l], c->h64.coef[l], n, dx, ir == 3 ? dr : nullptr,
