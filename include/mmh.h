@@ -198,6 +198,14 @@ typedef struct mmh_stats {
 } mmh_stats;
 int mmh_state_stats(mmh_ctx* ctx, mmh_stats* stats);
 
+/* Kernels of the levels of 32^3 and below run as clusters of up to 16 CTAs
+ * where the GPU, or the partition of it that the context's stream runs on,
+ * holds such a cluster, and as smaller clusters or one launch per level where
+ * it does not; the results have the same bits.  mmh_max_cluster(ctx, 8) takes
+ * the second way everywhere on this context, mmh_max_cluster(ctx, 16) goes back
+ * to the first. */
+int mmh_max_cluster(mmh_ctx* ctx, int ctas);
+
 /* The limiter's trigger masks of the last calcdefp run on the context
  * (mmh_calcdefp*, mmh_iterate), for checking them against the reference's:
  * expand and compress1 are pass 1's expansion and compression triggers

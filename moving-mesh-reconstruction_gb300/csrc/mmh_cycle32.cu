@@ -627,6 +627,14 @@ CycleArgs cycle_args(int n, const float* c0, const float* c1, const float* c2, c
 
 }  // namespace
 
+// the inner solve at 32^3 has the most shared memory of the four
+bool cycle32_fits(cudaStream_t s) {
+  static std::atomic<unsigned long long> d0{0}, d1{0};
+  smem_attr_once(k_solve32<32>, Layout<32>::BYTES_SOLVE, d0);
+  func_attr_once(k_solve32<32>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1, d1);
+  return cluster_fits(k_solve32<32>, kCta, kThreads, Layout<32>::BYTES_SOLVE, s);
+}
+
 void launch_cycle32(int n, const float* c0, const float* c1, const float* c2, const double* M, double dx, int nu1,
                     int nu2, const int* special, const float* rhs, float* u, cudaStream_t s) {
   const CycleArgs a = cycle_args(n, c0, c1, c2, M, dx, nu1, nu2, special);

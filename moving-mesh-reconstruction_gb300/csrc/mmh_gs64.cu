@@ -30,9 +30,9 @@ namespace mmh {
 namespace {
 
 // ---------------------------------------------------------------------------
-// n >= 32: one half sweep (the four in-plane colours of every plane of one
-// parity).  A CTA owns TY full rows of one plane.  phi of the plane (rows -3
-// .. TY+3) sits in shared memory, each row split into its even-x and odd-x
+// n >= 32 (and 16 where the box kernel's cluster does not fit): one half sweep
+// (the four in-plane colours of every plane of one parity).  A CTA owns TY full
+// rows of one plane.  phi of the plane (rows -3 .. TY+3) sits in shared memory, each row split into its even-x and odd-x
 // half, so the lanes of a colour read consecutive words; everything else is
 // read once per update from global memory (L1/L2), which costs a tenth of the
 // FP64 time.  Colour q is updated on the rows q-2, q, ... that the later
@@ -234,7 +234,7 @@ int lg(int n) {
   while ((1 << l) < n) ++l;
   return l;
 }
-int rows_ty(int n) { return n == 32 ? 8 : (n == 64 || n > 512 ? 16 : 32); }
+int rows_ty(int n) { return n <= 32 ? 8 : (n == 64 || n > 512 ? 16 : 32); }
 
 // ---------------------------------------------------------------------------
 // n = 4, 8, 16: nsweeps whole 8-colour sweeps in one launch.  A cluster of CL
@@ -544,16 +544,19 @@ __global__ void __launch_bounds__(BoxGeom<N>::NT) k_gs_box(double* __restrict__ 
   }
 }
 
+// whether the box kernel of n = 16 has its cluster of 16 CTAs
+bool box16_fits(cudaStream_t s) {
+  typedef BoxGeom<16> G;
+  static std::atomic<unsigned long long> attr_done{0};
+  func_attr_once(k_gs_box<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1, attr_done);
+  return cluster_fits(k_gs_box<16>, G::CL, G::NT, 0, s);
+}
 template <int N>
 void box_launch(double* phi, const double* rhs, const double* coef, double dx2, int nsweeps, cudaStream_t s) {
   typedef BoxGeom<N> G;
   if (G::CL == 1) {
     k_gs_box<N><<<1, G::NT, 0, s>>>(phi, rhs, coef, 2.0 * dx2, nsweeps);
     return;
-  }
-  if (G::CL > 8) {
-    static std::atomic<unsigned long long> attr_done{0};
-    func_attr_once(k_gs_box<N>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1, attr_done);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(G::CL);
@@ -590,13 +593,14 @@ void rows_launch(const double* src, const double* nbr, double* dst, const double
   cfg.numAttrs = CL ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k_gs_rows<PRE, CL>, src, nbr, dst, rhs, f, lgn, ty, dx2x2, kpar);
 }
-// faces: the coefficients' face sums (null: the coefficient planes themselves)
+// faces: the coefficients' face sums (null: the coefficient planes themselves).
+// A 16^3 grid goes by rows where its box kernel's cluster does not fit.
 double* gs64_sweeps(double* phi, const double* rhs, const double* coef, const Face64* faces, int n, double dx,
-                    int nsweeps, double* scratch, cudaStream_t s) {
+                    int nsweeps, double* scratch, cudaStream_t s, int max_cluster) {
   if (nsweeps <= 0) return phi;
   const i64 h3 = (i64)(n / 2) * (n / 2) * (n / 2);
   const double dx2 = dx * dx;
-  if (n <= 16) {
+  if (n <= 8 || (n == 16 && max_cluster >= 16 && box16_fits(s))) {
     prof_begin(KK_GS, s, h3 * 8 * nsweeps, n);
     if (n == 4) box_launch<4>(phi, rhs, coef, dx2, nsweeps, s);
     else if (n == 8) box_launch<8>(phi, rhs, coef, dx2, nsweeps, s);
@@ -628,14 +632,14 @@ double* gs64_sweeps(double* phi, const double* rhs, const double* coef, const Fa
 }  // namespace
 
 // nsweeps FP64 8-colour sweeps of phi on an n^3 grid; scratch: n^3 doubles
-// (n >= 32).  Returns the buffer that holds the swept field.
+// (n >= 16).  Returns the buffer that holds the swept field.
 double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
-                           double* scratch, cudaStream_t s) {
-  return gs64_sweeps(phi, rhs, coef, nullptr, n, dx, nsweeps, scratch, s);
+                           double* scratch, cudaStream_t s, int max_cluster) {
+  return gs64_sweeps(phi, rhs, coef, nullptr, n, dx, nsweeps, scratch, s, max_cluster);
 }
 double* launch_gs64_sweeps(double* phi, const double* rhs, const Face64& f, int n, double dx, int nsweeps,
                            double* scratch, cudaStream_t s) {
-  return gs64_sweeps(phi, rhs, nullptr, &f, n, dx, nsweeps, scratch, s);
+  return gs64_sweeps(phi, rhs, nullptr, &f, n, dx, nsweeps, scratch, s, 16);
 }
 
 Face64 launch_faces64(double* coef, int n, double* s0, double* s1, cudaStream_t s) {

@@ -41,9 +41,10 @@ void launch_residual_fma(const double* phi, const double* rhs, const double* coe
 // the swept field, phi or scratch (the other one is then free)
 template <class T> T* launch_gs_sweeps(T* phi, const T* rhs, const T* coef, int n, T dx, int nsweeps, T* scratch,
                                        cudaStream_t s, bool zero_init = false);
-// the same in FP64 (mmh_gs64.cu)
+// the same in FP64 (mmh_gs64.cu); max_cluster: the most CTAs a cluster may have
+// (8 or 16; 16 is used where it fits)
 double* launch_gs64_sweeps(double* phi, const double* rhs, const double* coef, int n, double dx, int nsweeps,
-                           double* scratch, cudaStream_t s);
+                           double* scratch, cudaStream_t s, int max_cluster = 16);
 // The FP64 form's operator on grids of 32^3 and up: sums of coefficients 1, 4,
 // 6 at a cell and the next one along their axis (twice the upper face's
 // coefficient), coefficients 2, 3, 5, the sum of the six face sums (-2 times
@@ -54,7 +55,7 @@ struct Face64 {
 // from the six coefficient planes, three of which it overwrites; s0, s1: n^3 each
 Face64 launch_faces64(double* coef, int n, double* s0, double* s1, cudaStream_t s);
 double* launch_gs64_sweeps(double* phi, const double* rhs, const Face64& f, int n, double dx, int nsweeps,
-                           double* scratch, cudaStream_t s);
+                           double* scratch, cudaStream_t s);  // n >= 32
 // launch_residual<double> and launch_apply<double> from the face sums (the same bits)
 void launch_residual64(const double* phi, const double* rhs, const Face64& f, int n, double dx, double* r,
                        unsigned long long* maxbits, cudaStream_t s);
@@ -104,7 +105,7 @@ void launch_add_f2d(double* a, const float* b, i64 count, cudaStream_t s);
 void launch_add(double* a, const double* b, i64 count, cudaStream_t s);  // a = a + b
 // exact FP64 solve of the 4^3 level (mixed form): M (64 x 64) from the level's
 // FP64 coefficients once per metric; z = M (r - mean r) per application
-void launch_coarse_inverse(const double* coef, double dx, double* M, cudaStream_t s);
+void launch_coarse_inverse(const double* coef, double dx, double* M, cudaStream_t s, int max_cluster = 16);
 void launch_coarse_apply(const float* r, const double* M, float* z, cudaStream_t s);
 
 // One FP32 V(nu1, nu2) cycle from the n^3 level (n = 32 or 16) down in one
@@ -112,7 +113,8 @@ void launch_coarse_apply(const float* r, const double* M, float* z, cudaStream_t
 // the level and of the next ones above 4^3 (c2 for n = 32 only); M: the 4^3
 // level's inverse; dx: the level's spacing; special: launch_restrict_resid's
 // argument on the level and the next ones.  The same bits as the per-level
-// launches.
+// launches.  Clusters of 16 CTAs: cycle32_fits says whether stream s has room.
+bool cycle32_fits(cudaStream_t s);
 void launch_cycle32(int n, const float* c0, const float* c1, const float* c2, const double* M, double dx, int nu1,
                     int nu2, const int* special, const float* rhs, float* u, cudaStream_t s);
 // The whole inner solve of the mixed form on such a grid, x from zero with

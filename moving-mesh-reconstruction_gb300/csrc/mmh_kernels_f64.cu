@@ -230,24 +230,24 @@ void launch_f2d(const float* a, double* b, i64 count, cudaStream_t s) {
 constexpr int kCoarseN = 64;
 // L entry by entry (the operator applied to unit vectors, so it is exactly
 // the smoother's operator), then an in-place Gauss-Jordan inversion (no
-// pivoting: -A is symmetric positive definite).  A cluster of 16 CTAs with
-// four rows each and one entry per thread, the matrix in registers: a pivot
-// step is an elimination of two FP64 instructions per thread, the pivot row's
-// division and scaling on its owner, and the row's broadcast through
+// pivoting: -A is symmetric positive definite).  A cluster of 16 CTAs (8 where
+// no 16 fit) shares the rows, one entry per thread, the matrix in registers: a
+// pivot step is an elimination of two FP64 instructions per thread, the pivot
+// row's division and scaling on its owner, and the row's broadcast through
 // distributed shared memory with one cluster barrier.  One CTA holding the
 // whole matrix is bound by its FP64 pipe (5000 cycles per step): 344 us per
 // metric, this form 63 us.  The same operations per entry, so the same bits.
-constexpr int kInvCtas = 16;
-__global__ void __launch_bounds__(256) k_coarse_inverse(const double* coef, double di2,
-                                                        double* M) {
+template <int CTAS>
+__global__ void __launch_bounds__(kCoarseN* kCoarseN / CTAS) k_coarse_inverse(const double* coef, double di2,
+                                                                              double* M) {
   pdl_begin();
-  constexpr int N = kCoarseN;
+  constexpr int N = kCoarseN, R = N / CTAS;
   __shared__ double unit[N][N];
-  __shared__ double diag[N], rowbuf[2][N], colp[2][4];
+  __shared__ double diag[N], rowbuf[2][N], colp[2][R];
   __shared__ double piv_s;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), tid = threadIdx.x;
-  const int r = tid >> 6, j = tid & 63, i = 4 * rank + r;
+  const int r = tid >> 6, j = tid & 63, i = R * rank + r;
   for (int q = tid; q < N * N; q += blockDim.x) unit[q / N][q % N] = q / N == q % N ? 1.0 : 0.0;
   cl.sync();  // the identity is here, and every CTA of the cluster runs
   double a;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(256) k_coarse_inverse(const double* coef, doub
     a = (t1 + t2 + tdiag * unit[j][i]) * di2;
   }
   if (i == j)
-    for (int q = 0; q < kInvCtas; ++q) *cl.map_shared_rank(&diag[i], q) = fabs(a);
+    for (int q = 0; q < CTAS; ++q) *cl.map_shared_rank(&diag[i], q) = fabs(a);
   cl.sync();
   if (tid == 0) {
     double d = 0.0;
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256) k_coarse_inverse(const double* coef, doub
     if (pivot) {
       a = (j == p ? 1.0 : a) * piv_s;
 #pragma unroll
-      for (int q = 0; q < kInvCtas; ++q) *cl.map_shared_rank(&rowbuf[p & 1][j], q) = a;
+      for (int q = 0; q < CTAS; ++q) *cl.map_shared_rank(&rowbuf[p & 1][j], q) = a;
     }
     cl.sync();
     if (!pivot) a = (j == p ? 0.0 : a) - colp[p & 1][r] * rowbuf[p & 1][j];
@@ -310,10 +310,13 @@ __global__ void __launch_bounds__(256) k_coarse_apply(const float* __restrict__ 
   if (tid < N) z[tid] = (float)((part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]));
 }
 
-void launch_coarse_inverse(const double* coef, double dx, double* M, cudaStream_t s) {
+void launch_coarse_inverse(const double* coef, double dx, double* M, cudaStream_t s, int max_cluster) {
   static std::atomic<unsigned long long> attr_done{0};
-  func_attr_once(k_coarse_inverse, cudaFuncAttributeNonPortableClusterSizeAllowed, 1, attr_done);
-  launch_cluster(k_coarse_inverse, kInvCtas, kInvCtas, 256, 0, s, coef, 1.0 / (dx * dx), M);
+  func_attr_once(k_coarse_inverse<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1, attr_done);
+  if (max_cluster >= 16 && cluster_fits(k_coarse_inverse<16>, 16, 256, 0, s))
+    launch_cluster(k_coarse_inverse<16>, 16, 16, 256, 0, s, coef, 1.0 / (dx * dx), M);
+  else
+    launch_cluster(k_coarse_inverse<8>, 8, 8, 512, 0, s, coef, 1.0 / (dx * dx), M);
   count_launch();
 }
 void launch_coarse_apply(const float* r, const double* M, float* z, cudaStream_t s) {

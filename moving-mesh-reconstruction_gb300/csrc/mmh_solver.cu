@@ -110,6 +110,10 @@ struct mmh_ctx {
   // the coefficient planes with each metric), and their two extra planes
   std::vector<Face64> face;
   std::vector<double*> face0, face1;
+  // clusters: the most CTAs one may have (8 or 16), and whether the 16 of
+  // mmh_cycle32.cu fit the stream's part of the GPU
+  int max_cluster = 16;
+  bool cycle_fits = false;
   bool faces_at(int l) const { return cfg.precision == MMH_FP64 && nl[l] >= 32; }
   // FP32 hierarchy (mixed)
   Hier<float> h32;
@@ -133,6 +137,14 @@ struct mmh_ctx {
   cudaGraphExec_t pgraph[2][16] = {};
   unsigned long long pgraph_launches[2][16] = {};
   bool pgraph_seen[2][16] = {};
+  void drop_graphs() {
+    for (int t = 0; t < 2; ++t)
+      for (int l = 0; l < 16; ++l) {
+        if (pgraph[t][l]) cudaGraphExecDestroy(pgraph[t][l]);
+        pgraph[t][l] = nullptr;
+        pgraph_seen[t][l] = false;
+      }
+  }
   void* pz[2][16] = {};  // the buffer a preconditioner application leaves its result in
   bool graphs = true;
   std::vector<void*> allocs;
@@ -245,7 +257,7 @@ int relax_level(mmh_ctx* c, int l, T*& u, T*& r, int nrelax, int mode, unsigned 
   T* swept;
   if constexpr (std::is_same<T, double>::value) {
     swept = c->faces_at(l) ? launch_gs64_sweeps(u, H.rhs[l], c->face[l], n, dx, nrelax, r, c->s)
-                           : launch_gs64_sweeps(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s);
+                           : launch_gs64_sweeps(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s, c->max_cluster);
   } else {
     swept = launch_gs_sweeps<T>(u, H.rhs[l], H.coef[l], n, dx, nrelax, r, c->s, zero_init);
   }
@@ -291,12 +303,13 @@ int guard_or_zerosum(mmh_ctx* c, int l, T* u, double margin, double floor_, bool
 int vcycle_fp64(mmh_ctx* c, int l);
 
 // Whether the FP32 levels from l down run as one launch (mmh_cycle32.cu): the
-// 32^3 and 16^3 levels of a cycle without guards and with the exact 4^3 solve.
+// 32^3 and 16^3 levels of a cycle without guards and with the exact 4^3 solve,
+// where a cluster of 16 CTAs fits.
 // While an FP32 kind is armed there they run launch by launch (the same bits).
 bool cycle32_at(const mmh_ctx* c, int l) {
   const int n = c->nl[l];
-  return (n == 32 || n == 16) && !prof_armed_f32(n) && c->coarse_inv && c->nl[c->nlev - 1] == 4 &&
-         c->cfg.schedule == MMH_SCHED_TOL && !c->cfg.precond_guards;
+  return (n == 32 || n == 16) && c->cycle_fits && c->max_cluster >= 16 && !prof_armed_f32(n) && c->coarse_inv &&
+         c->nl[c->nlev - 1] == 4 && c->cfg.schedule == MMH_SCHED_TOL && !c->cfg.precond_guards;
 }
 
 // the special restriction planes of the levels from n down (n, n/2, n/4)
@@ -423,7 +436,7 @@ int build_levels(mmh_ctx* c, int l0) {
     if (c->faces_at(l)) c->face[l] = launch_faces64(c->h64.coef[l], n, c->face0[l], c->face1[l], c->s);
   }
   if (c->coarse_inv && c->nl[c->nlev - 1] == 4)
-    launch_coarse_inverse(c->h64.coef[c->nlev - 1], double(1 << (c->nlev - 1)), c->coarse_inv, c->s);
+    launch_coarse_inverse(c->h64.coef[c->nlev - 1], double(1 << (c->nlev - 1)), c->coarse_inv, c->s, c->max_cluster);
   return MMH_OK;
 }
 
@@ -1510,9 +1523,7 @@ int mmh_destroy(mmh_ctx* c) {
     cufftDestroy(c->pd2z);
     cufftDestroy(c->pz2z);
   }
-  for (auto& row : c->pgraph)
-    for (cudaGraphExec_t& ex : row)
-      if (ex) cudaGraphExecDestroy(ex);
+  c->drop_graphs();
   for (void* p : c->allocs) cudaFree(p);
   if (c->hsc) cudaFreeHost(c->hsc);
   if (c->own_stream && c->s) cudaStreamDestroy(c->s);
@@ -1548,6 +1559,7 @@ int mmh_create(mmh_ctx** out, const mmh_config* cfg) {
     }
     c->own_stream = true;
   }
+  c->cycle_fits = cfg->precision == MMH_MIXED && n >= 16 && cycle32_fits(c->s);
   int rc = MMH_OK;
   i64 n3 = c->n3;
   // Scratch that is dead while the FP64 relaxing and its adjoint run
@@ -1779,6 +1791,15 @@ int mmh_gs_tile(int n, int* tx, int* ty) {
   return mmh::gs_tile_chosen(n, tx, ty) >= 0 ? MMH_OK : MMH_ERR_ARG;
 }
 
+int mmh_max_cluster(mmh_ctx* c, int ctas) {
+  if (!c || (ctas != 8 && ctas != 16)) return MMH_ERR_ARG;
+  if (ctas == c->max_cluster) return MMH_OK;
+  CK(cudaStreamSynchronize(c->s));
+  c->drop_graphs();  // they hold the launches of the limit before
+  c->max_cluster = ctas;
+  return MMH_OK;
+}
+
 int mmh_keep_masks(mmh_ctx* c, int on) {
   if (!c) return MMH_ERR_ARG;
   if (on && !c->masks) {
@@ -1936,7 +1957,8 @@ int mmh_relax_f64(mmh_ctx* c, double* arr, double* resid, const double* rhs, con
   }
   launch_metric<double>(c->defl[l], c->rhol[l], n, dx, c->h64.coef[l], c->s);
   double *du = c->h64.u[l], *dr = c->h64.r[l];
-  if (launch_gs64_sweeps(du, c->h64.rhs[l], c->h64.coef[l], n, dx, nrelax, dr, c->s) != du) std::swap(du, dr);
+  if (launch_gs64_sweeps(du, c->h64.rhs[l], c->h64.coef[l], n, dx, nrelax, dr, c->s, c->max_cluster) != du)
+    std::swap(du, dr);
   CK(cudaMemsetAsync(c->sc->errbits, 0, 8, c->s));
   if (ir != 0) {
     launch_residual<double>(du, c->h64.rhs[l], c->h64.coef[l], n, dx, ir == 3 ? dr : nullptr,

@@ -45,6 +45,7 @@ EXPORTS = (
     "mmh_relaxing_adjoint_f64", "mmh_iterate_adjoint_f64", "mmh_state_stats",
     "mmh_power_spectrum_f64", "mmh_haloden", "mmh_haloden_planes", "mmh_coarsen",
     "mmh_column_density", "mmh_gridfigure", "mmh_keep_masks", "mmh_masks", "mmh_gs_tile_pin", "mmh_gs_tile", "mmh_stencil_pin",
+    "mmh_max_cluster",
 )
 
 # kernel kinds for the timing hooks
@@ -457,6 +458,10 @@ class Context:
         m = np.zeros(nbins, dtype=np.int64)
         _chk(lib().mmh_power_spectrum_f64(self._h, _p(a), _p(b), int(nbins), _p(k), _p(p), _p(m)), "power_spectrum")
         return k, p, m
+
+    def max_cluster(self, ctas):
+        """Limit the clusters of the small levels' kernels to 8 CTAs, or back to 16."""
+        _chk(lib().mmh_max_cluster(self._h, int(ctas)), "max_cluster")
 
     def keep_masks(self, on=True):
         """Arm (or disarm) keeping the limiter masks of every calcdefp."""
