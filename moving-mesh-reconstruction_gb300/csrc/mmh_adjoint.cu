@@ -392,8 +392,8 @@ __global__ void k_adj_alpha(const double* __restrict__ baj, const double* __rest
 // branches are the forward's).  Axis by axis: k_adj_faces forms what each upper
 // face gives (7 planes, in the place of the metric, which is done with by
 // then), k_adj_gather adds up a cell's four faces.  Four cells read a face;
-// formed by each of them, the faces took 420 FP64 instructions per cell instead
-// of 100 (64^3: 217 us, now 114).  cb: n^3 doubles, the running sum of cbar.
+// formed by each of them, the faces took 434 FP64 instructions per cell instead
+// of 132, 29 + 15 an axis (64^3: 217 us, now 114).  cb: n^3 doubles, the running sum of cbar.
 __global__ void k_adj_faces(const double* __restrict__ sd, const double* __restrict__ cc,
                             const double* __restrict__ rbar, double scale, int n, int axis, double* __restrict__ fa) {
   const i64 n3 = (i64)n * n * n, t = (i64)blockIdx.x * blockDim.x + threadIdx.x;

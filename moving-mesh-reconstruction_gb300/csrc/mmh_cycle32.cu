@@ -438,12 +438,15 @@ __global__ void __launch_bounds__(kThreads) k_cycle32(CycleArgs a, const float* 
   }
 }
 
-// Dot product over the cluster with the sums of launch_dot_fast: products
+// Dot product over the cluster with the sums of k_pcg_dot on such a grid (one
+// product per thread there, its halving over empty blocks as well): products
 // rounded to FP32, blocks of 256 consecutive cells (a warp's 32 by shuffles,
 // the 8 warps in order), the block sums in FP64 by halving.  dot_post leaves
 // every CTA the block sums in slot[which]; after a cluster barrier dot_sum
 // (one warp) adds them.  Two uses of the same slots have a cluster barrier
-// between the reads of one and the writes of the next.
+// between the reads of one and the writes of the next.  The total is not
+// rounded to a fixed point as dot_rounded does: with E of the maxima that is 2^(E
+// - 96), which changes no total above 2^(E - 44).
 template <int N>
 __device__ __forceinline__ void dot_post(const Me& me, Shared* sh, int which, const float* a, const float* b) {
   typedef Slab<N> S;
@@ -476,10 +479,10 @@ __device__ __forceinline__ double dot_sum(const Shared* sh, int which) {
     t = lane < 16 ? v[lane] : 0.0;
   for (int d = 16; d > 0; d >>= 1) t = __dadd_rn(t, __shfl_down_sync(0xffffffffu, t, d));
   t = __shfl_sync(0xffffffffu, t, 0);
-  return fabs(t) < INFINITY ? t : 0.0;  // as launch_dot_fast
+  return fabs(t) < INFINITY ? t : 0.0;  // as dot_rounded
 }
 
-// The inner solve of the mixed form (pcg_core<float> from a zero guess): x = 0,
+// The inner solve of the mixed form (pcg_core32's): x = 0,
 // r = b in rhs; flexible conjugate gradients preconditioned by one cycle until
 // max|r| <= tol * bn or maxit iterations.  x out; out[0] = iterations, out[1]
 // = max|r| (as double bits), the residual left in rhs.

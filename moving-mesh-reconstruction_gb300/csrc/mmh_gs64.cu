@@ -258,7 +258,7 @@ int rows_ty(int n) { return n <= 32 ? 8 : (n == 64 || n > 512 ? 16 : 32); }
 // (warp S): a phase costs 13, 13, 20, 13 dependent FP64 instructions instead
 // of some 75 (64 cycles each).
 // Against one CTA with a thread per cell: 32 sweeps at 4^3 183 us (747), at
-// 8^3 323 us (771); 16 sweeps at 16^3 185 us (1508).
+// 8^3 244 us (771); 16 sweeps at 16^3 162 us (1508).
 // ---------------------------------------------------------------------------
 template <int N>
 struct BoxGeom {

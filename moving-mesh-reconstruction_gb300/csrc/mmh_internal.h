@@ -200,7 +200,7 @@ void launch_pcg_alpha32(const float* p, const float* q, i64 count, PcgDev* P, do
 void launch_pcg_beta32(const float* z, const float* q, const float* r, i64 count, PcgDev* P, double* part,
                        cudaStream_t s);
 
-// the mixed form's nsmooth: three axis passes, `in` overwritten
+// the mixed form's nsmooth: three axis passes; `in` may be overwritten
 void launch_smooth_sep(double* in, int n, double* out, cudaStream_t s);
 
 // float-float outer loop of the mixed form (mmh_kernels_f64.cu): a double

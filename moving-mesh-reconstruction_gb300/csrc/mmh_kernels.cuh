@@ -207,9 +207,12 @@ __device__ __forceinline__ double neg_of(double x) {
 // drains, and then wait until it has completed and its stores are visible.
 // Nothing comes before the wait, so the order of a stream is what it was; what
 // goes is part of the gap between two kernels (1.5 us: four iterations at 32^3 in
-// the mixed form 4.6 ms, 4.2 so).  Not for kernels inside the captured cycles nor
-// for those with much shared memory: FP64 solves became 3 to 8% slower, a batch
-// of realisations on several streams 11%.
+// the mixed form 4.6 ms, 4.2 so).  Not for the sweeps, residuals and transfers of
+// the captured cycles nor for kernels with much shared memory: FP64 solves became
+// 3 to 8% slower, a batch of realisations on several streams 11%.  The small
+// kernels that the FP64 cycle shares with the rest (k_fill, k_fxsum, k_fx_mean,
+// k_sub_mean_unless) are launched so inside it too: ref_64's two iterations 5.88
+// ms, 5.92 with plain launches of these.
 //   A kernel without pdl_begin must not be launched this way, and a kernel with
 // it, and what it inlines, takes no __restrict__ parameters and uses no __ldg:
 // its inputs may still be written while its first blocks wait, which

@@ -1282,8 +1282,9 @@ void launch_residual_ff(const double* phi, const double* rhs, const double* coef
 
 // One axis of the smoother [1/4, 1/2, 1/4] (the 27-point nsmooth of
 // limiter.f90:677-781 is its product over the three axes), periodic, as a
-// pass without its weights: out = in[-1] + in[+1] + 2 in (one add and one fused multiply-add; 2 in is exact).  The
-// last pass applies the three passes' weights, 1/64, at once (on the bits).  Scaling by a
+// pass without its weights: out = in[-1] + in[+1] + 2 in (one add and one fused
+// multiply-add; 2 in is exact).  The last pass applies the three passes'
+// weights, 1/64, at once (on the bits).  Scaling by a
 // power of two is exact and commutes with rounding, so the result has the
 // bits of three passes of (in[-1] + in[+1]) / 4 + in / 2.
 template <bool LAST>
@@ -1333,8 +1334,8 @@ __global__ void __launch_bounds__(256) k_smooth_rows(const double* in, int n, do
   }
 }
 // The 27-point smoother as three axis passes (the mixed form's nsmooth:
-// the same operator, other rounding): in -> out -> in -> out; in is
-// overwritten.
+// the same operator, other rounding): one launch up to 64^3, above in -> out ->
+// in -> out, which overwrites in.
 void launch_smooth_sep(double* in, int n, double* out, cudaStream_t s) {
   const i64 n3 = (i64)n * n * n;
   if (n <= 64) {
