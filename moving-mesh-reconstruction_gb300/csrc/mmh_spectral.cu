@@ -117,10 +117,11 @@ __global__ void k_fft_tables(double* tab, int n) {
 }
 
 // T(x, z) = sum_y (-1)^y d (blockIdx.y = 0), T(x, y) = sum_z (-1)^z d (1):
-// n x n each, x fastest
-__global__ void k_altsum(const double* __restrict__ d, int n, double* __restrict__ T) {
+// n x n each, x fastest.  Clears the x pass's word (see LineArgs).
+__global__ void k_altsum(const double* __restrict__ d, int n, double* __restrict__ T, unsigned* bad) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n * n) return;
+  if (t == 0 && blockIdx.y == 0) *bad = 0;
   const int x = t & (n - 1), o = t / n;
   const i64 n2 = (i64)n * n;
   const double* p = d + x + (blockIdx.y == 0 ? n2 * o : (i64)n * o);
@@ -325,12 +326,13 @@ void lines_run(const double* src, double* grad, double* delta, const double* tab
   smem_attr_once(k_lines<N>, smem, done);
   const i64 n2 = (i64)N * N, n3 = n2 * N;
   const dim3 grid(N / 2 / F::LC, N);
-  cudaMemsetAsync(bad, 0, sizeof(unsigned), s);
   if (grad) {
-    k_altsum<<<dim3((unsigned)((n2 + 127) / 128), 2), 128, 0, s>>>(src, N, T);
+    k_altsum<<<dim3((unsigned)((n2 + 127) / 128), 2), 128, 0, s>>>(src, N, T, bad);
     // both T fields, in place: a CTA has read its lines before it writes them
     k_lines<N><<<dim3(N / F::LC, 1), F::NT, smem, s>>>(LineArgs{T, T, nullptr, nullptr, tab, kHilbert, nullptr, nullptr});
     count_launch(2);
+  } else {
+    cudaMemsetAsync(bad, 0, sizeof(unsigned), s);
   }
   for (int ax = 0; ax < 3; ++ax) {
     const LineArgs a{src, grad ? grad + ax * n3 : nullptr, delta, ax == 0 ? nullptr : T + (ax - 1) * n2, tab, ax, bad,
